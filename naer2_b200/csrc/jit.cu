@@ -24,6 +24,7 @@ struct n2b_jit_kernel {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t kernel = nullptr;
     int device = 0;
+    bool early = false;  // the source waits for the launch before it itself (griddepcontrol.wait)
 };
 
 namespace {
@@ -133,6 +134,7 @@ int n2b_jit_compile(const char *source, const char *kernel_name, const char *con
     if (!n) return n2b_host::set_error(N2B_ECUDA, "NVRTC returned no device image");
     n2b_jit_kernel *k = new n2b_jit_kernel();
     k->device = device;
+    k->early = std::strstr(source, "griddepcontrol.wait") != nullptr;
     e = cudaLibraryLoadData(&k->lib, image.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&k->kernel, k->lib, kernel_name);
     if (e != cudaSuccess) {
@@ -186,8 +188,17 @@ int n2b_jit_launch_window(n2b_jit_kernel *const *kernels, const uint32_t *grids,
             std::memcpy(P + 24, &t, sizeof(t));
             std::memcpy(P + 28, &t0, sizeof(t0));
             void *args[] = {P};  // (the launch copies the parameter block)
-            e = cudaLaunchKernel(reinterpret_cast<const void *>(kernels[k]->kernel), dim3(grids[k]), dim3(blocks[k]),
-                                 args, 0, reinterpret_cast<cudaStream_t>(stream));
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(grids[k]);
+            cfg.blockDim = dim3(blocks[k]);
+            cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+            // a kernel that waits for its predecessor itself is scheduled under it (its set-up loads overlap)
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = kernels[k]->early ? 1 : 0;
+            e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void *>(kernels[k]->kernel), args);
         }
     }
     if (e != cudaSuccess) return n2b_host::set_error(N2B_ECUDA, std::string("launch: ") + cudaGetErrorString(e));

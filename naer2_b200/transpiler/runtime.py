@@ -17,11 +17,18 @@ import hashlib
 import numpy as np
 import torch
 
-from .. import _lib
+from .. import _lib, receives
+from ..hook import assigned_members
 from ..topology import delay_steps, pull_form
-from .template import NPB_C, build_source, ctype_of, edge_hook_context, hook_context, params_type, scan
+from .template import (EXACT_THREADS, NPB_C, Out, build_source, ctype_of, edge_hook_context, hook_context,
+                       params_type, scan)
 
-BLOCK = 128  # exact-time intake: one thread per neuron
+BLOCK = 128  # exact-time intake without arrival bits: one thread per neuron
+# A network's intake reads arrival bits (one bit per link and arrival slot, set by the spikes' deliveries) as long
+# as they and the outgoing rows take at most this much; past it, every neuron looks its whole incoming row up in
+# its sources' spike rings, which needs no more memory than the links. At 12,500 neurons of 1,250 links and 32
+# slots the bits are 64 MB, the rows 78 MB.
+ARRIVAL_BYTES = 32 << 30
 _CACHE: dict = {}  # (source hash, device) -> n2b_jit_kernel handle, for the process's lifetime
 
 
@@ -51,7 +58,6 @@ class EdgePlan:
     non-trivial hooks (or None)."""
 
     def __init__(self, conn, receive_hook):
-        from .. import receives
         from ..hook import used_members
 
         fabric = conn.fabric
@@ -86,10 +92,48 @@ class EdgePlan:
         return torch.full((n_links,), float(v.item() if isinstance(v, torch.Tensor) else v), dtype=torch.float32)
 
 
+def arrival_bytes(n_tgt: int, n_links: int, depth: int) -> int:
+    """Device bytes of a connection's arrival bits (`depth` slots of one bit per link, rows starting words of their
+    own) and outgoing rows (5 bytes per link), at most."""
+    return depth * 4 * (n_links // 32 + n_tgt) + 5 * n_links
+
+
+def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -> dict:
+    """The arrival bits of one connection, from its pull CSR: `wptr` int32 [n_tgt + 1], each row's first word in a
+    slot; `words` per slot; `depth`, the slots (a power of two above every delay); the outgoing rows `out_ptr`
+    int32 [n_src + 1], `pos` int32 (uint32 bits: the link's bit in a slot) and `dly` uint8, links of a source in
+    pull order; `bad`: links whose source or delay (1 .. mask) is out of range, in no outgoing row."""
+    dev = link.device
+    n_tgt = len(ptr) - 1
+    ptr = ptr.to(torch.int64)
+    lens = ptr.diff()
+    wptr = torch.zeros(n_tgt + 1, dtype=torch.int64, device=dev)
+    wptr[1:] = torch.cumsum((lens + 31) // 32, 0)
+    n_links = int(ptr[-1]) if n_tgt else 0
+    link = link[:n_links]
+    src, dly = link & 0xFFFFFF, (link >> 24) & 0xFF
+    pos = torch.repeat_interleave(wptr[:-1] * 32 - ptr[:-1], lens) + torch.arange(n_links, device=dev)
+    good = (dly >= 1) & (dly <= mask) & (src < n_src)
+    bad = n_links - int(good.sum())
+    if bad:
+        src, dly, pos = src[good], dly[good], pos[good]
+    order = torch.argsort(src, stable=True)
+    out_ptr = torch.zeros(n_src + 1, dtype=torch.int64, device=dev)
+    out_ptr[1:] = torch.cumsum(torch.bincount(src, minlength=n_src)[:n_src], 0)
+    dly = dly[order]
+    top = int(dly.max()) if dly.numel() else 1
+    pos = pos[order]
+    return {"wptr": wptr.to(torch.int32), "words": int(wptr[-1]), "depth": 1 << top.bit_length(),
+            "out_ptr": out_ptr.to(torch.int32),
+            "pos": torch.where(pos >= 2 ** 31, pos - 2 ** 32, pos).to(torch.int32), "dly": dly.to(torch.uint8),
+            "bad": bad}
+
+
 def plan_of(net) -> dict:
     """The transpiled form of a network, everything its step kernels need and nothing of its Python model classes:
     per population its CUDA source, the Params fields with the values of the scalar ones, its state attributes
-    (name -> "float" / "int" / "bool"), size, seed and spike-ring depth; per incoming connection (in order) its
+    (name -> "float" / "int" / "bool"), size, seed and spike-ring depth, and (networks whose intake reads arrival
+    bits) its outgoing connections; per incoming connection (in order) its
     source population, pull CSR (int32 ptr, uint32 link words) and per-link edge arrays (pull order) with the
     pull permutation. JitRuntime builds from it; save_plan / load_plan keep it in a file, so that a network can
     be transpiled where its model classes are and stepped where only the plan is."""
@@ -110,10 +154,17 @@ def plan_of(net) -> dict:
     depth = [max(2, 1 << int(np.ceil(np.log2(m + 1)))) for m in max_out]
     exact = bool(getattr(net, "exact", False))
     plan = {"dt": dt, "exact": exact, "pops": []}
+    incoming_of = [[c for c in net.connections if c._target is p] for p in pops]
+    outs = [[] for _ in pops]  # each population's outgoing connections: (target population, its connection)
+    for k, conns in enumerate(incoming_of):
+        for ci, c in enumerate(conns):
+            outs[index[id(c._source)]].append([k, ci])
+    arrivals = sum(arrival_bytes(len(p.shape), len(c.fabric.topology), depth[index[id(c._source)]])
+                   for p, conns in zip(pops, incoming_of) for c in conns) <= ARRIVAL_BYTES
     for k, p in enumerate(pops):
         node = p.node
         incoming = []
-        conns = [c for c in net.connections if c._target is p]
+        conns = incoming_of[k]
         site = 0
         for c in conns:
             port = c._target_port or "receive"
@@ -132,15 +183,20 @@ def plan_of(net) -> dict:
                 eh = getattr(ep, kind)
                 if eh is not None:
                     inc[kind] = (eh.ast, edge_hook_context(p, eh, ep.per_link, ep.static))
+            if ep.backward is not None:
+                dst = ep.backward.parameter_type_to_name.get(receives.destination)
+                inc["backward_writes"] = dst is not None and bool(assigned_members(ep.backward.ast, dst))
             incoming.append(inc)
         hooks = {"update": (node.update.ast, hook_context(p, node.update, site_base=site)),
                  "send": (node.send.ast, hook_context(p, node.send, site_base=site + 32))}
         src, fields = build_source(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
-                                   exact=exact, n=len(p.shape))
+                                   exact=exact, n=len(p.shape), arrivals=arrivals, n_out=len(outs[k]))
         attrs = {a: ("bool" if py is bool else "int" if py is int else "float") for a, py in p.dynamic_attrs.items()}
         entry = {"name": type(p.instance).__name__, "n": len(p.shape), "words": words[k], "depth": depth[k],
                  "seed": int(p.seed) & 0xFFFFFFFFFFFFFFFF, "source": src,
                  "fields": [(name, ctype) for name, ctype, _ in fields], "attrs": attrs, "conns": []}
+        if arrivals:
+            entry["outs"] = outs[k]
         for inc in incoming:
             c = inc["conn"]
             topo = c.fabric.topology
@@ -164,7 +220,8 @@ def save_plan(plan: dict, path) -> None:
 
     arrays, meta = {}, {"dt": plan["dt"], "exact": plan["exact"], "pops": []}
     for k, p in enumerate(plan["pops"]):
-        m = {key: p[key] for key in ("name", "n", "words", "depth", "seed", "source", "fields", "attrs")}
+        m = {key: p[key] for key in ("name", "n", "words", "depth", "seed", "source", "fields", "attrs", "outs")
+             if key in p}
         m["conns"] = []
         for ci, c in enumerate(p["conns"]):
             for key in ("ptr", "link", "perm"):
@@ -202,7 +259,12 @@ _CTYPES = {"long long": ctypes.c_int64, "float": ctypes.c_float, "int": ctypes.c
 
 def _params_struct(fields: list):
     """The ctypes Params structure of a plan's fields (pointers as void *)."""
-    return params_type([(name, ct, ctypes.c_void_p if ct.endswith("*") else _CTYPES[ct]) for name, ct in fields])
+    def ctype(ct):
+        if ct.startswith("N2Out["):
+            return Out * int(ct[6:-1])
+        return ctypes.c_void_p if ct.endswith("*") else _CTYPES[ct]
+
+    return params_type([(name, ct, ctype(ct)) for name, ct in fields])
 
 
 class JitRuntime:
@@ -234,6 +296,7 @@ class JitRuntime:
         self.raster_offs = [torch.zeros(max(1, self.record_rows) * max(1, p["n"]), dtype=torch.float32,
                                         device=dev) for p in plan["pops"]]
         self.kernels, self.params, self.sources = [], [], []
+        forms = []  # per population, its incoming connections' arrival forms
         self.edge_arrays = {}  # (connection id, edge name) -> (per-link values in pull order, pull permutation)
         tdtype = {"bool": torch.bool, "int": torch.int32, "float": torch.float32}
         for k, (p, pp) in enumerate(zip(pops, plan["pops"])):
@@ -255,22 +318,43 @@ class JitRuntime:
             P.raster_steps, P.rec0 = self.record_rows, self.rec_step0
             P.err = self.err[k:].data_ptr()
             P.counters = self.counters_t[k].data_ptr()
+            bad = 0
+            forms.append([])
             for ci, c in enumerate(pp["conns"]):
                 s = c["src"]
+                have = {f for f, _ in pp["fields"] if f.startswith(f"c{ci}_")}
                 ptr = self._dev(c["ptr"])
-                link = self._dev(c["link"] if c["link"].numel() else torch.zeros(1, dtype=torch.int32))
                 setattr(P, f"c{ci}_ptr", ptr.data_ptr())
-                setattr(P, f"c{ci}_link", link.data_ptr())
-                setattr(P, f"c{ci}_src_bits", self.bits[s].data_ptr())
-                setattr(P, f"c{ci}_src_words", words[s])
-                setattr(P, f"c{ci}_src_mask", depth[s] - 1)
-                setattr(P, f"c{ci}_src_off", self.offs[s].data_ptr())
-                setattr(P, f"c{ci}_src_n", plan["pops"][s]["n"])
+                if f"c{ci}_link" in have:
+                    link = self._dev(c["link"] if c["link"].numel() else torch.zeros(1, dtype=torch.int32))
+                    values = {"link": link.data_ptr(), "src_bits": self.bits[s].data_ptr(), "src_words": words[s],
+                              "src_mask": depth[s] - 1, "src_off": self.offs[s].data_ptr(),
+                              "src_n": plan["pops"][s]["n"]}
+                    for name, v in values.items():
+                        if f"c{ci}_{name}" in have:
+                            setattr(P, f"c{ci}_{name}", v)
+                if "outs" in pp:
+                    f = arrival_form(ptr, c["link"].to(dev), plan["pops"][s]["n"], depth[s] - 1)
+                    bad += f["bad"]
+                    f["arr"] = torch.zeros(max(1, f["depth"] * f["words"]), dtype=torch.int32, device=dev)
+                    self.keep += [f[x] for x in ("wptr", "out_ptr", "pos", "dly", "arr")]
+                    setattr(P, f"c{ci}_wptr", f["wptr"].data_ptr())
+                    setattr(P, f"c{ci}_arr", f["arr"].data_ptr())
+                    setattr(P, f"c{ci}_arr_words", f["words"])
+                    setattr(P, f"c{ci}_arr_mask", f["depth"] - 1)
+                    forms[k].append(f)
                 for e, v in c["per_link"].items():
                     v = self._dev(v if v.numel() else torch.zeros(1))
                     self.edge_arrays[(c["conn_id"], e)] = (v, c["perm"])
                     setattr(P, f"c{ci}_e_{e}", v.data_ptr())
+            if "outs" in pp:
+                P.bad = bad
             self.params.append(P)
+        for P, pp in zip(self.params, plan["pops"]):
+            for o, (tgt, ci) in enumerate(pp.get("outs", ())):
+                f = forms[tgt][ci]
+                P.outs[o] = Out(ptr=f["out_ptr"].data_ptr(), pos=f["pos"].data_ptr(), dly=f["dly"].data_ptr(),
+                                arr=f["arr"].data_ptr(), words=f["words"], mask=f["depth"] - 1)
         self.stream = torch.cuda.Stream(device=dev)
         self._s = ctypes.c_void_p(self.stream.cuda_stream)
         self.launches = 0
@@ -294,11 +378,11 @@ class JitRuntime:
         k = len(self.kernels)
         grids, blocks = (ctypes.c_uint32 * k)(), (ctypes.c_uint32 * k)()
         kerns, params, sizes = (ctypes.c_void_p * k)(), (ctypes.c_void_p * k)(), (ctypes.c_size_t * k)()
-        for i, (kern, P, p) in enumerate(zip(self.kernels, self.params, self.pops)):
-            per = BLOCK if self.exact else NPB_C  # neurons per block (clocked: SCAN threads each)
+        for i, (kern, P, p, pp) in enumerate(zip(self.kernels, self.params, self.pops, self.plan["pops"])):
             size = len(p.shape)
+            blocks[i] = scan(size) * NPB_C if not self.exact else EXACT_THREADS if "outs" in pp else BLOCK
+            per = BLOCK if self.exact and "outs" not in pp else NPB_C  # neurons per block
             grids[i] = (size + per - 1) // per
-            blocks[i] = BLOCK if self.exact else scan(size) * NPB_C
             kerns[i] = kern.value
             params[i] = ctypes.addressof(P)
             sizes[i] = ctypes.sizeof(P)

@@ -161,6 +161,35 @@ int n2b_jit_launch(n2b_jit_kernel *k, uint32_t grid, uint32_t block, const void 
     return N2B_OK;
 }
 
+int n2b_jit_resident_blocks(n2b_jit_kernel *k, uint32_t block, int32_t *blocks) {
+    if (!k || !blocks || block == 0 || block > 1024) return n2b_host::set_error(N2B_EINVAL, "bad arguments");
+    JitDeviceGuard guard;
+    int per_sm = 0, sms = 0;
+    cudaError_t e = cudaSetDevice(k->device);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void *>(k->kernel), (int)block,
+                                                          0);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, k->device);
+    if (e != cudaSuccess) return n2b_host::set_error(N2B_ECUDA, std::string("occupancy: ") + cudaGetErrorString(e));
+    *blocks = per_sm * sms;
+    return N2B_OK;
+}
+
+int n2b_jit_launch_cooperative(n2b_jit_kernel *k, uint32_t grid, uint32_t block, const void *params,
+                               size_t params_bytes, void *stream) {
+    if (!k || !params || params_bytes == 0 || grid == 0 || block == 0 || block > 1024)
+        return n2b_host::set_error(N2B_EINVAL, "bad arguments");
+    JitDeviceGuard guard;
+    cudaError_t e = cudaSetDevice(k->device);
+    if (e == cudaSuccess) {
+        void *args[] = {const_cast<void *>(params)};
+        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k->kernel), dim3(grid), dim3(block), args, 0,
+                                        reinterpret_cast<cudaStream_t>(stream));
+    }
+    if (e != cudaSuccess) return n2b_host::set_error(N2B_ECUDA, std::string("launch: ") + cudaGetErrorString(e));
+    return N2B_OK;
+}
+
 int n2b_jit_launch_window(n2b_jit_kernel *const *kernels, const uint32_t *grids, const uint32_t *blocks,
                           const void *const *params, const size_t *params_bytes, int32_t n_kernels, int64_t step0,
                           int64_t n_steps, double dt, void *stream) {

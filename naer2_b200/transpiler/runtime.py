@@ -20,8 +20,8 @@ import torch
 from .. import _lib, receives
 from ..hook import assigned_members
 from ..topology import delay_steps, pull_form
-from .template import (EXACT_THREADS, NPB_C, Out, build_source, ctype_of, edge_hook_context, hook_context,
-                       params_type, scan)
+from . import arrival
+from .template import NPB_C, build_source, ctype_of, edge_hook_context, hook_context, params_type, scan
 
 BLOCK = 128  # exact-time intake without arrival bits: one thread per neuron
 # A network's intake reads arrival bits (one bit per link and arrival slot, set by the spikes' deliveries) as long
@@ -29,15 +29,20 @@ BLOCK = 128  # exact-time intake without arrival bits: one thread per neuron
 # its sources' spike rings, which needs no more memory than the links. At 12,500 neurons of 1,250 links and 32
 # slots the bits are 64 MB, the rows 78 MB.
 ARRIVAL_BYTES = 32 << 30
+# A window kernel holds every block of the network at once: 592 blocks (18,944 neurons) are four per SM, 64 registers
+# a thread, which the step's code needs (five per SM would be 51). Larger networks, those of more than
+# arrival.WINDOW_POPS populations, and devices that hold fewer blocks step by one launch per population.
+WINDOW_BLOCKS, WINDOW_SMS = 592, 148
+BARRIER_LIMIT_NS = 2_000_000_000  # how long a window's block waits at its grid barrier before it gives up
 _CACHE: dict = {}  # (source hash, device) -> n2b_jit_kernel handle, for the process's lifetime
 
 
-def compile_source(source: str, device: int) -> ctypes.c_void_p:
+def compile_source(source: str, device: int, name: bytes = b"n2b_user_step") -> ctypes.c_void_p:
     key = (hashlib.sha256(source.encode()).hexdigest(), device)
     if key not in _CACHE:
         lib = _lib.load()
         h = ctypes.c_void_p()
-        _lib.check(lib.n2b_jit_compile(source.encode(), b"n2b_user_step", None, 0, device, ctypes.byref(h)),
+        _lib.check(lib.n2b_jit_compile(source.encode(), name, None, 0, device, ctypes.byref(h)),
                    "n2b_jit_compile")
         _CACHE[key] = h
     return _CACHE[key]
@@ -161,6 +166,7 @@ def plan_of(net) -> dict:
             outs[index[id(c._source)]].append([k, ci])
     arrivals = sum(arrival_bytes(len(p.shape), len(c.fabric.topology), depth[index[id(c._source)]])
                    for p, conns in zip(pops, incoming_of) for c in conns) <= ARRIVAL_BYTES
+    bodies = []  # arrival bits: the populations' part of the window kernel
     for k, p in enumerate(pops):
         node = p.node
         incoming = []
@@ -189,8 +195,13 @@ def plan_of(net) -> dict:
             incoming.append(inc)
         hooks = {"update": (node.update.ast, hook_context(p, node.update, site_base=site)),
                  "send": (node.send.ast, hook_context(p, node.send, site_base=site + 32))}
-        src, fields = build_source(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
-                                   exact=exact, n=len(p.shape), arrivals=arrivals, n_out=len(outs[k]))
+        if arrivals:
+            src, fields, body = arrival.build(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
+                                              len(outs[k]), exact)
+            bodies.append(body)
+        else:
+            src, fields = build_source(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
+                                       exact=exact, n=len(p.shape))
         attrs = {a: ("bool" if py is bool else "int" if py is int else "float") for a, py in p.dynamic_attrs.items()}
         entry = {"name": type(p.instance).__name__, "n": len(p.shape), "words": words[k], "depth": depth[k],
                  "seed": int(p.seed) & 0xFFFFFFFFFFFFFFFF, "source": src,
@@ -210,6 +221,10 @@ def plan_of(net) -> dict:
                                    "link": link.to(torch.int32).cpu(), "perm": perm.cpu(), "per_link": per_link,
                                    "written": list(ep.written), "conn_id": id(c)})
         plan["pops"].append(entry)
+    sizes = [len(p.shape) for p in pops]
+    total = sum(arrival.blocks_of(n) for n in sizes)
+    if arrivals and 0 < total <= WINDOW_BLOCKS and len(pops) <= arrival.WINDOW_POPS:
+        plan["window"] = arrival.window_source(exact, bodies, sizes, -(-total // WINDOW_SMS))
     plan["device"] = dev
     return plan
 
@@ -219,6 +234,8 @@ def save_plan(plan: dict, path) -> None:
     import json
 
     arrays, meta = {}, {"dt": plan["dt"], "exact": plan["exact"], "pops": []}
+    if "window" in plan:
+        meta["window"] = plan["window"]
     for k, p in enumerate(plan["pops"]):
         m = {key: p[key] for key in ("name", "n", "words", "depth", "seed", "source", "fields", "attrs", "outs")
              if key in p}
@@ -240,6 +257,8 @@ def load_plan(path) -> dict:
     z = np.load(path)
     meta = json.loads(bytes(z["plan_json"]).decode())
     plan = {"dt": meta["dt"], "exact": meta["exact"], "pops": []}
+    if "window" in meta:
+        plan["window"] = meta["window"]
     for k, m in enumerate(meta["pops"]):
         p = dict(m)
         p["fields"] = [tuple(f) for f in m["fields"]]
@@ -261,7 +280,7 @@ def _params_struct(fields: list):
     """The ctypes Params structure of a plan's fields (pointers as void *)."""
     def ctype(ct):
         if ct.startswith("N2Out["):
-            return Out * int(ct[6:-1])
+            return arrival.Out * int(ct[6:-1])
         return ctypes.c_void_p if ct.endswith("*") else _CTYPES[ct]
 
     return params_type([(name, ct, ctype(ct)) for name, ct in fields])
@@ -301,7 +320,6 @@ class JitRuntime:
         tdtype = {"bool": torch.bool, "int": torch.int32, "float": torch.float32}
         for k, (p, pp) in enumerate(zip(pops, plan["pops"])):
             self.sources.append(pp["source"])
-            self.kernels.append(compile_source(pp["source"], dindex))
             P = _params_struct(pp["fields"])()
             P.n, P.words, P.bit_mask = pp["n"], words[k], depth[k] - 1
             P.seed_lo, P.seed_hi = pp["seed"] & 0xFFFFFFFF, (pp["seed"] >> 32) & 0xFFFFFFFF
@@ -353,11 +371,31 @@ class JitRuntime:
         for P, pp in zip(self.params, plan["pops"]):
             for o, (tgt, ci) in enumerate(pp.get("outs", ())):
                 f = forms[tgt][ci]
-                P.outs[o] = Out(ptr=f["out_ptr"].data_ptr(), pos=f["pos"].data_ptr(), dly=f["dly"].data_ptr(),
-                                arr=f["arr"].data_ptr(), words=f["words"], mask=f["depth"] - 1)
+                P.outs[o] = arrival.Out(ptr=f["out_ptr"].data_ptr(), pos=f["pos"].data_ptr(), dly=f["dly"].data_ptr(),
+                                        arr=f["arr"].data_ptr(), words=f["words"], mask=f["depth"] - 1)
+        self.window = self.window_kernel = None  # the window kernel and its parameter block
+        self.window_grid = sum(arrival.blocks_of(p["n"]) for p in plan["pops"])
+        self.bar = torch.zeros(64, dtype=torch.int32, device=dev)  # its grid barrier: arrivals, abort word, stops
+        self.bar_base = 0  # arrivals of the windows so far
+        if "window" in plan:
+            self._window(plan["window"], dindex)
+        if self.window is None:
+            self.kernels = [compile_source(src, dindex) for src in self.sources]
         self.stream = torch.cuda.Stream(device=dev)
         self._s = ctypes.c_void_p(self.stream.cuda_stream)
         self.launches = 0
+
+    def _window(self, source: str, dindex: int) -> None:
+        """The window kernel, where its parameters fit and the device holds all its blocks at once."""
+        W = arrival.window_type([type(P) for P in self.params])
+        if ctypes.sizeof(W) > arrival.WINDOW_PARAMS:
+            return
+        lib, kern, blocks = _lib.load(), compile_source(source, dindex, b"n2b_user_window"), ctypes.c_int32()
+        _lib.check(lib.n2b_jit_resident_blocks(kern, arrival.THREADS, ctypes.byref(blocks)), "n2b_jit_resident_blocks")
+        if blocks.value >= self.window_grid:
+            self.window_kernel, self.window = kern, W()
+            self.window.dt = self.dt
+            self.window.grid.bar = self.bar.data_ptr()
 
     def _dev(self, t):
         t = t.to(self.device).contiguous()
@@ -367,32 +405,55 @@ class JitRuntime:
     # ------------------------------------------------------------------ stepping
 
     def advance(self, n_steps: int) -> None:
-        """Steps step_count .. step_count + n_steps - 1: per step one launch per population, in order, the whole
-        window in one library call (n2b_jit_launch_window writes each launch's step and times)."""
-        lib = _lib.load()
+        """Steps step_count .. step_count + n_steps - 1: one launch of the window kernel or, without it, per step one
+        launch per population, in order, the whole window in one library call (n2b_jit_launch_window writes each
+        launch's step and times)."""
         n_steps = int(n_steps)
         if n_steps <= 0:
             return
         self.stream.wait_stream(torch.cuda.current_stream(self.device))
         step = self.net.step_count
+        if self.window is not None:
+            self._advance_window(step, n_steps)
+        else:
+            self._advance_steps(step, n_steps)
+        last = step + n_steps - 1
+        for P in self.params:  # (the fields as the last launch had them)
+            P.step, P.t, P.t0 = last, (last + 1) * self.dt, last * self.dt
+        torch.cuda.current_stream(self.device).wait_stream(self.stream)
+
+    def _advance_window(self, step: int, n_steps: int) -> None:
+        lib, W = _lib.load(), self.window
+        W.step0, W.n_steps = step, n_steps
+        W.grid.base = self.bar_base
+        W.grid.limit_ns = int(getattr(self.net, "barrier_limit_ns", 0) or BARRIER_LIMIT_NS)
+        for k, P in enumerate(self.params):
+            setattr(W, f"p{k}", P)
+        _lib.check(lib.n2b_jit_launch_cooperative(self.window_kernel, self.window_grid, arrival.THREADS,
+                                                  ctypes.addressof(W), ctypes.sizeof(W), self._s),
+                   "n2b_jit_launch_cooperative")
+        self.bar_base = (self.bar_base + (n_steps - 1) * self.window_grid) & 0xFFFFFFFF
+        self.launches += 1
+
+    def _advance_steps(self, step: int, n_steps: int) -> None:
         k = len(self.kernels)
         grids, blocks = (ctypes.c_uint32 * k)(), (ctypes.c_uint32 * k)()
         kerns, params, sizes = (ctypes.c_void_p * k)(), (ctypes.c_void_p * k)(), (ctypes.c_size_t * k)()
-        for i, (kern, P, p, pp) in enumerate(zip(self.kernels, self.params, self.pops, self.plan["pops"])):
-            size = len(p.shape)
-            blocks[i] = scan(size) * NPB_C if not self.exact else EXACT_THREADS if "outs" in pp else BLOCK
-            per = BLOCK if self.exact and "outs" not in pp else NPB_C  # neurons per block
+        for i, (kern, P, pp) in enumerate(zip(self.kernels, self.params, self.plan["pops"])):
+            size = pp["n"]
+            if "outs" in pp:
+                per, blocks[i] = arrival.NPB_C, arrival.THREADS
+            elif self.exact:
+                per, blocks[i] = BLOCK, BLOCK
+            else:
+                per, blocks[i] = NPB_C, scan(size) * NPB_C
             grids[i] = (size + per - 1) // per
             kerns[i] = kern.value
             params[i] = ctypes.addressof(P)
             sizes[i] = ctypes.sizeof(P)
-        _lib.check(lib.n2b_jit_launch_window(kerns, grids, blocks, params, sizes, k, step, n_steps, self.dt,
-                                             self._s), "n2b_jit_launch_window")
-        last = step + n_steps - 1
-        for P in self.params:  # (the fields as the last launch had them)
-            P.step, P.t, P.t0 = last, (last + 1) * self.dt, last * self.dt
+        _lib.check(_lib.load().n2b_jit_launch_window(kerns, grids, blocks, params, sizes, k, step, n_steps, self.dt,
+                                                     self._s), "n2b_jit_launch_window")
         self.launches += n_steps * sum(1 for g in grids if g)
-        torch.cuda.current_stream(self.device).wait_stream(self.stream)
 
     def start_recording(self, steps: int) -> None:
         if self.record_rows == 0 or steps > self.record_rows:
@@ -454,6 +515,10 @@ class JitRuntime:
         bad = sum(self.status())
         if bad:
             raise RuntimeError(f"{bad} links with a delay outside their source's spike ring")
+        stops = int(self.bar[33])
+        if stops:
+            raise RuntimeError(f"a window of steps stopped: {stops} grid barrier wait(s) gave up (the run is "
+                               "incomplete; reset_counters clears the stop)")
 
     def counters(self) -> dict:
         self.stream.synchronize()
@@ -465,6 +530,8 @@ class JitRuntime:
         self.stream.synchronize()
         self.counters_t.zero_()
         self.err.zero_()
+        self.bar.zero_()
+        self.bar_base = 0
 
     def close(self) -> None:
         self.stream.synchronize()

@@ -97,12 +97,34 @@ def _run(make, k, period, steps, through_file=None):
 def test_arrival_bits_give_the_scanning_intake_bit_for_bit(cuda, monkeypatch, tmp_path, make, k, period):
     got, rt = _run(make, k, period, 61)
     assert all("outs" in p for p in rt.plan["pops"])
+    assert rt.window is not None  # a window of steps per launch
     loaded, _ = _run(make, k, period, 61, through_file=tmp_path / "plan.npz")
+    monkeypatch.setattr(jit_runtime, "WINDOW_BLOCKS", 0)
+    steps, rt = _run(make, k, period, 61)
+    assert rt.window is None and all("outs" in p for p in rt.plan["pops"])  # one launch per population and step
     monkeypatch.setattr(jit_runtime, "ARRIVAL_BYTES", 0)
     want, rt = _run(make, k, period, 61)
     assert not any("outs" in p for p in rt.plan["pops"])
     for a, b in zip(got, want):
         assert a.dtype == b.dtype and np.array_equal(a, b)
+    for a, b in zip(steps, want):
+        assert a.dtype == b.dtype and np.array_equal(a, b)
     for a, b in zip(loaded, want):
         assert np.array_equal(a, b)
     assert sum(int(np.unpackbits(w.view(np.uint8)).sum()) for w in want[:2]) > 50
+
+
+@pytest.mark.gpu
+def test_a_window_whose_barrier_gives_up_reports_it(cuda):
+    """A 1 ns limit makes a block's wait give up while every block still arrives: check() raises, later windows do
+    not run, and reset_counters clears the stop."""
+    net, _ = _plastic(33, 1)
+    net.barrier_limit_ns = 1
+    net.run_steps(200)
+    assert net.runtime.window is not None
+    with pytest.raises(RuntimeError, match="grid barrier"):
+        net.check()
+    net.runtime.reset_counters()
+    net.barrier_limit_ns = 0
+    net.run_steps(20)
+    net.check()

@@ -19,8 +19,8 @@ neurons' state in registers and its row bounds throughout, and the steps are sep
 wait that gives up sets an abort word, and the kernel winds down). A step is a chain of memory latencies, so what it
 costs is the launches around it and the loads that a launch starts with. Measured, us per step, links looked up ->
 arrival bits, one launch per population -> window: 12,500 neurons of 1,250 links (47 spikes a step) 92 -> 19.4 ->
-11.0; 1,501 neurons of 150 plastic links 33 -> 11.2 -> 6.8; 3,001 event-driven neurons of 125 links 73 -> 36 ->
-14.8.
+8.3; 1,501 neurons of 150 plastic links 33 -> 11.2 -> 6.8; 3,001 event-driven neurons of 125 links 73 -> 36 ->
+14.5.
 """
 
 from __future__ import annotations
@@ -34,6 +34,8 @@ SCAN = 8  # threads per neuron: a row of 1,250 links is 40 words, five to a thre
 THREADS = NPB_C * SCAN
 CAP = 16  # clocked intake: arrivals a thread lists of one connection (more stay in their words for the owner)
 OUT_CACHED = 8  # outgoing connections whose row bounds a block holds in shared memory
+PIECE = 256  # links of a row that a warp delivers at once, eight loads a lane in flight
+WORDS_AHEAD = 4  # incoming connections whose arrival words are loaded together at a step's start
 ROWS_AHEAD = 8  # incoming connections whose row bounds a thread holds
 WINDOW_PARAMS = 16384  # bytes of a window kernel's parameter block at most
 WINDOW_POPS = 16  # populations of a window kernel at most (each is a copy of the step's code)
@@ -41,14 +43,14 @@ WINDOW_POPS = 16  # populations of a window kernel at most (each is a copy of th
 _COMMON = r'''
 struct N2Out {
     const int *ptr;            // rows per source neuron
-    const u32 *pos;            // per link: its bit among a slot's words
-    const unsigned char *dly;  // per link: its delay in steps
+    const u32 *pos;            // per link: its bit among a slot's words (dly null: its delay in the top 8 bits)
+    const unsigned char *dly;  // per link: its delay in steps, of connections with more than 2^24 bits to a slot
     u32 *arr;                  // the arrival bits, [mask + 1][words]
     long long words;
     int mask, pad;
 };
 
-constexpr int SCAN = @SCAN@, NPB_C = @NPB@, CAP = @CAP@, MAX_ARRIVALS = @MAXA@, OUT_CACHED = @OUTC@;
+constexpr int SCAN = @SCAN@, NPB_C = @NPB@, CAP = @CAP@, MAX_ARRIVALS = @MAXA@, OUT_CACHED = @OUTC@, PIECE = @PIECE@;
 
 // A block's shared scratch. Clocked: the arrivals that each thread listed; exact times: each neuron's arrivals.
 struct N2Scratch {
@@ -58,22 +60,30 @@ struct N2Scratch {
 @LISTS@
 };
 
-// The links of one row r0 .. r1, strided over `nthr` threads (this one `at`): set each link's bit in the arrival
-// slot of its step. Four links' loads are in flight before their reductions: a row is a chain of memory
-// latencies, not of bandwidth.
-__device__ __forceinline__ void n2_deliver(const N2Out &o, long long n, int r0, int r1, int at, int nthr) {
-    for (int l = r0 + at; l < r1; l += 4 * nthr) {
-        u32 pos[4], d[4];
+// One warp, the links r0 .. r1 (at most PIECE) of a row: set each one's bit in the arrival slot of its step. Every
+// link's load is in flight before the first reduction: a row is a chain of memory latencies, not of bandwidth.
+__device__ __forceinline__ void n2_deliver(const N2Out &o, long long n, int r0, int r1) {
+    u32 pos[PIECE / 32], d[PIECE / 32];
+    const int l0 = r0 + (int)(threadIdx.x & 31);
+    if (o.dly) {
         #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int q = l + k * nthr;
-            d[k] = q < r1 ? __ldg(o.dly + q) : 0u;
-            pos[k] = q < r1 ? __ldg(o.pos + q) : 0u;
+        for (int k = 0; k < PIECE / 32; ++k) {
+            const int l = l0 + 32 * k;
+            d[k] = l < r1 ? __ldg(o.dly + l) : 0u;
+            pos[k] = l < r1 ? __ldg(o.pos + l) : 0u;
         }
+    } else {
         #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (d[k]) atomicOr(o.arr + (size_t)((n + d[k]) & o.mask) * o.words + (pos[k] >> 5), 1u << (pos[k] & 31u));
+        for (int k = 0; k < PIECE / 32; ++k) pos[k] = l0 + 32 * k < r1 ? __ldg(o.pos + l0 + 32 * k) : 0u;
+        #pragma unroll
+        for (int k = 0; k < PIECE / 32; ++k) {
+            d[k] = pos[k] >> 24;
+            pos[k] &= 0xFFFFFFu;
+        }
     }
+    #pragma unroll
+    for (int k = 0; k < PIECE / 32; ++k)
+        if (d[k]) atomicOr(o.arr + (size_t)((n + d[k]) & o.mask) * o.words + (pos[k] >> 5), 1u << (pos[k] & 31u));
 }
 
 // The grid barrier of a window: `bar[0]` counts arrivals, `bar[32]` is set when a wait gave up (bar[33]: how many).
@@ -138,7 +148,7 @@ class Grid(ctypes.Structure):
 
 def common(exact: bool) -> str:
     text = _COMMON.replace("@LISTS@", _LISTS[exact])
-    for key, v in (("SCAN", SCAN), ("NPB", NPB_C), ("CAP", CAP), ("MAXA", MAX_ARRIVALS), ("OUTC", OUT_CACHED)):
+    for key, v in (("SCAN", SCAN), ("NPB", NPB_C), ("CAP", CAP), ("MAXA", MAX_ARRIVALS), ("OUTC", OUT_CACHED), ("PIECE", PIECE)):
         text = text.replace(f"@{key}@", str(v))
     return text
 
@@ -165,10 +175,28 @@ def _words_of(c: int) -> str:
             u32 *arr = p.c{c}_arr + (size_t)(n & p.c{c}_arr_mask) * p.c{c}_arr_words;
             const int seg = (w1 - w0 + SCAN - 1) / SCAN;
             const int a = min(w1, w0 + sc * seg), b = min(w1, a + seg);
-            u32 x[4];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = a + i < b ? __ldcg(arr + a + i) : 0u;
+""" + (f"            u32 (&x)[4] = x{c};\n" if c < WORDS_AHEAD else f"            u32 x[4];\n{_first_words('arr', 'a', 'b', 12)}")
+
+
+def _first_words(arr: str, a: str, b: str, pad: int) -> str:
+    return (" " * pad + "#pragma unroll\n" + " " * pad +
+            f"for (int i = 0; i < 4; ++i) x[i] = {a} + i < {b} ? __ldcg({arr} + {a} + i) : 0u;\n")
+
+
+def _words_ahead(incoming: list) -> str:
+    """The first connections' first words, loaded together: their latencies overlap."""
+    out = ""
+    for c, inc in enumerate(incoming[:WORDS_AHEAD]):
+        if takes(inc):
+            out += f"""        u32 x{c}[4];
+        {{
+            const u32 *arr = p.c{c}_arr + (size_t)(n & p.c{c}_arr_mask) * p.c{c}_arr_words;
+            const int seg = (c{c}_w1 - c{c}_w0 + SCAN - 1) / SCAN;
+            const int a = min(c{c}_w1, c{c}_w0 + sc * seg), b = min(c{c}_w1, a + seg);
+            u32 (&x)[4] = x{c};
+{_first_words('arr', 'a', 'b', 12)}        }}
 """
+    return out
 
 
 def _prefetch(c: int, inc: dict) -> str:
@@ -330,21 +358,24 @@ def _rows_loop(rows: str) -> str:
 
 
 def _deliver_code(n_out: int) -> str:
-    """The block's deliveries: every (spike, connection) row is walked by one warp or, with fewer rows than warps, by
-    a group of them, so that a row of 1,000 links is a few loads per lane whatever the block's spikes."""
+    """The block's deliveries: its spikes' rows in pieces of PIECE links, dealt out to its warps in turn, so that two
+    or three spikes in one block (the step's slowest) are still a piece or two per warp."""
     if not n_out:
         return ""
-    rows = ("const int r0 = o < OUT_CACHED ? s.optr[o][q] : O.ptr[jq], r1 = o < OUT_CACHED ? s.optr[o][q + 1] : "
-            "O.ptr[jq + 1];" if n_out > OUT_CACHED else "const int r0 = s.optr[o][q], r1 = s.optr[o][q + 1];")
-    return f"""        // the spikes' outgoing rows
-{_rows_loop(f"__popc(fw) * {n_out}")}            const int o = i % {n_out};
-            u32 m = fw;
-            for (int k = i / {n_out}; k > 0; --k) m &= m - 1;
-            const int q = __ffs(m) - 1, jq = blk * NPB_C + q;
-            const N2Out &O = p.outs[o];
-            {rows}
-            n2_deliver(O, n, r0, r1, (int)threadIdx.x % (32 * g), 32 * g);
-        }}
+    rows = ("const int r0 = o < OUT_CACHED ? s.optr[o][q] : O.ptr[blk * NPB_C + q], r1 = o < OUT_CACHED ? "
+            "s.optr[o][q + 1] : O.ptr[blk * NPB_C + q + 1];"
+            if n_out > OUT_CACHED else "const int r0 = s.optr[o][q], r1 = s.optr[o][q + 1];")
+    return f"""        int turn = (int)(threadIdx.x >> 5);  // the spikes' outgoing rows: this warp's next piece
+        for (u32 m = fw; m; m &= m - 1) {{
+            const int q = __ffs(m) - 1;
+            for (int o = 0; o < {n_out}; ++o) {{
+                const N2Out &O = p.outs[o];
+                {rows}
+                const int pieces = (r1 - r0 + PIECE - 1) / PIECE;
+                for (; turn < pieces; turn += {THREADS // 32})
+                    n2_deliver(O, n, r0 + turn * PIECE, min(r1, r0 + (turn + 1) * PIECE));
+                turn -= pieces;
+            }}
         }}
 """
 
@@ -416,19 +447,20 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
     shared = backward and not any(inc.get("backward_writes", True) for _, inc in backward)
     read = [a for a in attrs if any(f"s_{a}" in _backward_body(pop_name, c, inc) for c, inc in backward)] if shared else []
     src += [f"    __shared__ {ctype_of(attrs[a])[0]} n2d_{a}[NPB_C];\n" for a in read]
-    src.append("""    for (int step = 0;; ++step, ++n) {
+    src.append("""    u64 spikes = 0, events = 0;  // the block's, counted by its first thread
+    for (int step = 0;; ++step, ++n) {
         const float t = WINDOW ? (float)((double)(n + 1) * dt) : p.t, t0 = WINDOW ? (float)((double)n * dt) : p.t0;
         bool fired = false;
         float spike_t = t;
         u32 arrived = 0;
         u32 link_k = 0xFFFFFFu;
-        if (threadIdx.x == 0) {
+@WORDS@        if (threadIdx.x == 0) {
             s.word = 0u;
             s.arrivals = 0u;
             if (p.bad && blk == 0) atomicAdd(p.err, p.bad);
         }
         __syncthreads();
-""")
+""".replace("@WORDS@", _words_ahead(incoming)))
     if exact:
         src.append("        int na = 0;  // the neuron's arrivals of the step\n")
         src += [_exact_collect(c, inc) for c, inc in enumerate(incoming) if takes(inc)]
@@ -469,8 +501,8 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
                 const long long r = n - p.rec0;
                 if (p.raster && r >= 0 && r < p.raster_steps) p.raster[(size_t)r * p.words + blk] = fw;
             }
-            if (fw) atomicAdd(p.counters + 1, (u64)__popc(fw));
-            if (s.arrivals) atomicAdd(p.counters, (u64)s.arrivals);
+            spikes += __popc(fw);
+            events += s.arrivals;
         }
 """)
     src.append(_deliver_code(n_out))
@@ -490,7 +522,7 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
     }
 """)
     src += [f"    if (live && own) p.s_{a}[j] = s_{a};\n" for a in attrs]
-    src.append("}\n")
+    src.append("    if (spikes) atomicAdd(p.counters + 1, spikes);\n    if (events) atomicAdd(p.counters, events);\n}\n")
     return "".join(src)
 
 

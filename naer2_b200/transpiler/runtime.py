@@ -107,7 +107,7 @@ def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -
     """The arrival bits of one connection, from its pull CSR: `wptr` int32 [n_tgt + 1], each row's first word in a
     slot; `words` per slot; `depth`, the slots (a power of two above every delay); the outgoing rows `out_ptr`
     int32 [n_src + 1], `pos` int32 (uint32 bits: the link's bit in a slot) and `dly` uint8, links of a source in
-    pull order; `bad`: links whose source or delay (1 .. mask) is out of range, in no outgoing row."""
+    pull order -- with at most 2^24 bits to a slot the delay is in the top 8 bits of `pos` and `dly` is None; `bad`: links whose source or delay (1 .. mask) is out of range, in no outgoing row."""
     dev = link.device
     n_tgt = len(ptr) - 1
     ptr = ptr.to(torch.int64)
@@ -127,11 +127,14 @@ def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -
     out_ptr[1:] = torch.cumsum(torch.bincount(src, minlength=n_src)[:n_src], 0)
     dly = dly[order]
     top = int(dly.max()) if dly.numel() else 1
-    pos = pos[order]
-    return {"wptr": wptr.to(torch.int32), "words": int(wptr[-1]), "depth": 1 << top.bit_length(),
+    pos, words = pos[order], int(wptr[-1])
+    packed = 32 * words <= 1 << 24
+    if packed:
+        pos = pos | (dly.to(torch.int64) << 24)
+    return {"wptr": wptr.to(torch.int32), "words": words, "depth": 1 << top.bit_length(),
             "out_ptr": out_ptr.to(torch.int32),
-            "pos": torch.where(pos >= 2 ** 31, pos - 2 ** 32, pos).to(torch.int32), "dly": dly.to(torch.uint8),
-            "bad": bad}
+            "pos": torch.where(pos >= 2 ** 31, pos - 2 ** 32, pos).to(torch.int32),
+            "dly": None if packed else dly.to(torch.uint8), "bad": bad}
 
 
 def plan_of(net) -> dict:
@@ -355,7 +358,7 @@ class JitRuntime:
                     f = arrival_form(ptr, c["link"].to(dev), plan["pops"][s]["n"], depth[s] - 1)
                     bad += f["bad"]
                     f["arr"] = torch.zeros(max(1, f["depth"] * f["words"]), dtype=torch.int32, device=dev)
-                    self.keep += [f[x] for x in ("wptr", "out_ptr", "pos", "dly", "arr")]
+                    self.keep += [f[x] for x in ("wptr", "out_ptr", "pos", "dly", "arr")]  # (dly may be None)
                     setattr(P, f"c{ci}_wptr", f["wptr"].data_ptr())
                     setattr(P, f"c{ci}_arr", f["arr"].data_ptr())
                     setattr(P, f"c{ci}_arr_words", f["words"])
@@ -371,7 +374,8 @@ class JitRuntime:
         for P, pp in zip(self.params, plan["pops"]):
             for o, (tgt, ci) in enumerate(pp.get("outs", ())):
                 f = forms[tgt][ci]
-                P.outs[o] = arrival.Out(ptr=f["out_ptr"].data_ptr(), pos=f["pos"].data_ptr(), dly=f["dly"].data_ptr(),
+                P.outs[o] = arrival.Out(ptr=f["out_ptr"].data_ptr(), pos=f["pos"].data_ptr(),
+                                        dly=f["dly"].data_ptr() if f["dly"] is not None else None,
                                         arr=f["arr"].data_ptr(), words=f["words"], mask=f["depth"] - 1)
         self.window = self.window_kernel = None  # the window kernel and its parameter block
         self.window_grid = sum(arrival.blocks_of(p["n"]) for p in plan["pops"])

@@ -33,7 +33,9 @@ def test_arrival_form_gives_every_link_a_bit_of_its_own(n_src, n_tgt, longest, m
     good = np.ones(n, bool)
     good[:bad] = False
     out_src = np.repeat(np.arange(n_src), np.diff(f["out_ptr"].numpy()))
-    got = list(zip(out_src, f["dly"].numpy().astype(int), f["pos"].numpy().view(np.uint32).astype(int)))
+    got_pos = f["pos"].numpy().view(np.uint32).astype(np.int64)
+    got_dly = got_pos >> 24 if f["dly"] is None else f["dly"].numpy()  # at most 2^24 bits to a slot: packed
+    got = list(zip(out_src, got_dly, got_pos & 0xFFFFFF if f["dly"] is None else got_pos))
     assert sorted(got) == sorted(zip(src[good], dly[good], pos[good]))
     top = int(dly[good].max()) if good.any() else 1
     assert f["depth"] > top and f["depth"] & (f["depth"] - 1) == 0

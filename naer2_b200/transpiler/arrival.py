@@ -19,8 +19,8 @@ neurons' state in registers and its row bounds throughout, and the steps are sep
 wait that gives up sets an abort word, and the kernel winds down). A step is a chain of memory latencies, so what it
 costs is the launches around it and the loads that a launch starts with. Measured, us per step, links looked up ->
 arrival bits, one launch per population -> window: 12,500 neurons of 1,250 links (47 spikes a step) 92 -> 19.4 ->
-8.3; 1,501 neurons of 150 plastic links 33 -> 11.2 -> 6.8; 3,001 event-driven neurons of 125 links 73 -> 36 ->
-14.5.
+7.5; 1,501 neurons of 150 plastic links 33 -> 11.2 -> 6.1; 3,001 event-driven neurons of 125 links 73 -> 36 ->
+11.6.
 """
 
 from __future__ import annotations
@@ -30,9 +30,11 @@ import ctypes
 from .cuda import lower_hook
 from .template import _PRELUDE, MAX_ARRIVALS, NPB_C, UNIFORM, _arrival_body, base_fields, ctype_of
 
-SCAN = 8  # threads per neuron: a row of 1,250 links is 40 words, five to a thread
+SCAN = 8  # threads per neuron: a row of 1,000 links is 32 words, four to a thread
 THREADS = NPB_C * SCAN
-CAP = 16  # clocked intake: arrivals a thread lists of one connection (more stay in their words for the owner)
+CHUNK = 4 * SCAN  # words of a row taken at once, four to a thread
+EDGE_CAP = {False: 16, True: MAX_ARRIVALS}  # arrivals whose edge values are loaded ahead of their hooks (by exact)
+EDGE_ATTRS = {False: 8, True: 2}  # ... of at most so many edge attributes
 OUT_CACHED = 8  # outgoing connections whose row bounds a block holds in shared memory
 PIECE = 256  # links of a row that a warp delivers at once, eight loads a lane in flight
 WORDS_AHEAD = 4  # incoming connections whose arrival words are loaded together at a step's start
@@ -45,14 +47,15 @@ struct N2Out {
     const int *ptr;            // rows per source neuron
     const u32 *pos;            // per link: its bit among a slot's words (dly null: its delay in the top 8 bits)
     const unsigned char *dly;  // per link: its delay in steps, of connections with more than 2^24 bits to a slot
-    u32 *arr;                  // the arrival bits, [mask + 1][words]
+    u32 *arr;                  // the arrival bits, [depth][words]
     long long words;
-    int mask, pad;
+    int depth, pad;            // slots: the largest delay + 1 (step n's is n mod depth)
 };
 
-constexpr int SCAN = @SCAN@, NPB_C = @NPB@, CAP = @CAP@, MAX_ARRIVALS = @MAXA@, OUT_CACHED = @OUTC@, PIECE = @PIECE@;
+constexpr int SCAN = @SCAN@, NPB_C = @NPB@, CHUNK = 4 * SCAN, MAX_ARRIVALS = @MAXA@, OUT_CACHED = @OUTC@, PIECE = @PIECE@;
+constexpr int EDGE_CAP = @ECAP@;
 
-// A block's shared scratch. Clocked: the arrivals that each thread listed; exact times: each neuron's arrivals.
+// A block's shared scratch. Clocked: each neuron's arrival words of a chunk; exact times: each neuron's arrivals.
 struct N2Scratch {
     u32 word, arrivals;
     int optr[OUT_CACHED][NPB_C + 1];
@@ -63,6 +66,7 @@ struct N2Scratch {
 // One warp, the links r0 .. r1 (at most PIECE) of a row: set each one's bit in the arrival slot of its step. Every
 // link's load is in flight before the first reduction: a row is a chain of memory latencies, not of bandwidth.
 __device__ __forceinline__ void n2_deliver(const N2Out &o, long long n, int r0, int r1) {
+    const u32 now = (u32)((u64)n % (u32)o.depth);
     u32 pos[PIECE / 32], d[PIECE / 32];
     const int l0 = r0 + (int)(threadIdx.x & 31);
     if (o.dly) {
@@ -83,7 +87,10 @@ __device__ __forceinline__ void n2_deliver(const N2Out &o, long long n, int r0, 
     }
     #pragma unroll
     for (int k = 0; k < PIECE / 32; ++k)
-        if (d[k]) atomicOr(o.arr + (size_t)((n + d[k]) & o.mask) * o.words + (pos[k] >> 5), 1u << (pos[k] & 31u));
+        if (d[k]) {
+            const u32 slot = now + d[k] < (u32)o.depth ? now + d[k] : now + d[k] - (u32)o.depth;
+            atomicOr(o.arr + (size_t)slot * o.words + (pos[k] >> 5), 1u << (pos[k] & 31u));
+        }
 }
 
 // The grid barrier of a window: `bar[0]` counts arrivals, `bar[32]` is set when a wait gave up (bar[33]: how many).
@@ -128,7 +135,7 @@ __device__ __forceinline__ bool n2_grid_sync(const N2Grid &g, int k) {
 }
 '''
 
-_LISTS = {False: "    u32 list[NPB_C * SCAN * CAP];\n    int cnt[NPB_C * SCAN];",
+_LISTS = {False: "    u32 words[NPB_C][CHUNK];",
           True: "    float a_t[NPB_C][MAX_ARRIVALS];\n    int a_l[NPB_C][MAX_ARRIVALS];\n"
                 "    unsigned short a_c[NPB_C][MAX_ARRIVALS];\n    unsigned char a_o[NPB_C][MAX_ARRIVALS];"}
 
@@ -136,7 +143,7 @@ _LISTS = {False: "    u32 list[NPB_C * SCAN * CAP];\n    int cnt[NPB_C * SCAN];"
 class Out(ctypes.Structure):
     """One outgoing connection (the source's N2Out)."""
     _fields_ = [("ptr", ctypes.c_void_p), ("pos", ctypes.c_void_p), ("dly", ctypes.c_void_p),
-                ("arr", ctypes.c_void_p), ("words", ctypes.c_int64), ("mask", ctypes.c_int32),
+                ("arr", ctypes.c_void_p), ("words", ctypes.c_int64), ("depth", ctypes.c_int32),
                 ("pad", ctypes.c_int32)]
 
 
@@ -146,11 +153,19 @@ class Grid(ctypes.Structure):
                 ("pad", ctypes.c_uint32)]
 
 
-def common(exact: bool) -> str:
-    text = _COMMON.replace("@LISTS@", _LISTS[exact])
-    for key, v in (("SCAN", SCAN), ("NPB", NPB_C), ("CAP", CAP), ("MAXA", MAX_ARRIVALS), ("OUTC", OUT_CACHED), ("PIECE", PIECE)):
+def common(exact: bool, edges: int) -> str:
+    """The text shared by a network's populations; edges: edge attributes held in the scratch (`staged`)."""
+    lists = _LISTS[exact] + (f"\n    float e[{edges}][NPB_C][EDGE_CAP];" if edges else "")
+    text = _COMMON.replace("@LISTS@", lists)
+    for key, v in (("SCAN", SCAN), ("NPB", NPB_C), ("MAXA", MAX_ARRIVALS), ("OUTC", OUT_CACHED), ("PIECE", PIECE),
+                   ("ECAP", EDGE_CAP[exact])):
         text = text.replace(f"@{key}@", str(v))
     return text
+
+
+def staged(incoming: list, exact: bool) -> int:
+    """Edge attributes of these connections whose values are loaded ahead of the hooks, at most EDGE_ATTRS."""
+    return min(EDGE_ATTRS[exact], max((len(inc["edge_dynamic"]) for inc in incoming if takes(inc)), default=0))
 
 
 def indent(text: str, pad: int) -> str:
@@ -168,128 +183,149 @@ def _row_bounds(c: int) -> str:
             f"c{c}_w1 = live ? p.c{c}_wptr[j + 1] : 0;\n")
 
 
-def _words_of(c: int) -> str:
-    """The row's bounds, its slot, and this thread's run of its words."""
+def _chunk_head(c: int) -> str:
+    """The loop over a row's words in chunks (the same number of them for the whole warp): word kb + SCAN i + sc is
+    x[i] of the neuron's thread sc, four loads in flight; the first connections' first chunk is loaded already."""
     again = "" if c < ROWS_AHEAD else f"            const int {_row_bounds(c)}"
+    if c >= ROWS_AHEAD:
+        again += f"            const int c{c}_rounds = {_rounds(c)};\n"
+    first = f"x{c}[i]" if c < WORDS_AHEAD else "w0 + SCAN * i + sc < w1 ? __ldcg(arr + w0 + SCAN * i + sc) : 0u"
     return f"""{again}            const int r0 = c{c}_r0, w0 = c{c}_w0, w1 = c{c}_w1;
-            u32 *arr = p.c{c}_arr + (size_t)(n & p.c{c}_arr_mask) * p.c{c}_arr_words;
-            const int seg = (w1 - w0 + SCAN - 1) / SCAN;
-            const int a = min(w1, w0 + sc * seg), b = min(w1, a + seg);
-""" + (f"            u32 (&x)[4] = x{c};\n" if c < WORDS_AHEAD else f"            u32 x[4];\n{_first_words('arr', 'a', 'b', 12)}")
+            u32 *arr = p.c{c}_arr + (size_t)slot{c} * p.c{c}_arr_words;
+            u32 x[4];
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = {first};
+            for (int kb = 0, round = 0; round < c{c}_rounds; ++round, kb += CHUNK) {{
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) {{
+                    const int k = w0 + kb + SCAN * i + sc;
+                    if (round) x[i] = k < w1 ? __ldcg(arr + k) : 0u;
+                    if (x[i]) arr[k] = 0u;
+                }}
+"""
 
 
-def _first_words(arr: str, a: str, b: str, pad: int) -> str:
-    return (" " * pad + "#pragma unroll\n" + " " * pad +
-            f"for (int i = 0; i < 4; ++i) x[i] = {a} + i < {b} ? __ldcg({arr} + {a} + i) : 0u;\n")
+def _rounds(c: int) -> str:
+    return f"(int)(__reduce_max_sync(0xffffffffu, (u32)(c{c}_w1 - c{c}_w0)) + CHUNK - 1) / CHUNK"
 
 
 def _words_ahead(incoming: list) -> str:
     """The first connections' first words, loaded together: their latencies overlap."""
-    out = ""
-    for c, inc in enumerate(incoming[:WORDS_AHEAD]):
-        if takes(inc):
-            out += f"""        u32 x{c}[4];
+    return "".join(f"""        u32 x{c}[4];
         {{
-            const u32 *arr = p.c{c}_arr + (size_t)(n & p.c{c}_arr_mask) * p.c{c}_arr_words;
-            const int seg = (c{c}_w1 - c{c}_w0 + SCAN - 1) / SCAN;
-            const int a = min(c{c}_w1, c{c}_w0 + sc * seg), b = min(c{c}_w1, a + seg);
-            u32 (&x)[4] = x{c};
-{_first_words('arr', 'a', 'b', 12)}        }}
+            const u32 *arr = p.c{c}_arr + (size_t)slot{c} * p.c{c}_arr_words + c{c}_w0;
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) x{c}[i] = SCAN * i + sc < c{c}_w1 - c{c}_w0 ? __ldcg(arr + SCAN * i + sc) : 0u;
+        }}
+""" for c, inc in enumerate(incoming[:WORDS_AHEAD]) if takes(inc))
+
+
+# Each thread's first arrival (start[i]) of its word i among the neuron's arrivals of the chunk, in word order, and
+# their number (total): counts of two words to a register, scanned over the neuron's threads.
+_RANKS = """                u32 n01 = __popc(x[0]) | __popc(x[1]) << 16, n23 = __popc(x[2]) | __popc(x[3]) << 16;
+                const u32 own01 = n01, own23 = n23;
+                #pragma unroll
+                for (int o = 1; o < SCAN; o <<= 1) {
+                    const u32 u01 = __shfl_up_sync(0xffffffffu, n01, o, SCAN), u23 = __shfl_up_sync(0xffffffffu, n23, o, SCAN);
+                    if (sc >= o) { n01 += u01; n23 += u23; }
+                }
+                const u32 t01 = __shfl_sync(0xffffffffu, n01, SCAN - 1, SCAN), t23 = __shfl_sync(0xffffffffu, n23, SCAN - 1, SCAN);
+                n01 -= own01;
+                n23 -= own23;
+                const int h0 = t01 & 0xFFFFu, h1 = h0 + (t01 >> 16), h2 = h1 + (t23 & 0xFFFFu), total = h2 + (t23 >> 16);
+                const int start[4] = {(int)(n01 & 0xFFFFu), h0 + (int)(n01 >> 16), h1 + (int)(n23 & 0xFFFFu), h2 + (int)(n23 >> 16)};
 """
-    return out
 
 
-def _prefetch(c: int, inc: dict) -> str:
-    """The listed link's edge values towards the SM, ahead of the owner's loads."""
-    return "".join(f'asm volatile("prefetch.global.L1 [%0];" ::"l"(p.c{c}_e_{e} + l)); ' for e in inc["edge_dynamic"])
+def _stage_edges(c: int, inc: dict, exact: bool, at: str, pad: int) -> str:
+    """The edge values of link l into the scratch's place `at`."""
+    return "".join(" " * pad + f"s.e[{a}][jl][{at}] = p.c{c}_e_{e}[l];\n"
+                   for a, e in enumerate(inc["edge_dynamic"][:EDGE_ATTRS[exact]]))
 
 
-def _clocked_intake(c: int, inc: dict, arrival: str) -> str:
-    """Connection c's arrivals: each of the neuron's SCAN threads (neighbouring lanes of a warp) lists the links of
-    its words' set bits and clears them, as long as its list holds a whole word's; the words after that stay set for
-    the owner, which runs the hooks over the lists in word order and then over such words, i.e. in link order."""
+def _clocked_intake(c: int, inc: dict, body: str) -> str:
+    """Connection c's arrivals: the neuron's threads put their words with a set bit into shared memory and clear
+    them; the neuron's first thread (the owner) runs the hooks over the words' bits, i.e. in link order. Edge values
+    are loaded by the threads together, ahead of the owner's chain of hooks (of the chunk's first EDGE_CAP arrivals)."""
+    edges = inc["edge_dynamic"]
+    stage, loads = "", ""
+    if edges:
+        stage = _RANKS + f"""                #pragma unroll
+                for (int i = 0; i < 4; ++i) {{
+                    int at = start[i];
+                    for (u32 v = x[i]; v && at < EDGE_CAP; v &= v - 1, ++at) {{
+                        const int l = r0 + 32 * (kb + SCAN * i + sc) + __ffs(v) - 1;
+{_stage_edges(c, inc, False, "at", 24)}                    }}
+                }}
+"""
+        for a, e in enumerate(edges):
+            loads += (f"float e_{e} = at < EDGE_CAP ? s.e[{a}][jl][at] : p.c{c}_e_{e}[l];\n" if a < EDGE_ATTRS[False]
+                      else f"float e_{e} = p.c{c}_e_{e}[l];\n")
+    run = loads + ("++at;\n" if edges else "") + "link_k = arrived++;\n{\n" + body + "}\n"
     return f"""        {{  // connection {c}
-{_words_of(c)}            u32 *list = s.list + (jl * SCAN + sc) * CAP;
-            int cnt = 0;
-            bool left = false;  // words left for the owner
-            for (int k = a; k < b; k += 4) {{
+{_chunk_head(c)}{stage}                u32 some = 0u;  // the neuron's words of the chunk with a set bit
                 #pragma unroll
                 for (int i = 0; i < 4; ++i) {{
-                    if (k > a) x[i] = k + i < b ? __ldcg(arr + k + i) : 0u;
-                    left = left || (x[i] && cnt + __popc(x[i]) > CAP);
-                    if (!x[i] || left) continue;
-                    for (u32 v = x[i]; v; v &= v - 1) {{
-                        const int l = r0 + 32 * (k + i - w0) + __ffs(v) - 1;
-                        list[cnt++] = (u32)l;
-                        {_prefetch(c, inc)}
-                    }}
-                    arr[k + i] = 0u;
+                    some |= ((__ballot_sync(0xffffffffu, x[i] != 0u) >> (threadIdx.x & 31 & ~(SCAN - 1))) & ((1u << SCAN) - 1)) << (SCAN * i);
+                    if (x[i]) s.words[jl][SCAN * i + sc] = x[i];
                 }}
-            }}
-            s.cnt[jl * SCAN + sc] = left ? ~cnt : cnt;
-            const u32 some = __ballot_sync(0xffffffffu, cnt || left);
-            __syncwarp();
-            if (live && own) {{  // the hooks, in link order
-                for (u32 segs = (some >> (threadIdx.x & 31)) & ((1u << SCAN) - 1); segs; segs &= segs - 1) {{
-                    const int q = __ffs(segs) - 1;
-                    const int cs = s.cnt[jl * SCAN + q], listed = cs < 0 ? ~cs : cs;
-                    for (int i = 0; i < listed; ++i) {{
-                        const int l = (int)s.list[(jl * SCAN + q) * CAP + i];
-                        {indent(arrival, 24)}                    }}
-                    if (cs >= 0) continue;
-                    const int as = min(w1, w0 + q * seg), bs = min(w1, as + seg);
-                    for (int k = as; k < bs; ++k) {{
-                        u32 v = __ldcg(arr + k);  // (the listed words are clear)
-                        if (v) arr[k] = 0u;
-                        for (; v; v &= v - 1) {{
-                            const int l = r0 + 32 * (k - w0) + __ffs(v) - 1;
-                            {indent(arrival, 28)}                        }}
+                __syncwarp();
+                if (own) {{  // the hooks, in link order
+                    {"int at = 0;" if edges else ""}
+                    for (; some; some &= some - 1) {{
+                        const int k = __ffs(some) - 1;
+                        for (u32 v = s.words[jl][k]; v; v &= v - 1) {{
+                            const int l = r0 + 32 * (kb + k) + __ffs(v) - 1;
+                            {indent(run, 28)}                        }}
                     }}
                 }}
+                __syncwarp();  // the words are rewritten by the next chunk
             }}
             link_k = 0xFFFFFFu;
-            __syncwarp();  // the lists are rewritten by the next connection
         }}
 """
 
 
 def _exact_collect(c: int, inc: dict) -> str:
-    """Connection c's arrivals of the step into the neuron's list, in link order, with their times; past
-    MAX_ARRIVALS they are counted and dropped."""
+    """Connection c's arrivals of the step into the neuron's list, in link order; past MAX_ARRIVALS they are counted
+    and dropped."""
     return f"""        {{  // connection {c}
-{_words_of(c)}            int mine = 0;
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) mine += __popc(x[i]);
-            for (int k = a + 4; k < b; ++k) mine += __popc(__ldcg(arr + k));
-            int at = mine;
-            #pragma unroll
-            for (int o = 1; o < SCAN; o <<= 1) {{
-                const int v = __shfl_up_sync(0xffffffffu, at, o, SCAN);
-                if (sc >= o) at += v;
-            }}
-            const int total = __shfl_sync(0xffffffffu, at, SCAN - 1, SCAN);
-            at += na - mine;
-            na += total;
-            for (int k = a; mine > 0 && k < b; ++k) {{
-                u32 v = k - a < 4 ? (k - a < 2 ? (k == a ? x[0] : x[1]) : (k - a == 2 ? x[2] : x[3])) : __ldcg(arr + k);
-                if (v) arr[k] = 0u;
-                for (; v; v &= v - 1, ++at) {{
-                    if (at >= MAX_ARRIVALS) {{ atomicAdd(p.err, 1); continue; }}
-                    const int l = r0 + 32 * (k - w0) + __ffs(v) - 1;
-                    const u32 w = __ldg(p.c{c}_link + l);
-                    {_prefetch(c, inc)}
-                    const int src = (int)(w & 0xFFFFFFu), d = (int)(w >> 24);
-                    s.a_t[jl][at] = t0 + __ldcg(p.c{c}_src_off + (size_t)((n - d) & p.c{c}_src_mask) * p.c{c}_src_n + src);
-                    s.a_l[jl][at] = l;
-                    s.a_c[jl][at] = {c};
+{_chunk_head(c)}{_RANKS}                #pragma unroll
+                for (int i = 0; i < 4; ++i) {{
+                    int at = na + start[i];
+                    for (u32 v = x[i]; v; v &= v - 1, ++at) {{
+                        if (at >= MAX_ARRIVALS) {{ atomicAdd(p.err, 1); continue; }}
+                        s.a_l[jl][at] = r0 + 32 * (kb + SCAN * i + sc) + __ffs(v) - 1;
+                        s.a_c[jl][at] = {c};
+                    }}
                 }}
+                na += total;
+            }}
+        }}
+"""
+
+
+def _exact_times(incoming: list) -> str:
+    """The listed arrivals' times and edge values: the SCAN threads take one each, so that their loads (the link, then
+    its source's spike) overlap."""
+    cases = "".join(f"""                case {c}: {{
+                    const u32 w = __ldg(p.c{c}_link + l);
+{_stage_edges(c, inc, True, "e", 20)}                    const int src = (int)(w & 0xFFFFFFu), d = (int)(w >> 24);
+                    s.a_t[jl][e] = t0 + __ldcg(p.c{c}_src_off + (size_t)((n - d) & p.c{c}_src_mask) * p.c{c}_src_n + src);
+                }} break;
+""" for c, inc in enumerate(incoming) if takes(inc))
+    return f"""        na = min(na, MAX_ARRIVALS);
+        __syncwarp();
+        for (int e = sc; e < na; e += SCAN) {{
+            const int l = s.a_l[jl][e];
+            switch (s.a_c[jl][e]) {{
+{cases}                default: break;
             }}
         }}
 """
 
 
 _EXACT_SORT = """        // by time, equal times in the order they were listed: each arrival's rank, the SCAN threads together
-        na = min(na, MAX_ARRIVALS);
         __syncwarp();
         bool odd = false;  // (a time that is not a number has no rank)
         for (int e = sc; e < na; e += SCAN) {
@@ -314,12 +350,16 @@ _EXACT_SORT = """        // by time, equal times in the order they were listed: 
 """
 
 
+def _exact_loads(c: int, inc: dict) -> str:
+    return "".join(f"float e_{e} = s.e[{a}][jl][o];\n" if a < EDGE_ATTRS[True] else f"float e_{e} = p.c{c}_e_{e}[l];\n"
+                   for a, e in enumerate(inc["edge_dynamic"]))
+
+
 def _exact_deliver(pop_name: str, incoming: list, hooks: dict) -> str:
     """The owner: receive (and edge forward) for each arrival at its own time, send after each group of equal ones."""
     cases = "".join(
         f"""                    case {c}: {{
-                        {indent("".join(f"float e_{e} = p.c{c}_e_{e}[l];" + chr(10) for e in inc["edge_dynamic"])
-                                + _arrival_body(pop_name, c, inc), 24)}                    }} break;
+                        {indent(_exact_loads(c, inc) + _arrival_body(pop_name, c, inc), 24)}                    }} break;
 """ for c, inc in enumerate(incoming) if takes(inc))
     fn, ctx = hooks["send"]
     return f"""        if (live && own) {{
@@ -401,7 +441,7 @@ def params_fields(attrs: dict, incoming: list, n_out: int, exact: bool) -> list:
     for c, inc in enumerate(incoming):
         fields += [(f"c{c}_ptr", "const int *", ctypes.c_void_p), (f"c{c}_wptr", "const int *", ctypes.c_void_p),
                    (f"c{c}_arr", "u32 *", ctypes.c_void_p), (f"c{c}_arr_words", "long long", ctypes.c_int64),
-                   (f"c{c}_arr_mask", "int", ctypes.c_int32)]
+                   (f"c{c}_arr_depth", "int", ctypes.c_int32)]
         if exact:
             fields += [(f"c{c}_link", "const u32 *", ctypes.c_void_p),
                        (f"c{c}_src_off", "const float *", ctypes.c_void_p),
@@ -432,7 +472,8 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
     # what no launch writes, then (one step per launch) the launch before this one: the next launch may be scheduled
     # and the row bounds loaded while it is still running
     src.append('    if (!WINDOW) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");\n')
-    src += [f"    const int {_row_bounds(c)}" for c, inc in enumerate(incoming[:ROWS_AHEAD]) if takes(inc)]
+    src += [f"    const int {_row_bounds(c)}    const int c{c}_rounds = {_rounds(c)};\n"
+            for c, inc in enumerate(incoming[:ROWS_AHEAD]) if takes(inc)]
     if n_out:
         src.append(f"""    for (int k = threadIdx.x; k < {min(n_out, OUT_CACHED)} * (NPB_C + 1); k += {THREADS}) {{
         const int q = k % (NPB_C + 1);
@@ -447,6 +488,8 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
     shared = backward and not any(inc.get("backward_writes", True) for _, inc in backward)
     read = [a for a in attrs if any(f"s_{a}" in _backward_body(pop_name, c, inc) for c, inc in backward)] if shared else []
     src += [f"    __shared__ {ctype_of(attrs[a])[0]} n2d_{a}[NPB_C];\n" for a in read]
+    # each connection's slot of the step, kept as the steps go on
+    src += [f"    int slot{c} = (int)((u64)n % (u32)p.c{c}_arr_depth);\n" for c, inc in enumerate(incoming) if takes(inc)]
     src.append("""    u64 spikes = 0, events = 0;  // the block's, counted by its first thread
     for (int step = 0;; ++step, ++n) {
         const float t = WINDOW ? (float)((double)(n + 1) * dt) : p.t, t0 = WINDOW ? (float)((double)n * dt) : p.t0;
@@ -465,13 +508,11 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
         src.append("        int na = 0;  // the neuron's arrivals of the step\n")
         src += [_exact_collect(c, inc) for c, inc in enumerate(incoming) if takes(inc)]
         if any(takes(inc) for inc in incoming):
-            src += [_EXACT_SORT, _exact_deliver(pop_name, incoming, hooks)]
+            src += [_exact_times(incoming), _EXACT_SORT, _exact_deliver(pop_name, incoming, hooks)]
     else:
         for c, inc in enumerate(incoming):
             if takes(inc):
-                loads = "".join(f"float e_{e} = p.c{c}_e_{e}[l];\n" for e in inc["edge_dynamic"])
-                body = "link_k = arrived++;\n{\n" + _arrival_body(pop_name, c, inc) + "}\n"
-                src.append(_clocked_intake(c, inc, loads + body))
+                src.append(_clocked_intake(c, inc, _arrival_body(pop_name, c, inc)))
     src.append("        if (live && own) {\n")
     for name in ("update", "send"):
         fn, ctx = hooks[name]
@@ -519,8 +560,9 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
         src.append("        }\n        }\n")
     src.append("""        if (!WINDOW || step + 1 == n_steps) break;
         if (!n2_grid_sync(grid, step)) break;
-    }
 """)
+    src += [f"        if (++slot{c} == p.c{c}_arr_depth) slot{c} = 0;\n" for c, inc in enumerate(incoming) if takes(inc)]
+    src.append("    }\n")
     src += [f"    if (live && own) p.s_{a}[j] = s_{a};\n" for a in attrs]
     src.append("    if (spikes) atomicAdd(p.counters + 1, spikes);\n    if (events) atomicAdd(p.counters, events);\n}\n")
     return "".join(src)
@@ -540,16 +582,17 @@ def build(pop_name: str, attrs: dict, hooks: dict, incoming: list, n_out: int, e
     destination's state, and n_out: the population's outgoing connections."""
     fields = params_fields(attrs, incoming, n_out, exact)
     body = population(pop_name, attrs, hooks, incoming, n_out, exact, fields)
-    return _PRELUDE + common(exact) + body + STEP_KERNEL, fields, body
+    return _PRELUDE + common(exact, staged(incoming, exact)) + body + STEP_KERNEL, fields, body
 
 
 def blocks_of(n: int) -> int:
     return (n + NPB_C - 1) // NPB_C
 
 
-def window_source(exact: bool, bodies: list, sizes: list, per_sm: int) -> str:
-    """The window kernel over every population: `bodies` their `population` texts, `sizes` their neurons."""
-    src = [_PRELUDE, common(exact)]
+def window_source(exact: bool, bodies: list, sizes: list, edges: int, per_sm: int) -> str:
+    """The window kernel over every population: `bodies` their `population` texts, `sizes` their neurons, `edges` the
+    most edge attributes that one of them stages."""
+    src = [_PRELUDE, common(exact, edges)]
     src += [f"namespace n2p{k} {{\n{body}}}\n\n" for k, body in enumerate(bodies)]
     src.append("struct Window {\n    long long step0;\n    double dt;\n    N2Grid grid;\n    long long n_steps;\n")
     src += [f"    n2p{k}::Params p{k};\n" for k in range(len(bodies))]

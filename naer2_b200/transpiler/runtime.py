@@ -105,7 +105,8 @@ def arrival_bytes(n_tgt: int, n_links: int, depth: int) -> int:
 
 def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -> dict:
     """The arrival bits of one connection, from its pull CSR: `wptr` int32 [n_tgt + 1], each row's first word in a
-    slot; `words` per slot; `depth`, the slots (a power of two above every delay); the outgoing rows `out_ptr`
+    slot; `words` per slot; `depth`, the slots (the largest delay + 1: a slot is read
+    and cleared in the step before the first that can set it again); the outgoing rows `out_ptr`
     int32 [n_src + 1], `pos` int32 (uint32 bits: the link's bit in a slot) and `dly` uint8, links of a source in
     pull order -- with at most 2^24 bits to a slot the delay is in the top 8 bits of `pos` and `dly` is None; `bad`: links whose source or delay (1 .. mask) is out of range, in no outgoing row."""
     dev = link.device
@@ -131,7 +132,7 @@ def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -
     packed = 32 * words <= 1 << 24
     if packed:
         pos = pos | (dly.to(torch.int64) << 24)
-    return {"wptr": wptr.to(torch.int32), "words": words, "depth": 1 << top.bit_length(),
+    return {"wptr": wptr.to(torch.int32), "words": words, "depth": top + 1,
             "out_ptr": out_ptr.to(torch.int32),
             "pos": torch.where(pos >= 2 ** 31, pos - 2 ** 32, pos).to(torch.int32),
             "dly": None if packed else dly.to(torch.uint8), "bad": bad}
@@ -169,7 +170,7 @@ def plan_of(net) -> dict:
             outs[index[id(c._source)]].append([k, ci])
     arrivals = sum(arrival_bytes(len(p.shape), len(c.fabric.topology), depth[index[id(c._source)]])
                    for p, conns in zip(pops, incoming_of) for c in conns) <= ARRIVAL_BYTES
-    bodies = []  # arrival bits: the populations' part of the window kernel
+    bodies, edges = [], 0  # arrival bits: the populations' part of the window kernel, edge attributes they stage
     for k, p in enumerate(pops):
         node = p.node
         incoming = []
@@ -202,6 +203,7 @@ def plan_of(net) -> dict:
             src, fields, body = arrival.build(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
                                               len(outs[k]), exact)
             bodies.append(body)
+            edges = max(edges, arrival.staged(incoming, exact))
         else:
             src, fields = build_source(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
                                        exact=exact, n=len(p.shape))
@@ -227,7 +229,7 @@ def plan_of(net) -> dict:
     sizes = [len(p.shape) for p in pops]
     total = sum(arrival.blocks_of(n) for n in sizes)
     if arrivals and 0 < total <= WINDOW_BLOCKS and len(pops) <= arrival.WINDOW_POPS:
-        plan["window"] = arrival.window_source(exact, bodies, sizes, -(-total // WINDOW_SMS))
+        plan["window"] = arrival.window_source(exact, bodies, sizes, edges, -(-total // WINDOW_SMS))
     plan["device"] = dev
     return plan
 
@@ -362,7 +364,7 @@ class JitRuntime:
                     setattr(P, f"c{ci}_wptr", f["wptr"].data_ptr())
                     setattr(P, f"c{ci}_arr", f["arr"].data_ptr())
                     setattr(P, f"c{ci}_arr_words", f["words"])
-                    setattr(P, f"c{ci}_arr_mask", f["depth"] - 1)
+                    setattr(P, f"c{ci}_arr_depth", f["depth"])
                     forms[k].append(f)
                 for e, v in c["per_link"].items():
                     v = self._dev(v if v.numel() else torch.zeros(1))
@@ -376,7 +378,7 @@ class JitRuntime:
                 f = forms[tgt][ci]
                 P.outs[o] = arrival.Out(ptr=f["out_ptr"].data_ptr(), pos=f["pos"].data_ptr(),
                                         dly=f["dly"].data_ptr() if f["dly"] is not None else None,
-                                        arr=f["arr"].data_ptr(), words=f["words"], mask=f["depth"] - 1)
+                                        arr=f["arr"].data_ptr(), words=f["words"], depth=f["depth"])
         self.window = self.window_kernel = None  # the window kernel and its parameter block
         self.window_grid = sum(arrival.blocks_of(p["n"]) for p in plan["pops"])
         self.bar = torch.zeros(64, dtype=torch.int32, device=dev)  # its grid barrier: arrivals, abort word, stops

@@ -3,15 +3,24 @@ and on the GPU against the form that looks every link's source up (`ARRIVAL_BYTE
 give bit for bit: rows below, at and past a word's 32 links, more arrivals in one step than a thread's list or a
 neuron's event queue holds, plastic edges, exact times, and plans saved and loaded."""
 
+import itertools
+
 import numpy as np
 import pytest
 import torch
 
+from naer2_b200 import population
 from naer2_b200.patterns import fixed_indegree
 from naer2_b200.transpiler import JitRuntime, PlannedNetwork, load_plan, plan_of, save_plan
 from naer2_b200.transpiler import runtime as jit_runtime
 from naer2_b200.transpiler.runtime import arrival_bytes, arrival_form
 from tests.dsl_models import DecayLIF, JitterPacemaker, PairSTDP, Pacemaker, Syn, TraceLIF
+
+
+@pytest.fixture(autouse=True)
+def _own_seeds(monkeypatch):
+    """Populations made here draw their default seeds from a count of their own."""
+    monkeypatch.setattr(population, "_SEEDS", itertools.count(1 << 20))
 
 
 @pytest.mark.parametrize("n_src, n_tgt, longest, mask, bad", [(1, 1, 1, 1, 0), (7, 5, 0, 3, 0), (40, 30, 31, 15, 0),
@@ -38,8 +47,8 @@ def test_arrival_form_gives_every_link_a_bit_of_its_own(n_src, n_tgt, longest, m
     got = list(zip(out_src, got_dly, got_pos & 0xFFFFFF if f["dly"] is None else got_pos))
     assert sorted(got) == sorted(zip(src[good], dly[good], pos[good]))
     top = int(dly[good].max()) if good.any() else 1
-    assert f["depth"] > top and f["depth"] & (f["depth"] - 1) == 0
-    assert f["depth"] <= mask + 1 and 4 * f["depth"] * f["words"] + 5 * n <= arrival_bytes(n_tgt, n, mask + 1)
+    assert f["depth"] == top + 1
+    assert 4 * f["depth"] * f["words"] + 5 * n <= arrival_bytes(n_tgt, n, mask + 1)
 
 
 def _plastic(k, period):

@@ -167,9 +167,20 @@ struct n2b_net {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int32_t window = 0;
+    // steps without a grid barrier between them (chunk_kernel; 0: a barrier per step), its neurons per tile and tiles
+    int32_t chunk = 0, chunk_tn = 0, chunk_tiles = 0;
 };
 
 namespace {
+
+const void *chunk_kernel_of(int32_t tn) {
+    switch (tn) {
+        case 32: return (const void *)n2b::chunk_kernel<32>;
+        case 64: return (const void *)n2b::chunk_kernel<64>;
+        case 128: return (const void *)n2b::chunk_kernel<128>;
+        default: return (const void *)n2b::chunk_kernel<256>;
+    }
+}
 
 template <int NPB, bool INL>
 cudaError_t launch_one(n2b_net *net, int64_t n_steps, cudaStream_t s) {
@@ -200,8 +211,12 @@ cudaError_t launch_block(n2b_net *net, int64_t n_steps, cudaStream_t s) {
 
 cudaError_t launch_steps(n2b_net *net, int64_t n_steps, cudaStream_t s) {
     if (net->L.n_tiles > 0 && n_steps > 0) {
-        cudaError_t e = net->inl ? launch_block<true>(net, n_steps, s) : launch_block<false>(net, n_steps, s);
-        if (e != cudaSuccess) return e;
+        int32_t k = (int32_t)n_steps;
+        void *args[] = {(void *)&net->args, (void *)&k, (void *)&net->chunk, (void *)&net->chunk_tiles};
+        cudaError_t e = net->chunk ? cudaLaunchCooperativeKernel(chunk_kernel_of(net->chunk_tn), dim3(net->grid),
+                                                                 dim3(n2b::CHUNK_THREADS), args, 0, s)
+                        : net->inl ? launch_block<true>(net, n_steps, s) : launch_block<false>(net, n_steps, s);
+        if (e != cudaSuccess || net->chunk) return e;  // (a chunked window advances the counter itself)
     }
     n2b::advance_kernel<<<1, 1, 0, s>>>(reinterpret_cast<long long *>(net->ws + net->L.step), n_steps,
                                         reinterpret_cast<unsigned *>(net->ws + net->L.barrier));
@@ -237,6 +252,39 @@ int coresident_blocks(int32_t block, bool inl, bool dense, int device, size_t dy
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
     *out = per_sm * sms;
+    return N2B_OK;
+}
+
+// How many steps of a network of push connections need no grid barrier between them: the smallest delay of its
+// links, as far as every population's slots hold that many steps past its largest incoming delay; below 2, 0 (a
+// barrier per step, the deliveries of delay >= 2 spread over the grid). Reads the links once; the room of the push table,
+// not yet written, holds the ranges.
+int chunk_steps(const n2b_population *pops, int32_t n_pops, const std::vector<n2b::ConnDev> &push,
+                const std::vector<int32_t> &push_tgt, char *ws, const Layout &L, cudaStream_t s, int32_t *out) {
+    *out = 0;
+    std::vector<int32_t> range(2 * push.size());
+    for (size_t c = 0; c < push.size(); ++c) {
+        range[2 * c] = 255;
+        range[2 * c + 1] = 0;
+    }
+    if (!push.empty()) {
+        int32_t *dev = reinterpret_cast<int32_t *>(ws + L.push);
+        N2B_CUDA(cudaMemcpyAsync(dev, range.data(), sizeof(int32_t) * range.size(), cudaMemcpyHostToDevice, s));
+        for (size_t c = 0; c < push.size(); ++c)
+            if (push[c].n_links > 0)
+                n2b::delay_range_kernel<<<std::min((push[c].n_links + 255) / 256, 1184), 256, 0, s>>>(
+                    push[c].link, push[c].n_links, dev + 2 * c);
+        N2B_CUDA(cudaGetLastError());
+        N2B_CUDA(cudaMemcpyAsync(range.data(), dev, sizeof(int32_t) * range.size(), cudaMemcpyDeviceToHost, s));
+        N2B_CUDA(cudaStreamSynchronize(s));
+    }
+    int32_t k = n2b::CHUNK_MAX;
+    for (int32_t p = 0; p < n_pops; ++p)
+        if (pops[p].ext_len > 65536) k = 0;  // a chunk keeps its external counts in 16 bits
+    for (size_t c = 0; c < push.size(); ++c)
+        if (push[c].n_links > 0 && pops[push_tgt[c]].n > 0)
+            k = std::min(k, std::min(range[2 * c], pops[push_tgt[c]].acc_depth - range[2 * c + 1]));
+    if (k >= 2) *out = k;
     return N2B_OK;
 }
 
@@ -284,6 +332,7 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
     // host images of the tables
     std::vector<n2b::PopDev> pd(std::max(n_pops, 1));
     std::vector<n2b::ConnDev> push, pull;
+    std::vector<int32_t> push_tgt;
     std::vector<int4> tiles;
     for (int32_t p = 0; p < n_pops; ++p) {
         const n2b_population &P = pops[p];
@@ -342,7 +391,10 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
     for (int32_t p = 0; p < n_pops; ++p) {
         pd[p].out_first = (int32_t)push.size();
         for (int32_t c = 0; c < n_conns; ++c)
-            if (conns[c].mode == N2B_PUSH && conns[c].src == p) push.push_back(conn_dev(conns[c]));
+            if (conns[c].mode == N2B_PUSH && conns[c].src == p) {
+                push.push_back(conn_dev(conns[c]));
+                push_tgt.push_back(conns[c].tgt);
+            }
         pd[p].n_out = (int32_t)push.size() - pd[p].out_first;
         pd[p].pull_first = (int32_t)pull.size();
         for (int32_t c = 0; c < n_conns; ++c)
@@ -406,6 +458,14 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
             N2B_CUDA(cudaMemcpyAsync(pd[p].ext_tab, pops[p].ext_table, sizeof(uint32_t) * k, cudaMemcpyDeviceToHost, s));
     }
     N2B_CUDA(cudaStreamSynchronize(s));
+    const int persistent = opt && opt->persistent;
+    const bool inl = n_pops <= n2b::INLINE_POPS && (int32_t)push.size() <= n2b::INLINE_PUSH &&
+                     (int32_t)pull.size() <= n2b::INLINE_PULL;
+    int32_t chunk = 0;
+    if (persistent && inl && pull.empty() && L.n_tiles > 0) {
+        rc = chunk_steps(pops, n_pops, push, push_tgt, ws, L, s, &chunk);
+        if (rc) return rc;
+    }
     if (n_pops) N2B_CUDA(cudaMemcpyAsync(ws + L.pops, pd.data(), sizeof(n2b::PopDev) * n_pops, cudaMemcpyHostToDevice, s));
     if (!push.empty())
         N2B_CUDA(cudaMemcpyAsync(ws + L.push, push.data(), sizeof(n2b::ConnDev) * push.size(), cudaMemcpyHostToDevice, s));
@@ -429,9 +489,6 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
 
     int sms = 0;
     N2B_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int persistent = opt && opt->persistent;
-    const bool inl = n_pops <= n2b::INLINE_POPS && (int32_t)push.size() <= n2b::INLINE_PUSH &&
-                     (int32_t)pull.size() <= n2b::INLINE_PULL;
     // default: per-step launches two blocks per SM; persistent windows one per SM, and at least one per tile
     // plus half an SM's worth of tile-free blocks for the far links (capped by what can be resident; a
     // smaller grid makes the grid barrier cheaper: config 1 steps 2-4% faster at 148 blocks than at 296)
@@ -464,7 +521,26 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
         grid = std::min(std::min(want, most), n2b::BAR_MAX_BLOCKS);
         grid = std::max(grid, 1);
     }
+    int32_t chunk_tn = 0, chunk_tiles = 0;
+    if (chunk) {
+        // the smallest tiles that two blocks per SM still hold at once: a tile's spikes are its block's to deliver
+        // (1,000 neurons: 32 blocks of 32)
+        for (chunk_tn = 32;; chunk_tn *= 2) {
+            chunk_tiles = 0;
+            for (int32_t p = 0; p < n_pops; ++p) chunk_tiles += (pops[p].n + chunk_tn - 1) / chunk_tn;
+            if (chunk_tiles <= 2 * sms || chunk_tn == 256) break;
+        }
+        chunk = std::min(chunk, n2b::chunk_most(chunk_tn));
+        int per_sm = 0;
+        N2B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chunk_kernel_of(chunk_tn), n2b::CHUNK_THREADS, 0));
+        if (per_sm < 1) return fail(N2B_ECUDA, "the chunk kernel cannot be resident");
+        grid = std::min(chunk_tiles, per_sm * sms);
+        if (opt && opt->grid > 0) grid = std::min(grid, opt->grid);
+    }
     n2b_net *net = new n2b_net();
+    net->chunk = chunk;
+    net->chunk_tn = chunk_tn;
+    net->chunk_tiles = chunk_tiles;
     net->device = device;
     net->block = block;
     net->persistent = persistent;

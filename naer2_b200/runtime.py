@@ -35,6 +35,7 @@ from .models import params_of
 from .topology import delay_steps, pack_links, pull_split_form, push_form
 
 MAX_SHIFT = 40
+MAX_LOOKAHEAD = 32  # steps without a grid barrier between them, at most (csrc/n2b_device.cuh, CHUNK_MAX)
 
 
 def next_pow2(x: int) -> int:
@@ -123,6 +124,10 @@ class NetDesc:
     pops: list
     conns: list
     n_links: int
+    # the smallest delay of any link (1 with pull connections or without links): steps that need no grid barrier
+    # between them, when the slots hold that many past each population's largest incoming delay (max_in_delay)
+    lookahead: int = 1
+    max_in_delay: list = field(default_factory=list)
 
 
 def describe(net, modes: dict | None = None, forms: bool = True) -> NetDesc:
@@ -142,6 +147,7 @@ def describe(net, modes: dict | None = None, forms: bool = True) -> NetDesc:
     kp = [params_of(p, dt) for p in pops]
     max_in_delay = [0] * len(pops)
     max_pull_delay = [0] * len(pops)
+    min_delay, pulls = None, False
     in_max = [0.0] * len(pops)
     in_sum: list = [None] * len(pops)
     cinfo = []
@@ -165,9 +171,12 @@ def describe(net, modes: dict | None = None, forms: bool = True) -> NetDesc:
             if warr is None:
                 part = part * abs(wscalar)
             in_sum[t] = part.cpu() if in_sum[t] is None else in_sum[t] + part.cpu()
-            max_in_delay[t] = max(max_in_delay[t], int(steps.max()))
+            least, most = torch.stack(torch.aminmax(steps)).tolist()
+            max_in_delay[t] = max(max_in_delay[t], most)
+            min_delay = least if min_delay is None else min(min_delay, least)
             if mode == "pull":
-                max_pull_delay[s] = max(max_pull_delay[s], int(steps.max()))
+                max_pull_delay[s] = max(max_pull_delay[s], most)
+        pulls = pulls or mode == "pull"
         cinfo.append((s, t, topo, steps, wscalar, warr, mode))
     for k in range(len(pops)):
         in_max[k] = float(in_sum[k].max()) if in_sum[k] is not None and len(in_sum[k]) else 0.0
@@ -208,7 +217,9 @@ def describe(net, modes: dict | None = None, forms: bool = True) -> NetDesc:
         cdesc.append(ConnDesc(src=s, tgt=t, mode=mode, n_links=len(topo), ptr=ptr, link=link,
                               weight=wscalar if wscalar is not None else 0.0, w=w, split=split,
                               topo=topo, steps=steps, warr=warr))
-    return NetDesc(dt=dt, pops=pdesc, conns=cdesc, n_links=sum(c.n_links for c in cdesc))
+    return NetDesc(dt=dt, pops=pdesc, conns=cdesc, n_links=sum(c.n_links for c in cdesc),
+                   lookahead=1 if pulls or min_delay is None else min(min_delay, MAX_LOOKAHEAD),
+                   max_in_delay=max_in_delay)
 
 
 class NetworkRuntime:
@@ -238,7 +249,9 @@ class NetworkRuntime:
             n, words = d.n, (d.n + 31) // 32
             self.words.append(words)
             cp = self.cpop[k]
-            cp.model, cp.n, cp.acc_depth, cp.bit_depth = d.model, n, d.acc_depth, d.bit_depth
+            # slots for the steps that run between two grid barriers as well (at most twice the depth)
+            depth = max(d.acc_depth, min(256, next_pow2(desc.max_in_delay[k] + desc.lookahead))) if d.acc_depth else 0
+            cp.model, cp.n, cp.acc_depth, cp.bit_depth = d.model, n, depth, d.bit_depth
             cp.shift, cp.ref_steps, cp.fire_threshold = d.shift, d.ref_steps, d.fire_threshold
             cp.ext_len, cp.seed, cp.ext_wfx = len(d.ext_table), d.seed, d.ext_wfx
             for i, x in enumerate(d.p):
@@ -251,8 +264,8 @@ class NetworkRuntime:
                 if not tensor.is_contiguous():
                     p._state[attr] = tensor = tensor.contiguous()
                 setattr(cp, slot, tensor.data_ptr())
-            if d.acc_depth:
-                cp.acc = dev_tensor(torch.zeros(d.acc_depth * n, dtype=torch.int64)).data_ptr()
+            if depth:
+                cp.acc = dev_tensor(torch.zeros(depth * n, dtype=torch.int64)).data_ptr()
             if d.bit_depth:
                 cp.bits = dev_tensor(torch.zeros(d.bit_depth * words, dtype=torch.int32)).data_ptr()
             if len(d.ext_table):

@@ -169,6 +169,13 @@ int n2b_capture(n2b_net *net, int32_t window_steps, void *stream);
  * steps). Replaces WindowGraph.replay (naer2/graph.py:120-136). */
 int n2b_replay(n2b_net *net, int64_t n_windows, void *stream);
 
+/* n_steps steps on `stream`, in order with the work on the stream `caller`
+ * (they start after what is on it, what comes on it next starts after them):
+ * whole windows of window_steps from the captured graph (captured on first
+ * use, or when another window was), the rest by n2b_step. One call for what
+ * Network.step does (naer2/network.py:80-152, 264-321). */
+int n2b_advance(n2b_net *net, int64_t n_steps, int32_t window_steps, void *stream, void *caller);
+
 /* Set the step counter (asynchronously, on `stream`); work of the previous
  * step still in the work list is dropped. */
 int n2b_set_step(n2b_net *net, int64_t step, void *stream);

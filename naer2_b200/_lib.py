@@ -67,6 +67,7 @@ SIGNATURES = {
                                   ctypes.c_int32, ctypes.POINTER(Options), _P, ctypes.c_size_t, _P,
                                   ctypes.POINTER(_P)]),
     "n2b_step": (ctypes.c_int, [_P, ctypes.c_int64, _P]),
+    "n2b_advance": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.c_int32, _P, _P]),
     "n2b_capture": (ctypes.c_int, [_P, ctypes.c_int32, _P]),
     "n2b_replay": (ctypes.c_int, [_P, ctypes.c_int64, _P]),
     "n2b_set_step": (ctypes.c_int, [_P, ctypes.c_int64, _P]),

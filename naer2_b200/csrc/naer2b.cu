@@ -169,6 +169,7 @@ struct n2b_net {
     int32_t window = 0;
     // steps without a grid barrier between them (chunk_kernel; 0: a barrier per step), its neurons per tile and tiles
     int32_t chunk = 0, chunk_tn = 0, chunk_tiles = 0;
+    cudaEvent_t before = nullptr, after = nullptr;  // n2b_advance: the caller's stream and the net's, in order
 };
 
 namespace {
@@ -643,6 +644,29 @@ int n2b_replay(n2b_net *net, int64_t n_windows, void *stream) {
     return N2B_OK;
 }
 
+int n2b_advance(n2b_net *net, int64_t n_steps, int32_t window_steps, void *stream, void *caller) {
+    DeviceGuard guard;
+    if (!net) return fail(N2B_EINVAL, "net is NULL");
+    if (n_steps < 0 || window_steps <= 0) return fail(N2B_EINVAL, "n_steps < 0 or window_steps <= 0");
+    N2B_CUDA(cudaSetDevice(net->device));
+    if (!net->before) N2B_CUDA(cudaEventCreateWithFlags(&net->before, cudaEventDisableTiming));
+    if (!net->after) N2B_CUDA(cudaEventCreateWithFlags(&net->after, cudaEventDisableTiming));
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream), c = reinterpret_cast<cudaStream_t>(caller);
+    N2B_CUDA(cudaEventRecord(net->before, c));
+    N2B_CUDA(cudaStreamWaitEvent(s, net->before, 0));
+    const int64_t full = n_steps / window_steps, rest = n_steps % window_steps;
+    int rc = N2B_OK;
+    if (full > 0) {
+        if (net->window != window_steps) rc = n2b_capture(net, window_steps, stream);
+        if (!rc) rc = n2b_replay(net, full, stream);
+    }
+    if (!rc && rest > 0) rc = n2b_step(net, rest, stream);
+    if (rc) return rc;
+    N2B_CUDA(cudaEventRecord(net->after, s));
+    N2B_CUDA(cudaStreamWaitEvent(c, net->after, 0));
+    return N2B_OK;
+}
+
 int n2b_set_step(n2b_net *net, int64_t step, void *stream) {
     DeviceGuard guard;
     if (!net) return fail(N2B_EINVAL, "net is NULL");
@@ -719,6 +743,8 @@ int n2b_destroy(n2b_net *net) {
     if (!net) return N2B_OK;
     cudaSetDevice(net->device);
     drop_graph(net);
+    if (net->before) cudaEventDestroy(net->before);
+    if (net->after) cudaEventDestroy(net->after);
     delete net;
     return N2B_OK;
 }

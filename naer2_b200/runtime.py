@@ -308,7 +308,6 @@ class NetworkRuntime:
         _lib.check(lib.n2b_set_step(self.handle, net.step_count, self._s), "n2b_set_step")
         _lib.check(lib.n2b_record(self.handle, self.rec_step0, self._s), "n2b_record")
         self._leave()
-        self.window = 0
         self.launches = 0  # step kernels launched (one fused step each)
 
     # ------------------------------------------------------------------ stepping
@@ -320,18 +319,9 @@ class NetworkRuntime:
         torch.cuda.current_stream(self.device).wait_stream(self.stream)
 
     def advance(self, n_steps: int) -> None:
-        lib = _lib.load()
         window = max(1, int(self.net.window))
-        full, rem = divmod(int(n_steps), window)
-        self._enter()
-        if full:
-            if self.window != window:
-                _lib.check(lib.n2b_capture(self.handle, window, self._s), "n2b_capture")
-                self.window = window
-            _lib.check(lib.n2b_replay(self.handle, full, self._s), "n2b_replay")
-        if rem:
-            _lib.check(lib.n2b_step(self.handle, rem, self._s), "n2b_step")
-        self._leave()
+        caller = torch.cuda.current_stream(self.device).cuda_stream
+        _lib.check(_lib.load().n2b_advance(self.handle, int(n_steps), window, self._s, caller), "n2b_advance")
         self.launches += n_steps
 
     def start_recording(self, steps: int) -> None:

@@ -1487,11 +1487,12 @@ __device__ __forceinline__ void finish_window(const StepArgs &a, int n_steps) {
 }
 
 // A window of n_steps steps in one cooperative launch (every block resident), steps separated by the grid barrier.
-// DENSE: three blocks per SM (registers capped for it; far items two at a time; no pull connections), for
-// networks with more tiles than two blocks per SM hold -- every tile then keeps a block of its own; otherwise
-// two blocks per SM and far items four at a time.
-template <int NPB, bool INL, bool DENSE>
-__global__ void __launch_bounds__(NPB, DENSE ? 3 : 2)
+// KIND DENSE: three blocks per SM (registers capped for it; far items two at a time), for networks with more tiles
+// than two blocks per SM hold -- every tile then keeps a block of its own; the others: two blocks per SM and far items
+// four at a time. Only WITH_PULL has the pull's code (5.32 to 5.17 us a step at 12,500 neurons, 6.05 to 5.95 at 38,585).
+enum { WITH_PULL, PLAIN, DENSE };
+template <int NPB, bool INL, int KIND>
+__global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
     persistent_kernel(const __grid_constant__ StepArgs a, const int n_steps) {
     if (*(volatile unsigned *)(a.barrier + BAR_ABORT)) return;  // an earlier window gave up: nothing runs
     const long long n0 = *a.step;
@@ -1507,10 +1508,10 @@ __global__ void __launch_bounds__(NPB, DENSE ? 3 : 2)
     cache_rows<NPB, INL>(a, P, j, live, s_cache);
     __shared__ SConn s_tab[SMEM_CONNS];
     const SConn *s_conn = fill_conns<INL>(a, s_tab, a.n_push);
-    PullStage *stage = warp_stage(a);
+    PullStage *stage = KIND == WITH_PULL ? warp_stage(a) : nullptr;
     __syncthreads();
     for (int k = 0; k < n_steps; ++k) {
-        step_body<NPB, INL, DENSE ? 2 : 4, !DENSE>(a, n0 + k, k, &mine, s_cache, s_conn, stage);
+        step_body<NPB, INL, KIND == DENSE ? 2 : 4, KIND == WITH_PULL>(a, n0 + k, k, &mine, s_cache, s_conn, stage);
         if (!grid_sync(a, (unsigned)k)) break;
         N2B_STAMP(a, k, 4);
     }

@@ -158,7 +158,7 @@ struct n2b_net {
     int32_t grid = 0;
     int32_t persistent = 0;
     int32_t inl = 0;  // tables in the kernel parameters
-    int32_t dense = 0;  // persistent windows: the three-blocks-per-SM kernel (more tiles than two per SM hold)
+    int32_t kind = n2b::WITH_PULL;  // persistent windows: which persistent_kernel
     int32_t n_pops = 0;
     size_t dyn_smem = 0;  // dynamic shared memory of the step kernels (the staged pull's buffers)
     Layout L{};
@@ -188,8 +188,9 @@ cudaError_t launch_one(n2b_net *net, int64_t n_steps, cudaStream_t s) {
     if (net->persistent) {
         int32_t k = (int32_t)n_steps;
         void *args[] = {(void *)&net->args, (void *)&k};
-        const void *kern = net->dense ? (const void *)n2b::persistent_kernel<NPB, INL, true>
-                                      : (const void *)n2b::persistent_kernel<NPB, INL, false>;
+        const void *kern = net->kind == n2b::DENSE   ? (const void *)n2b::persistent_kernel<NPB, INL, n2b::DENSE>
+                           : net->kind == n2b::PLAIN ? (const void *)n2b::persistent_kernel<NPB, INL, n2b::PLAIN>
+                                                     : (const void *)n2b::persistent_kernel<NPB, INL, n2b::WITH_PULL>;
         return cudaLaunchCooperativeKernel(kern, dim3(net->grid), dim3(NPB), args, net->dyn_smem, s);
     }
     n2b::StepArgs &a = net->args;
@@ -226,9 +227,9 @@ cudaError_t launch_steps(n2b_net *net, int64_t n_steps, cudaStream_t s) {
 
 // The step kernels' dynamic shared memory limit raised to `dyn` (the staged pull's buffers), and the persistent
 // kernel's resident blocks per SM with it.
-template <int NPB, bool INL, bool DENSE>
+template <int NPB, bool INL, int KIND>
 cudaError_t occupancy(int *per_sm, size_t dyn) {
-    const void *pk = (const void *)n2b::persistent_kernel<NPB, INL, DENSE>;
+    const void *pk = (const void *)n2b::persistent_kernel<NPB, INL, KIND>;
     cudaError_t e = cudaFuncSetAttribute(pk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute((const void *)n2b::step_kernel<NPB, INL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -237,18 +238,20 @@ cudaError_t occupancy(int *per_sm, size_t dyn) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, pk, NPB, dyn);
 }
 
-template <bool DENSE>
+template <int KIND>
 cudaError_t occupancy_of(int32_t block, bool inl, size_t dyn, int *per_sm) {
     switch (block) {
-        case 64: return inl ? occupancy<64, true, DENSE>(per_sm, dyn) : occupancy<64, false, DENSE>(per_sm, dyn);
-        case 256: return inl ? occupancy<256, true, DENSE>(per_sm, dyn) : occupancy<256, false, DENSE>(per_sm, dyn);
-        default: return inl ? occupancy<128, true, DENSE>(per_sm, dyn) : occupancy<128, false, DENSE>(per_sm, dyn);
+        case 64: return inl ? occupancy<64, true, KIND>(per_sm, dyn) : occupancy<64, false, KIND>(per_sm, dyn);
+        case 256: return inl ? occupancy<256, true, KIND>(per_sm, dyn) : occupancy<256, false, KIND>(per_sm, dyn);
+        default: return inl ? occupancy<128, true, KIND>(per_sm, dyn) : occupancy<128, false, KIND>(per_sm, dyn);
     }
 }
 
-int coresident_blocks(int32_t block, bool inl, bool dense, int device, size_t dyn, int *out) {
+int coresident_blocks(int32_t block, bool inl, int kind, int device, size_t dyn, int *out) {
     int per_sm = 0, sms = 0;
-    cudaError_t e = dense ? occupancy_of<true>(block, inl, dyn, &per_sm) : occupancy_of<false>(block, inl, dyn, &per_sm);
+    cudaError_t e = kind == n2b::DENSE   ? occupancy_of<n2b::DENSE>(block, inl, dyn, &per_sm)
+                    : kind == n2b::PLAIN ? occupancy_of<n2b::PLAIN>(block, inl, dyn, &per_sm)
+                                         : occupancy_of<n2b::WITH_PULL>(block, inl, dyn, &per_sm);
     if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
@@ -501,15 +504,15 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
     const size_t stage_bytes = n2b::pull_stage_bytes(weighted_pull);
     const size_t dyn = pull.empty() ? 0 : stage_bytes * (size_t)(block / 32) + sizeof(uint32_t) * cache_words;
     int most = 0;
-    int rc2 = coresident_blocks(block, inl, false, device, dyn, &most);  // also raises the kernels' dynamic limit
+    int kind = pull.empty() ? n2b::PLAIN : n2b::WITH_PULL;
+    int rc2 = coresident_blocks(block, inl, kind, device, dyn, &most);  // also raises the kernels' dynamic limit
     if (rc2) return rc2;
-    bool dense = false;
     if (persistent && L.n_tiles > most && pull.empty()) {  // more tiles than blocks: the denser kernel (push only)
         int most3 = 0;
-        rc2 = coresident_blocks(block, inl, true, device, dyn, &most3);
+        rc2 = coresident_blocks(block, inl, n2b::DENSE, device, dyn, &most3);
         if (rc2) return rc2;
         if (most3 > most) {
-            dense = true;
+            kind = n2b::DENSE;
             most = most3;
         }
     }
@@ -518,7 +521,7 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
         // a grid-wide pull is spread over every warp of the launch, and the dense kernel's tile-free blocks take
         // the far items (PD14: 7.17 us per step at 444 blocks against 7.65 at 379): by default as many blocks
         // as can be resident
-        if ((pull_items > 0 || dense) && !(opt && opt->grid > 0)) want = most;
+        if ((pull_items > 0 || kind == n2b::DENSE) && !(opt && opt->grid > 0)) want = most;
         grid = std::min(std::min(want, most), n2b::BAR_MAX_BLOCKS);
         grid = std::max(grid, 1);
     }
@@ -549,7 +552,7 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
     net->grid = grid;
     net->n_pops = n_pops;
     net->dyn_smem = dyn;
-    net->dense = dense;
+    net->kind = kind;
     net->L = L;
     net->ws = ws;
     n2b::StepArgs &a = net->args;

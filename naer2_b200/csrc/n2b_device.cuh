@@ -984,6 +984,7 @@ __device__ __forceinline__ Row row_of(const ConnDev &C, int j) {
 // A block's shared scratch of one tile phase (declared once per kernel).
 template <int NPB>
 struct Scratch {
+    long long rec0;                   // raster row 0's step
     int cnt;
     int spk[NPB];                      // the tile's spiking neurons (population indices), compacted
     int row[NPB + 1];                  // connections past MERGE_OUT: per spike its row start
@@ -1000,7 +1001,7 @@ struct Scratch {
 // before their reductions (an in-order issue would otherwise wait on each load before the next).
 constexpr int NEAR_BATCH = 4;
 
-template <int NPB, bool INL>
+template <int NPB, bool INL, bool EARLY>
 __device__ __forceinline__ void deliver_spikes(const StepArgs &a, const PopDev &P, int tile_y, const int *s_cache,
                                                int cnt, long long n, Scratch<NPB> &sc, const SConn *s_conn,
                                                int k = 0) {
@@ -1009,10 +1010,10 @@ __device__ __forceinline__ void deliver_spikes(const StepArgs &a, const PopDev &
     const int m = min(P.n_out, MERGE_OUT);
     int *pref = sc.w_pref[warp], *r0s = sc.w_r0[warp];
     // fewer spikes than warps: each spike's walk split over a group of g warps (g a power of two)
-    int g = 1;
-    while (2 * g * cnt <= NW) g *= 2;
-    const int sub = warp % g;
-    for (int p = warp / g; p < cnt; p += NW / g) {
+    int lg = 0;
+    while ((2 << lg) * cnt <= NW) ++lg;
+    const int g = 1 << lg, sub = warp & (g - 1);
+    for (int p = warp >> lg; p < cnt; p += NW >> lg) {
         const int jj = sc.spk[p];
         Row r = Row{0, 0, 0};
         if (lane < m) {
@@ -1041,6 +1042,22 @@ __device__ __forceinline__ void deliver_spikes(const StepArgs &a, const PopDev &
         }
         if (lane == 0) pref[m] = total_near;
         __syncwarp();
+        // EARLY: the far items are listed while the first near links are in flight (the claim's answer comes about
+        // when they do): with the groups' shifts and rec0 read once, 5.17 to 4.6-4.7 us a step at 12,500 neurons, 5.95
+        // to 5.4 at 38,585. In the kernel with the pull path, at its limit of 128 registers, they are listed after
+        // (listed early there, the dense-input network steps in 16.2 us instead of 15.6).
+        auto list_items = [&]() {
+            base = __shfl_sync(FULL, base, 0);
+            if (lane < m && items_c > 0) {
+                int at = base + items_incl - items_c;
+                int4 *list = a.items + (size_t)(n % 3) * (size_t)a.item_cap;
+                for (int q = r.sp; q < r.r1; q += NPB, ++at) {
+                    if (at < a.item_cap) list[at] = make_int4(P.out_first + lane, q, min(q + NPB, r.r1), 0);
+                    else atomicAdd(a.err + 3, 1);
+                }
+            }
+        };
+        bool listed = sub != 0;  // (the group's first warp lists them)
         for (int b0 = sub * 32; b0 < total_near; b0 += 32 * g * NEAR_BATCH) {
             uint32_t rec[NEAR_BATCH];
             float w[NEAR_BATCH];
@@ -1059,22 +1076,16 @@ __device__ __forceinline__ void deliver_spikes(const StepArgs &a, const PopDev &
                     cc[b] = c;
                 }
             }
+            if (EARLY && !listed) {  // the same in every lane
+                list_items();
+                listed = true;
+            }
 #pragma unroll
             for (int b = 0; b < NEAR_BATCH; ++b)
                 if (cc[b] >= 0) deliver_rec(a, conn_view(a, s_conn, P.out_first + cc[b]), rec[b], w[b], n, 1);
         }
+        if (!listed) list_items();
         __syncwarp();
-        if (sub == 0) {
-            base = __shfl_sync(FULL, base, 0);
-            if (lane < m && items_c > 0) {
-                int at = base + items_incl - items_c;
-                int4 *list = a.items + (size_t)(n % 3) * (size_t)a.item_cap;
-                for (int q = r.sp; q < r.r1; q += NPB, ++at) {
-                    if (at < a.item_cap) list[at] = make_int4(P.out_first + lane, q, min(q + NPB, r.r1), 0);
-                    else atomicAdd(a.err + 3, 1);
-                }
-            }
-        }
     }
 }
 
@@ -1214,7 +1225,7 @@ __device__ __forceinline__ void tile_phase(const StepArgs &a, const long long n,
         const int w = (tile.y >> 5) + warp;
         if (P.bits) P.bits[(size_t)(n & P.bit_mask) * P.words + w] = b;
         if (P.raster) {
-            const long long row = n - *a.rec0;
+            const long long row = n - sc.rec0;
             if (row >= 0 && row < P.raster_steps) P.raster[(size_t)row * P.words + w] = b;
         }
     }
@@ -1234,7 +1245,7 @@ __device__ __forceinline__ void tile_phase(const StepArgs &a, const long long n,
     }
 
     // 4. the spikes' outgoing rows
-    if (n_out > 0) deliver_spikes<NPB, INL>(a, P, tile.y, CACHED ? s_cache : nullptr, cnt, n, sc, s_conn, k);
+    if (n_out > 0) deliver_spikes<NPB, INL, !PULL>(a, P, tile.y, CACHED ? s_cache : nullptr, cnt, n, sc, s_conn, k);
     for (int c = MERGE_OUT; c < n_out; ++c) {
         const ConnDev &C = push_at<INL>(a, P.out_first + c);
         const Row r = fire ? row_of(C, j) : Row{0, 0, 0};
@@ -1349,8 +1360,8 @@ __device__ __forceinline__ void far_phase(const StepArgs &a, const long long n, 
 
 template <int NPB, bool INL, int FG, bool PULL = true>
 __device__ __forceinline__ void step_body(const StepArgs &a, const long long n, int k, Neuron *cached,
-                                          const int *s_cache, const SConn *s_conn, PullStage *stage) {
-    __shared__ Scratch<NPB> sc;
+                                          const int *s_cache, const SConn *s_conn, PullStage *stage,
+                                          Scratch<NPB> &sc) {
     N2B_STAMP(a, k, 0);
     const int far_n = far_count(a, n - 1);  // in flight under the tile
     if (blockIdx.x == 0 && threadIdx.x == 0) {  // step n + 1's list and tile counter, list n's chunk counter
@@ -1407,8 +1418,10 @@ __global__ void __launch_bounds__(NPB, 2) step_kernel(const __grid_constant__ St
     __shared__ SConn s_tab[SMEM_CONNS];
     const SConn *s_conn = fill_conns<INL>(a, s_tab, a.n_push);
     PullStage *stage = warp_stage(a);
+    __shared__ Scratch<NPB> sc;
+    if (threadIdx.x == 0) sc.rec0 = *a.rec0;
     __syncthreads();
-    step_body<NPB, INL, 2>(a, *a.step + a.offset, 0, nullptr, nullptr, s_conn, stage);
+    step_body<NPB, INL, 2>(a, *a.step + a.offset, 0, nullptr, nullptr, s_conn, stage, sc);
 }
 
 __device__ __forceinline__ unsigned long long globaltimer() {
@@ -1496,6 +1509,8 @@ __global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
     persistent_kernel(const __grid_constant__ StepArgs a, const int n_steps) {
     if (*(volatile unsigned *)(a.barrier + BAR_ABORT)) return;  // an earlier window gave up: nothing runs
     const long long n0 = *a.step;
+    __shared__ Scratch<NPB> sc;
+    if (threadIdx.x == 0) sc.rec0 = *a.rec0;  // (read at each step it would miss the L1, in the step's chain)
     // the block's first tile stays in registers for the whole window
     const bool has_tile = (int)blockIdx.x < a.n_tiles;
     const int4 tile = has_tile ? tile_at<INL, NPB>(a, blockIdx.x) : make_int4(0, 0, 0, 0);
@@ -1511,7 +1526,8 @@ __global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
     PullStage *stage = KIND == WITH_PULL ? warp_stage(a) : nullptr;
     __syncthreads();
     for (int k = 0; k < n_steps; ++k) {
-        step_body<NPB, INL, KIND == DENSE ? 2 : 4, KIND == WITH_PULL>(a, n0 + k, k, &mine, s_cache, s_conn, stage);
+        step_body<NPB, INL, KIND == DENSE ? 2 : 4, KIND == WITH_PULL>(a, n0 + k, k, &mine, s_cache, s_conn, stage,
+                                                                           sc);
         if (!grid_sync(a, (unsigned)k)) break;
         N2B_STAMP(a, k, 4);
     }

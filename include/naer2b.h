@@ -212,14 +212,15 @@ int n2b_destroy(n2b_net *net);
  * The backward uses g = 1 / (1 + slope |Vpre - theta|)^2 for ds/dVpre (the
  * fast-sigmoid surrogate; the exact derivative of the smooth f), the reset
  * included. The forward keeps the spikes of every step (one bit per neuron,
- * sample and step) and the membrane every `checkpoint` steps; the backward
- * recomputes each segment from its checkpoint, then runs it backwards over
+ * sample and step), the membrane every `checkpoint` steps and, where that
+ * takes 4 GiB at most, g of every step; the backward runs it backwards (else
+ * it recomputes each segment's g from its checkpoint first) over
  * the transposed (outgoing) rows. */
 
 /* error words: 0 links with a bad code (skipped); 1 recomputed spikes that
  * differ from the forward's; 2 in_cta_max / out_cta_max below the rows' counts;
- * 3 waits of the backward's per-step exchange that gave up (the results are
- * then wrong; the kernel still ends) */
+ * 3 waits of the per-step exchange (forward or backward) that gave up (the
+ * results are then wrong; the kernel still ends) */
 #define N2B_BPTT_ERR_WORDS 4
 
 typedef struct n2b_bptt_desc {
@@ -243,8 +244,8 @@ typedef struct n2b_bptt_desc {
     int32_t reserved;
 } n2b_bptt_desc;
 
-/* Device workspace bytes of the layer (spike tape, checkpoints, one segment's
- * surrogate derivatives, per-group gradient partials). */
+/* Device workspace bytes of the layer (spike tape, checkpoints, the surrogate
+ * derivatives of every step or of one segment, per-group gradient partials). */
 int n2b_bptt_workspace_bytes(const n2b_bptt_desc *d, size_t *bytes);
 
 /* Forward over all steps: u [T][B][H] input current, w_rec [nnz] (incoming

@@ -6,8 +6,9 @@ sparse delayed recurrence (w_rec, delays 1..5 steps) -> R leaky non-spiking read
 over time of each readout, m [B, R], for a cross-entropy loss.
 The recurrence and its adjoint run in `n2b_bptt_forward` / `n2b_bptt_backward` (naer2_b200/csrc/bptt.cu)
 behind `torch.autograd.Function`: the forward keeps the spikes of every step (one bit per neuron, sample and
-step) and the membrane every `checkpoint` steps; the backward recomputes each segment from its checkpoint and
-runs it backwards over the transposed (outgoing) rows. The model equations are stated in include/naer2b.h.
+step), the membrane every `checkpoint` steps and, where that takes 4 GiB at most, the surrogate's derivative of
+every step; the backward runs it backwards over the transposed (outgoing) rows, else it recomputes each segment
+from its checkpoint first. The model equations are stated in include/naer2b.h.
 
 naer2 itself has no differentiable path; this layer follows the BPTT workload's description (700 input
 channels, 1024 hidden neurons at 10% recurrent density, delays of 1-5 steps, 20 readouts, fast-sigmoid
@@ -41,13 +42,12 @@ def draw_links(hidden: int, density: float, max_delay: int = MAX_DELAY, seed: in
 def bank_order(post: np.ndarray, grp: np.ndarray) -> np.ndarray:
     """An order of the outgoing links within each (pre, delay) group for the adjoint's shared-memory gather.
 
-    The adjoint gives each neuron four threads; the thread `sub` of a neuron takes the links 4k + sub of each
-    of its delay groups (k = 0, 1, ...), and one 128-bit load of a quarter warp serves the 8 threads of two
-    neurons 2i, 2i + 1 at the same k. Each thread reads the q row of its link's target, rows 48 bytes apart,
-    so the load touches the 16-byte bank group (3 post + half) mod 8: targets with distinct post mod 8 are
-    served in one pass, equal ones in several. Greedily, each chunk k of the two neurons' groups takes links
-    with distinct residues mod 8, the most frequent remaining residues first. Returns positions into `post`
-    (a permutation within each group); the sums are the same up to their order."""
+    The adjoint gives each neuron eight threads, four link shares of a group times two halves of the samples: share
+    `sub` takes the links 4k + sub (k = 0, 1, ...), so that a quarter warp's 128-bit loads read the q rows of one
+    chunk k's four targets, 32 bytes each: targets with distinct post mod 4 are served in one pass, equal ones in
+    several. Greedily, each chunk takes links with distinct residues mod 4, the most frequent remaining residues
+    first, and of each residue the half (mod 8) that the next neuron's chunk does not use (a warp's other loads).
+    Returns positions into `post` (a permutation within each group); the sums are the same up to their order."""
     hidden = grp.shape[0]
     perm = np.arange(len(post))
     res = post % 8
@@ -65,13 +65,19 @@ def bank_order(post: np.ndarray, grp: np.ndarray) -> np.ndarray:
                 used = set()
                 for pool, out, (s, e) in zip(pools, outs, spans):
                     take, got = min(4, e - s - len(out)), 0
-                    for r in sorted(range(8), key=lambda r: -len(pool[r])):
+                    # each residue mod 4 by how many links it has left; of its two residues mod 8 the fuller one
+                    # that the pair has not used
+                    for r in sorted(range(4), key=lambda r: -len(pool[r]) - len(pool[r + 4])):
                         if got == take:
                             break
-                        if pool[r] and r not in used:
-                            out.append(pool[r].pop())
-                            used.add(r)
-                            got += 1
+                        lo, hi = (r, r + 4) if len(pool[r]) >= len(pool[r + 4]) else (r + 4, r)
+                        if not pool[lo]:
+                            continue
+                        if lo in used and hi not in used and pool[hi]:
+                            lo = hi
+                        out.append(pool[lo].pop())
+                        used.add(lo)
+                        got += 1
                     while got < take:  # no distinct residue left: the fullest one
                         out.append(pool[max(range(8), key=lambda r: len(pool[r]))].pop())
                         got += 1

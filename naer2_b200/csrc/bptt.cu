@@ -14,19 +14,20 @@
 //                                           + sum_r w_out[i][r] o[t][r] - theta alpha q[t+1][i])
 //   dU[t][i] = q[t][i];  dw_k = sum_t,b s[t - d_k][pre_k] q[t][post_k];  dw_out[i][r] = sum_t,b s[t][i] o[t][r]
 //
-// Layout: a group of 8 CTAs runs 8 samples; CTA `rank` owns hidden neurons [rank*HC, rank*HC + HC), HC = H/8,
-// four threads per neuron (two samples each; the link loops split a row among the four, interleaved). The
-// forward's group is a thread-block cluster; the adjoint's is a plain group of one cooperative launch (one
-// CTA per SM: at that size only 15 clusters of 8 are resident on 148 SMs, but every group must be).
-// Forward: every CTA keeps the spikes of the last 6 steps of all H neurons for its 8 samples (one byte of 8
-// sample bits per neuron, or 8 floats in the smooth model) in shared memory; each step a neuron's new entry
-// is written into all 8 CTAs' rings (distributed shared memory) before one cluster barrier. Backward: each
-// K-step segment is first recomputed from its membrane checkpoint and the stored spikes of every step by two
-// grid-wide kernels (the recurrent inputs of all its steps at once, then one membrane scan per neuron and
-// sample; same arithmetic, same order: the same Vpre bit for bit), then run backwards by one
-// cooperative launch; q of all neurons is exchanged through a two-slot ring in global memory (L2) with one
-// counted arrival per CTA and step, and each neuron pushes its outgoing rows' q sums into a 6-slot ring of its
-// own partials, kept in global memory between the segments' launches.
+// Layout: a group of 8 CTAs runs 8 samples; CTA `rank` owns hidden neurons [rank*HC, rank*HC + HC), HC = H/8.
+// Spiking forward (fwd_group_kernel) and adjoint (bwd_kernel): eight threads per neuron, groups of one cooperative
+// launch (one CTA per SM: at that size only 15 clusters of 8 are resident on 148 SMs, but every group must be) that
+// exchange a step's spikes, or its q, through the L2. The smooth model, and rows that do not fit a CTA's shared
+// memory, take fwd_kernel: four threads per neuron (two samples each), the group a thread-block cluster, every CTA
+// writing its neurons' entries into all 8 CTAs' spike rings (distributed shared memory) before one cluster barrier.
+// The forward keeps the last spikes of all H neurons for its 8 samples in shared memory (one byte of 8 sample bits per
+// neuron, or 8 floats in the smooth model). Backward: what it needs of the forward is the surrogate's derivative of
+// every step. Up to FULL_TAPE_BYTES the forward keeps them; past that each K-step segment is first recomputed from its
+// membrane checkpoint and the stored spikes by two grid-wide kernels (the recurrent inputs of all its steps at once,
+// then one membrane scan per neuron and sample; same arithmetic, same order: the same Vpre bit for bit). The adjoint
+// runs all steps, or the segment, backwards in one cooperative launch: q of all neurons is exchanged through a two-slot
+// ring in global memory, and each neuron pushes its outgoing rows' q sums into a 6-slot ring of its own partials,
+// kept in global memory between the segments' launches.
 // Every sum has a fixed order (no float atomics), so results are bit-for-bit reproducible.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -67,6 +68,10 @@ struct Args {
     float *s_f;         // [T][NC][H][8]   (smooth)
     float *v_ckpt;      // [nseg][B][H]
     float *g_seg;       // [K][B][H]: the segment's recurrent input, then its surrogate derivatives
+    uint8_t *s_plain;   // [T][NC][H]: the plain forward's spikes
+    unsigned long long *xw;  // [NC][XSLOTS][H / 4]: the forward's published words
+    float *tot;         // [T][B][R]: every step's readout sums
+    float *g_all;       // [T][B][H]: every step's surrogate derivatives, or null (segments recomputed)
     float *dU;          // [T][B][H]
     const float *w_out; // [H][R]
     float *m;           // [B][R]
@@ -79,9 +84,10 @@ struct Args {
     float *q_st;        // [B][H] q[t0] of the last segment done
     float *o_st;        // [B][R] the readout adjoint at t0
     float *qx;          // [NC][2][H][8] the adjoint's q exchange ring (slot t & 1)
-    uint32_t *xcnt;     // [NC] the adjoint's arrivals per group (zeroed before each launch)
+    uint32_t *qflag;    // [NC][2][H / 4] its flags, one per warp (cleared before a call's first launch)
+    float *o_all;       // [T][B][R]: every step's readout adjoint (all steps in one launch)
     int32_t *err;       // [N2B_BPTT_ERR_WORDS]
-    int wait_polls;     // polls before an exchange wait gives up
+    int wait_polls;     // polls before a wait of the adjoint's exchange gives up
 };
 
 __device__ __forceinline__ float surrogate(float x, float slope) {
@@ -117,19 +123,17 @@ __host__ __device__ inline FwdSmem fwd_smem(int H, int HC, int R, bool smooth, b
     return L;
 }
 
-constexpr int QROW = 12;  // floats per neuron in the q exchange buffer: 8 samples, padded for the banks
-
 struct BwdSmem {
     size_t pnew, part, dwo, obuf, grp, code, w, dw, total;
 };
-__host__ __device__ inline BwdSmem bwd_smem(int H, int HC, int R, int out_cta_max) {
+__host__ __device__ inline BwdSmem bwd_smem(int H, int HC, int R, int out_cta_max, bool full) {
     BwdSmem L{};
     size_t o = 0;
     auto a16 = [](size_t x) { return (x + 15) & ~size_t(15); };
-    L.pnew = o; o = a16(o + sizeof(float) * H * QROW);
+    L.pnew = o; o = a16(o + sizeof(float) * H * NS);
     L.part = o; o = a16(o + sizeof(float) * RING * HC * NS);
-    L.dwo = o; o = a16(o + sizeof(float) * HC * R);
-    L.obuf = o; o = a16(o + sizeof(float) * 2 * NS * R);  // o[t] in half t & 1
+    L.dwo = o; o = a16(o + (full ? 0 : sizeof(float) * HC * R));
+    L.obuf = o; o = a16(o + (full ? 0 : sizeof(float) * 2 * NS * R));  // o[t] in half t & 1
     L.grp = o; o = a16(o + sizeof(int32_t) * HC * (MAXD + 1));
     L.code = o; o = a16(o + sizeof(uint16_t) * out_cta_max);
     L.w = o; o = a16(o + sizeof(float) * out_cta_max);
@@ -138,28 +142,27 @@ __host__ __device__ inline BwdSmem bwd_smem(int H, int HC, int R, int out_cta_ma
     return L;
 }
 
-// One CTA's arrival at a group step (thread 0, after a __syncthreads that follows the CTA's writes): a release
-// add on the group's counter; later (other work in between), a bounded acquire spin until `target` arrivals
-// (every CTA of the group at this step). A wait that gives up counts in err[3] and sets `aborted`, after which
-// the CTA still arrives but no longer waits, so that neither it nor the CTAs that wait for its arrivals can hang.
+// The forward's exchange between a group's CTAs, step by step: four neurons' spikes are published as one 64-bit word, the
+// step's number + 1 beside the 32 bits, and every CTA polls the words themselves (one write and one read through the
+// L2; no fence, counter or barrier). The words are cleared before a call's first launch. Polls are bounded, here and in
+// the adjoint: one that gives up counts in err[3] and sets the CTA's `aborted`, after which it polls no more -- it
+// publishes its own words all the same, so that neither it nor the CTAs that wait for them can hang.
 constexpr int XCHG_SPIN_LIMIT = 1 << 21;  // default polls (n2b_bptt_desc.wait_polls = 0): about a second
-__device__ __forceinline__ void group_arrive(uint32_t *cnt) {
-    __threadfence();
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+__device__ __forceinline__ void publish(unsigned long long *p, uint32_t word, uint32_t tag) {
+    const unsigned long long v = ((unsigned long long)tag << 32) | word;
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ void group_wait(const uint32_t *cnt, uint32_t target, int32_t *err, int limit,
-                                           int &aborted) {
-    if (aborted) return;
-    for (int it = 0;; ++it) {
-        uint32_t v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
-        if (v >= target) return;
-        if (it >= limit) {
-            atomicAdd(err + 3, 1);
-            aborted = 1;
-            return;
+// The word published under `tag`, polled for at most `limit` times.
+__device__ __forceinline__ bool await(const unsigned long long *p, uint32_t tag, int limit, uint32_t &word) {
+    for (int it = 0; it < limit; ++it) {
+        unsigned long long v;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+        if ((uint32_t)(v >> 32) == tag) {
+            word = (uint32_t)v;
+            return true;
         }
     }
+    return false;
 }
 
 // The spikes that the incoming links read: the forward's shared-memory ring (6 slots, the slot of step t in
@@ -368,6 +371,340 @@ __global__ void __launch_bounds__(512) fwd_kernel(const __grid_constant__ Args a
     cl.sync();  // no CTA leaves while another may still address its shared memory
 }
 
+// ------------------------------------------------------------------------------------------------ forward, by spikes
+
+// The spiking forward with the incoming rows in shared memory: a group of 8 CTAs of one cooperative launch, a CTA per
+// SM (clusters of 8 would not do: 16 of them do not fit 148 SMs one CTA each, and two CTAs on an SM halve the pace of
+// their groups, and so of the launch). A step is a chain -- the group's spikes of the step before, each row's look at
+// its sources, the sums in link order, the new spikes -- of which little is arithmetic, so:
+//   - a warp publishes its four neurons' spikes as one 64-bit word, the step's number beside the 32 bits, and every
+//     CTA polls the group's words themselves: one write and one read through the L2, no fence, counter or barrier;
+//   - which of a row's links of delay 2..5 have a spike (one byte load and a bit each; the codes are the byte's address
+//     past the step's, four to a 64-bit load) is found before the step's words are there;
+//   - only those links and the delay-1 links are then added, in link order: fwd_kernel's sums bit for bit (a link
+//     without a spike adds nothing there either);
+//   - the input currents are loaded two steps ahead, and the readout is a pair of kernels of its own over the spikes
+//     (its sums do not feed the recurrence).
+// Measured at batch 128, 500 steps, 1024 hidden neurons of 102 links, 1.9% of them spiking: 4.18 ms in fwd_kernel, 1.71 ms
+// here (1.9 with the readout's kernels).
+constexpr int NB = NS;        // threads per neuron: one sample each; in the link loops four link shares times two halves
+constexpr int LS = NB / 2;    // of the samples
+constexpr int SLOTS = 8;      // spike ring slots in shared memory (t & 7)
+constexpr int XSLOTS = 4;     // slots of the group's published words (t & 3)
+constexpr int WORD_LINKS = 32, MASK_LINKS = 2 * WORD_LINKS;  // links of a share with a place in its masks
+constexpr int NEAR_REGS = 4;  // delay-1 links a thread holds in registers (a share has about five, two lanes look at them)
+constexpr size_t SMEM_MAX = 227 * 1024;
+
+struct ScanSmem {
+    size_t ring, ptr, row, code, w, total;
+};
+__host__ __device__ inline int scan_stride(int H) {  // bytes of a ring slot: a power of two
+    int s = 32;
+    while (s < H) s *= 2;
+    return s;
+}
+__host__ __device__ inline ScanSmem scan_smem(int H, int HC, int in_cta_max) {
+    ScanSmem L{};
+    size_t o = 0;
+    auto a16 = [](size_t x) { return (x + 15) & ~size_t(15); };
+    L.ring = o; o = a16(o + (size_t)SLOTS * scan_stride(H));
+    L.ptr = o; o = a16(o + sizeof(int32_t) * (HC + 1));
+    L.row = o; o = a16(o + sizeof(int32_t) * (HC + 1));
+    // each of a row's NT shares padded to whole 64-bit loads (of a row of len links: at most len + 15 codes)
+    L.code = o; o = a16(o + sizeof(uint16_t) * ((size_t)in_cta_max + 15 * HC));
+    L.w = o; o = a16(o + sizeof(float) * in_cta_max);
+    L.total = o;
+    return L;
+}
+// Codes of one share of a row of len links, padded.
+__host__ __device__ inline int scan_share(int len) { return ((len + NT - 1) / NT + 3) / 4 * 4; }
+
+// Of four bytes, which have a bit in their low nibble, as four bits.
+__device__ __forceinline__ uint32_t low_nibbles(uint32_t x) {
+    const uint32_t t = (((x & 0x0F0F0F0Fu) + 0x0F0F0F0Fu) >> 4) & 0x01010101u;  // 15 + a nibble carries unless it is 0
+    return (t * 0x00204081u) >> 21 & 0xFu;                                      // bits 0, 8, 16, 24 to 21 .. 24
+}
+
+__global__ void __launch_bounds__(NB * 128) fwd_group_kernel(const __grid_constant__ Args a, int in_cta_max, int g0) {
+    const int rank = (int)blockIdx.x % CL;
+    const int q = g0 + (int)blockIdx.x / CL;
+    const int H = a.H, HC = a.HC, B = a.B;
+    const int h0 = rank * HC, stride = scan_stride(H);
+    const ScanSmem L = scan_smem(H, HC, in_cta_max);
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char *ring = smem + L.ring;
+    int32_t *lptr = reinterpret_cast<int32_t *>(smem + L.ptr);
+    int32_t *row = reinterpret_cast<int32_t *>(smem + L.row);
+    uint16_t *code = reinterpret_cast<uint16_t *>(smem + L.code);
+    float *w = reinterpret_cast<float *>(smem + L.w);
+    __shared__ int aborted;
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
+
+    if (tid == 0) aborted = 0;
+    for (size_t k = tid; k < L.ptr / 4; k += nthr) reinterpret_cast<uint32_t *>(ring)[k] = 0u;
+    const int base = a.in_ptr[h0];
+    for (int k = tid; k <= HC; k += nthr) lptr[k] = a.in_ptr[h0 + k] - base;
+    __syncthreads();
+    const bool in_smem = lptr[HC] <= in_cta_max;
+    if (!in_smem && tid == 0) atomicAdd(a.err + 2, 1);  // a wrong in_cta_max: the rows stay global
+    if (in_smem && tid < 32) {  // each row's first code
+        int sum = 0;
+        for (int p0 = 0; p0 < HC; p0 += 32) {
+            const int p = p0 + lane;
+            const int n = p < HC ? NT * scan_share(lptr[p + 1] - lptr[p]) : 0;
+            int incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (p < HC) row[p] = sum + incl - n;
+            sum += __shfl_sync(FULL, incl, 31);
+        }
+    }
+    __syncthreads();
+    for (int p = tid / 32; in_smem && p < HC; p += nthr / 32) {  // a warp per row: its links, validated once
+        const int rs = lptr[p], len = lptr[p + 1] - rs, share = scan_share(len);
+        for (int k = lane; k < NT * share; k += 32) {  // share k / share, link number k % share of it
+            const int l = (k % share) * NT + k / share;
+            uint32_t c = 1u << 11;  // padding and bad links: a link of weight 0, one step from neuron 0
+            if (l < len) {
+                const uint32_t g = a.in_code[base + rs + l];
+                const bool bad = (g >> 11) < 1 || (g >> 11) > MAXD || (g & 0x7FFu) >= (uint32_t)H;
+                if (bad) atomicAdd(a.err + 0, 1);
+                else c = g;
+                w[rs + l] = bad ? 0.f : a.in_w[base + rs + l];
+            }
+            // the byte of step t - d is at ((t + 8 - d) & 7) * stride + pre
+            code[row[p] + k] = (uint16_t)((SLOTS - (c >> 11)) * stride + (c & 0x7FFu));
+        }
+    }
+    __syncthreads();
+
+    const unsigned mask = (unsigned)(SLOTS * stride - 1);
+    const bool nt = tid < NB * HC;
+    const int pl = nt ? tid / NB : 0;                     // the thread's neuron
+    const int half = (tid >> 2) & 1, sub = tid % LS;      // in the link loops: its half of the samples, its share
+    const int own = tid % NB;                             // its sample (LS half + sub)
+    const int post = h0 + pl;
+    const int len = nt ? lptr[pl + 1] - lptr[pl] : 0;
+    const int links = len > sub ? (len - sub + NT - 1) / NT : 0;  // of this share
+    const int kept = in_smem ? links : 0;
+    const uint16_t *sc = code + (in_smem ? row[pl] + sub * scan_share(lptr[pl + 1] - lptr[pl]) : 0);
+    const float *sw = w + lptr[pl] + sub;
+    // the codes this lane looks at before the step's words are there, of the share's first 32 links: the two halves'
+    // lanes take every other group of four (padding and links past the share's end are masked out below)
+    uint2 codes[WORD_LINKS / 8];
+#pragma unroll
+    for (int g = 0; g < WORD_LINKS / 8; ++g) {
+        const int i = 8 * g + 4 * half;
+        codes[g] = i < kept ? *reinterpret_cast<const uint2 *>(sc + i) : make_uint2(0u, 0u);
+    }
+    // the share's links of delay 1 (their spikes come with the step's words), by place; of its first 32 links' the
+    // two halves' lanes hold every other one's code (and place, in the bits above 16), those past the registers stay in `rest`
+    uint32_t near[2] = {0u, 0u}, rest = 0u, held[NEAR_REGS];
+    {
+        int k = 0;
+        for (int i = 0; i < min(kept, MASK_LINKS); ++i) {
+            if (sc[i] < (SLOTS - 1) * stride) continue;
+            near[i / WORD_LINKS] |= 1u << (i % WORD_LINKS);
+            if (i < WORD_LINKS && k++ >= 2 * NEAR_REGS) rest |= 1u << i;
+        }
+#pragma unroll
+        for (int h = 0; h < NEAR_REGS; ++h) {
+            uint32_t m = near[0];
+            for (int j = 2 * h + half; j > 0 && m; --j) m &= m - 1;
+            const int i = m ? __ffs(m) - 1 : 0;
+            held[h] = m ? sc[i] | (uint32_t)i << 16 | 1u << 31 : 0u;
+        }
+    }
+    uint32_t *ring32 = reinterpret_cast<uint32_t *>(ring);
+    unsigned long long *xw = a.xw + (size_t)q * XSLOTS * (H / 4);
+    uint8_t *bits_out = a.tape ? a.s_bits : a.s_plain;
+    const float *u = a.U + ((size_t)q * NS + own) * H + post;
+    const size_t ustep = (size_t)B * H;
+    float V = 0.f, u0 = nt ? __ldcs(u) : 0.f, u1 = (nt && a.T > 1) ? __ldcs(u + ustep) : 0.f;
+    const unsigned nib = 0xFu << (LS * half);
+    for (int t = 0; t < a.T; ++t) {
+        const float u2 = (nt && t + 2 < a.T) ? __ldcs(u + (size_t)(t + 2) * ustep) : 0.f;
+        if (a.tape && !a.g_all && t % a.K == 0 && nt)
+            a.v_ckpt[((size_t)(t / a.K) * B + (size_t)q * NS + own) * H + post] = V;
+        const unsigned tb = (unsigned)(t & (SLOTS - 1)) * stride;
+        // which of the share's links of delay 2..5 have a spike, in either half of the samples (each lane for every
+        // other group of four links; the halves exchange)
+        uint32_t hit[2] = {0u, 0u};
+        {
+            uint32_t lo = 0u, hi = 0u;
+#pragma unroll
+            for (int g = 0; g < WORD_LINKS / 8; ++g) {
+                const uint2 c4 = codes[g];
+                const uint32_t b0 = ring[(tb + (c4.x & 0xFFFFu)) & mask], b1 = ring[(tb + (c4.x >> 16)) & mask];
+                const uint32_t b2 = ring[(tb + (c4.y & 0xFFFFu)) & mask], b3 = ring[(tb + (c4.y >> 16)) & mask];
+                const uint32_t all = b0 | b1 << 8 | b2 << 16 | b3 << 24;
+                lo |= low_nibbles(all) << (8 * g);
+                hi |= low_nibbles(all >> 4) << (8 * g);
+            }
+            lo <<= 4 * half;
+            hi <<= 4 * half;
+            hit[0] = (half ? hi : lo) | __shfl_xor_sync(FULL, half ? lo : hi, LS);
+            hit[0] &= (kept < WORD_LINKS ? (1u << kept) - 1u : ~0u) & ~near[0];
+        }
+        if (__any_sync(FULL, kept > WORD_LINKS)) {  // rows of more than 128 links
+            for (int i = WORD_LINKS; i < min(kept, MASK_LINKS); ++i)
+                if (ring[(tb + sc[i]) & mask] & nib) hit[1] |= 1u << (i - WORD_LINKS);
+            hit[1] |= near[1];
+        }
+        if (t > 0) {  // the group's spikes of step t - 1
+            if (tid < H / 4) {
+                uint32_t word = 0u;
+                if (!*(volatile int *)&aborted &&
+                    !await(xw + (size_t)((t - 1) % XSLOTS) * (H / 4) + tid, (uint32_t)t, XCHG_SPIN_LIMIT, word)) {
+                    atomicAdd(a.err + 3, 1);
+                    *(volatile int *)&aborted = 1;
+                }
+                ring32[((t - 1) & (SLOTS - 1)) * (stride / 4) + tid] = word;
+            }
+            __syncthreads();
+        }
+        {  // ... and of its links of delay 1
+            uint32_t lo = 0u, hi = 0u;
+#pragma unroll
+            for (int h = 0; h < NEAR_REGS; ++h) {
+                const uint32_t byte = ring[(tb + (held[h] & 0xFFFFu)) & mask], bit = (held[h] >> 31) << (held[h] >> 16 & 31u);
+                if (byte & 0x0Fu) lo |= bit;
+                if (byte & 0xF0u) hi |= bit;
+            }
+            hit[0] |= (half ? hi : lo) | __shfl_xor_sync(FULL, half ? lo : hi, LS);
+            for (uint32_t m = rest; m; m &= m - 1) {
+                const int i = __ffs(m) - 1;
+                if (ring[(tb + sc[i]) & mask] & nib) hit[0] |= 1u << i;
+            }
+        }
+        float acc[LS] = {0.f, 0.f, 0.f, 0.f};
+        auto add = [&](uint32_t byte, float wl) {
+            const uint32_t b = byte & nib;
+            if (b & 0x11u) acc[0] = __fadd_rn(acc[0], wl);
+            if (b & 0x22u) acc[1] = __fadd_rn(acc[1], wl);
+            if (b & 0x44u) acc[2] = __fadd_rn(acc[2], wl);
+            if (b & 0x88u) acc[3] = __fadd_rn(acc[3], wl);
+        };
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            uint32_t h = hit[m];
+            while (h) {  // two links' loads at a time
+                const int i = m * WORD_LINKS + __ffs(h) - 1;
+                h &= h - 1;
+                const int j = h ? m * WORD_LINKS + __ffs(h) - 1 : i;
+                const uint32_t bi = ring[(tb + sc[i]) & mask], bj = h ? ring[(tb + sc[j]) & mask] : 0u;
+                const float wi = sw[NT * i], wj = sw[NT * j];
+                h &= h - 1;
+                add(bi, wi);
+                add(bj, wj);
+            }
+        }
+        for (int i = in_smem ? MASK_LINKS : 0; i < links; ++i) {  // links past the masks, or every link from memory
+            if (in_smem) {
+                add(ring[(tb + sc[i]) & mask], sw[NT * i]);
+                continue;
+            }
+            const uint32_t g = a.in_code[base + lptr[pl] + sub + NT * i];
+            const int pre = (int)(g & 0x7FFu), d = (int)(g >> 11);
+            if (d < 1 || d > MAXD || pre >= H) {
+                if (half == 0) atomicAdd(a.err + 0, 1);
+                continue;
+            }
+            add(ring[(tb + (unsigned)((SLOTS - d) * stride + pre)) & mask], a.in_w[base + lptr[pl] + sub + NT * i]);
+        }
+        __syncwarp();
+        // the shares added pairwise, (s0 + s1) + (s2 + s3); the lane keeps its own sample's
+#pragma unroll
+        for (int b = 0; b < LS; ++b) acc[b] = __fadd_rn(acc[b], __shfl_xor_sync(FULL, acc[b], 1));
+#pragma unroll
+        for (int b = 0; b < LS; ++b) acc[b] = __fadd_rn(acc[b], __shfl_xor_sync(FULL, acc[b], 2));
+        float vp = 0.f, sp = 0.f;
+        if (nt) sp = lif_step<false>(a, V, u0, sub == 0 ? acc[0] : sub == 1 ? acc[1] : sub == 2 ? acc[2] : acc[3], vp);
+        u0 = u1;
+        u1 = u2;
+        // the warp's four neurons' bytes, samples in lane order
+        const uint32_t word = __ballot_sync(FULL, sp != 0.f);
+        if (lane == 0 && nt) {
+            publish(xw + (size_t)(t % XSLOTS) * (H / 4) + (post >> 2), word, (uint32_t)t + 1u);
+            *reinterpret_cast<uint32_t *>(bits_out + ((size_t)t * a.NC + q) * H + post) = word;
+        }
+        if (a.tape && a.g_all && nt)
+            __stcs(a.g_all + ((size_t)t * B + (size_t)q * NS + own) * H + post, surrogate(__fadd_rn(vp, -a.theta), a.slope));
+    }
+}
+
+// The readout of every step, from the stored spikes: a block per (step, group), its 8 samples' spikes as bit masks,
+// then a thread per (sample, readout): sum over each eighth of the neurons in ascending order, the eighths added in
+// order (as the CTAs of fwd_kernel sum and add).
+constexpr int READOUT_THREADS = 256;
+__global__ void __launch_bounds__(READOUT_THREADS) readout_kernel(const __grid_constant__ Args a) {
+    __shared__ uint32_t bits[NS][32];
+    const int t = blockIdx.x, q = blockIdx.y, lane = threadIdx.x & 31;
+    const uint8_t *src = (a.tape ? a.s_bits : a.s_plain) + ((size_t)t * a.NC + q) * a.H;
+    for (int g = threadIdx.x / 32; g < a.H / 32; g += READOUT_THREADS / 32) {
+        const uint32_t byte = src[32 * g + lane];
+#pragma unroll
+        for (int b = 0; b < NS; ++b) {
+            const uint32_t m = __ballot_sync(FULL, (byte >> b) & 1u);
+            if (lane == b) bits[b][g] = m;
+        }
+    }
+    __syncthreads();
+    for (int pair = threadIdx.x; pair < NS * a.R; pair += READOUT_THREADS) {
+        const int b = pair / a.R;
+        const float *w = a.w_out + pair % a.R;
+        float tot = 0.f, sum = 0.f;
+        int end = a.HC;  // of the eighth being summed
+        for (int g = 0; g < a.H / 32; ++g)
+            for (uint32_t m = bits[b][g]; m; m &= m - 1) {
+                const int n = 32 * g + __ffs(m) - 1;
+                if (n >= end) {  // (an eighth without a spike adds 0)
+                    tot = __fadd_rn(tot, sum);
+                    sum = 0.f;
+                    while (n >= end) end += a.HC;
+                }
+                sum = __fadd_rn(sum, __ldg(w + (size_t)n * a.R));
+            }
+        a.tot[((size_t)t * a.NC + q) * NS * a.R + pair] = __fadd_rn(tot, sum);
+    }
+}
+
+// The readouts over time: a thread per (sample, readout); MAX_AHEAD steps' sums loaded together (the loads' latency is
+// what it costs).
+constexpr int MAX_AHEAD = 32;
+__global__ void __launch_bounds__(32) readout_max_kernel(const __grid_constant__ Args a) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, n = a.B * a.R;
+    if (k >= n) return;
+    float O = 0.f, mx = -INFINITY;
+    int ts = -1;
+    float next[MAX_AHEAD];
+#pragma unroll
+    for (int j = 0; j < MAX_AHEAD; ++j) next[j] = j < a.T ? a.tot[(size_t)j * n + k] : 0.f;
+    for (int t0 = 0; t0 < a.T; t0 += MAX_AHEAD) {
+        float v[MAX_AHEAD];
+#pragma unroll
+        for (int j = 0; j < MAX_AHEAD; ++j) {
+            v[j] = next[j];
+            const int t = t0 + MAX_AHEAD + j;
+            next[j] = t < a.T ? a.tot[(size_t)t * n + k] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < MAX_AHEAD; ++j) {
+            if (t0 + j >= a.T) break;
+            O = __fadd_rn(__fmul_rn(a.beta, O), v[j]);
+            if (O > mx) {
+                mx = O;
+                ts = t0 + j;
+            }
+        }
+    }
+    a.m[k] = mx;
+    a.tstar[k] = ts;
+}
+
 // ------------------------------------------------------------------------------------------------ recompute
 
 // The recurrent input R of every step of a segment [t0, t1) from the stored spikes: NT threads per
@@ -488,71 +825,72 @@ __global__ void __launch_bounds__(256) recompute_v_kernel(const __grid_constant_
 
 // ------------------------------------------------------------------------------------------------ adjoint
 
-// One delay group of a neuron's outgoing row at step t: acc[b] += w q[t][post][b] over this thread's share
-// of the links (gs + sub, gs + sub + NT, ...), OUT_U links a round: all loads of a round (codes, weights, q
-// rows, dw) are issued before its arithmetic and stores, so that a round costs one chain of shared-memory
-// latencies. With DW (warp-uniform: some lane's neuron spiked at t - d), the lanes with `dwl` also add
-// sum_b s[b] q[t][post][b] to dw[l]. A skipped code (0xFFFF) reads row 0 and adds nothing.
-constexpr int OUT_U = 4;
+// The adjoint's threads: NB per neuron, one sample each -- or, in the link loops, LS link shares of a row times two
+// halves of the samples, a 16-byte load of a q row per lane. A step is bound by shared memory: 13,000 links per CTA
+// read 32 bytes of q each. What else the loads cost is kept down: a quarter warp reads four links of one neuron, whose
+// rows lie in different banks (32 bytes each, targets distinct mod 4: bank_order in bptt.py), lanes past a row's end
+// load nothing, and every neuron's loop ends at its own row. At 1024 hidden neurons of 102 links, 128 samples and
+// 500 steps: 5.3 ms (with 4 threads a neuron, a recomputation of each segment and a cluster barrier per step 6.9).
+
+// One delay group of a neuron's outgoing row: acc[b] += w q[post][4 half + b] over this lane's share of the links
+// (gs + sub, gs + sub + LS, ...). With DW (some lane's neuron spiked at the links' step), the lanes with `dwl` also
+// add sum_b s[b] q[post][b] to dw[l]: each half its samples' sum, then the pair's to dw by half 0. A skipped code
+// (0xFFFF) adds nothing. Every lane of the warp calls it; the loop's length is the warp's.
 template <bool SMOOTH, bool DW>
 __device__ __forceinline__ void out_group(const uint16_t *ocode, const float *ow, const float *pnew, float *dw,
-                                          int gs, int ge, int sub, bool dwl, uint32_t sbyte, const float *sf,
-                                          float acc[NS]) {
-    for (int base = gs + sub; base < ge; base += OUT_U * NT) {
-        uint32_t c[OUT_U];
-        float wl[OUT_U], od[OUT_U];
-        float4 y0[OUT_U], y1[OUT_U];
-        bool ok[OUT_U];
-#pragma unroll
-        for (int u = 0; u < OUT_U; ++u) {
-            const int l = base + u * NT;
-            c[u] = l < ge ? ocode[l] : 0xFFFFu;
-            wl[u] = l < ge ? ow[l] : 0.f;
+                                          int gs, int ge, int sub, int half, bool dwl, uint32_t sbyte,
+                                          const float sf[LS], float acc[LS]) {
+    const int rounds = (int)__reduce_max_sync(FULL, (unsigned)max(0, (ge - gs - sub + LS - 1) / LS));
+    const float4 *rows = reinterpret_cast<const float4 *>(pnew) + half;
+    int l = gs + sub;
+#pragma unroll 2
+    for (int k = 0; k < rounds; ++k, l += LS) {
+        const uint32_t c = l < ge ? ocode[l] : 0xFFFFu;
+        const bool ok = c != 0xFFFFu;
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+        float wl = 0.f;
+        if (ok) {
+            y = rows[2 * (c & 0x7FFu)];  // < H: checked when the rows were copied
+            wl = ow[l];
         }
-#pragma unroll
-        for (int u = 0; u < OUT_U; ++u) {
-            ok[u] = c[u] != 0xFFFFu;
-            const size_t post = ok[u] ? (c[u] & 0x7FFu) : 0u;  // < H: checked when the rows were copied
-            y0[u] = reinterpret_cast<const float4 *>(pnew)[post * (QROW / 4)];
-            y1[u] = reinterpret_cast<const float4 *>(pnew)[post * (QROW / 4) + 1];
-            if constexpr (DW) od[u] = (dwl && ok[u]) ? dw[base + u * NT] : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < OUT_U; ++u) {
-            if (!ok[u]) continue;
-            const float x[NS] = {y0[u].x, y0[u].y, y0[u].z, y0[u].w, y1[u].x, y1[u].y, y1[u].z, y1[u].w};
-#pragma unroll
-            for (int b = 0; b < NS; ++b) acc[b] = __fmaf_rn(wl[u], x[b], acc[b]);
-            if constexpr (DW) {
-                if (dwl) {
-                    float dk = 0.f;
-#pragma unroll
-                    for (int b = 0; b < NS; ++b) {
-                        if constexpr (SMOOTH) dk = __fmaf_rn(sf[b], x[b], dk);
-                        else if ((sbyte >> b) & 1u) dk = __fadd_rn(dk, x[b]);
-                    }
-                    dw[base + u * NT] = __fadd_rn(od[u], dk);
-                }
+        acc[0] = __fmaf_rn(wl, y.x, acc[0]);
+        acc[1] = __fmaf_rn(wl, y.y, acc[1]);
+        acc[2] = __fmaf_rn(wl, y.z, acc[2]);
+        acc[3] = __fmaf_rn(wl, y.w, acc[3]);
+        if constexpr (DW) {
+            float dk = 0.f;
+            if constexpr (SMOOTH) {
+                dk = __fmaf_rn(sf[3], y.w, __fmaf_rn(sf[2], y.z, __fmaf_rn(sf[1], y.y, __fmul_rn(sf[0], y.x))));
+            } else {
+                if (sbyte & 1u) dk = y.x;
+                if (sbyte & 2u) dk = __fadd_rn(dk, y.y);
+                if (sbyte & 4u) dk = __fadd_rn(dk, y.z);
+                if (sbyte & 8u) dk = __fadd_rn(dk, y.w);
             }
+            dk = __fadd_rn(dk, __shfl_xor_sync(FULL, dk, 1));
+            if (dwl && ok && half == 0) dw[l] = __fadd_rn(dw[l], dk);
         }
     }
 }
 
-// The adjoint of segment [t0, t1), run backwards; `first`: the last segment of the sequence (state starts at
+// The adjoint of the steps [t0, t1), run backwards; `first`: the last steps of the sequence (state starts at
 // zero), else the state of the segment after it is loaded (partial ring, q, readout adjoint, dw, dw_out).
-// Each step, every CTA writes the q[t] of its neurons into slot t & 1 of the group's ring in global memory,
-// arrives on the group's counter, waits for all 8 arrivals and copies q[t] of all H neurons into its own
-// shared buffer (pnew). Two slots suffice: a CTA writes slot t & 1 only after every CTA of the group arrived
-// at step t + 1, which each does after its copy of slot t & 1 at step t + 2. The launch is cooperative, so
-// the CTAs of a group are resident together; `g0` is the launch's first group.
-template <bool SMOOTH>
-__global__ void __launch_bounds__(512) bwd_kernel(const __grid_constant__ Args a, int out_cta_max, int t0, int t1,
-                                                   int first, int g0) {
+// Each step, every warp writes the q[t] of its four neurons into slot t & 1 of the group's ring in global memory and
+// releases a flag (the step's number + 1) after them; later (the links of q[t + 1] in between) every CTA polls the group's
+// flags and copies the q[t] of all H neurons into its own shared buffer (pnew). Two slots suffice: a slot t & 1 is written
+// only after its CTA has every q[t + 1], which each CTA releases after its copy of q[t + 2]. (Published like the
+// forward's words, q would be twice the bytes to copy: 5.75 ms for the kernel at the workload's size, 5.26 this way.)
+// The launch is cooperative, so the CTAs of a group are resident together; `g0` is the launch's first group.
+// FULL: all steps in one launch. What of a step does not depend on q is then made beforehand by kernels of its own --
+// the readout's part of dL/ds (readout_dV_kernel, left in dU, where q[t] takes its place) and dw_out (dwo_kernel).
+template <bool SMOOTH, bool FULL>
+__global__ void __launch_bounds__(NB * 128) bwd_kernel(const __grid_constant__ Args a, int out_cta_max, int t0, int t1,
+                                                       int first, int g0) {
     const int rank = (int)blockIdx.x % CL;
     const int q = g0 + (int)blockIdx.x / CL;
     const int H = a.H, HC = a.HC, R = a.R, B = a.B;
     const int h0 = rank * HC;
-    const BwdSmem L = bwd_smem(H, HC, R, out_cta_max);
+    const BwdSmem L = bwd_smem(H, HC, R, out_cta_max, FULL);
     extern __shared__ __align__(16) unsigned char smem[];
     float *pnew = reinterpret_cast<float *>(smem + L.pnew);
     float *part = reinterpret_cast<float *>(smem + L.part);
@@ -566,9 +904,11 @@ __global__ void __launch_bounds__(512) bwd_kernel(const __grid_constant__ Args a
     const int tid = threadIdx.x, nthr = blockDim.x;
     float *part_st = a.part_st + ((size_t)q * CL + rank) * RING * HC * NS;  // this group's CTA, in any launch
 
-    const bool nt = tid < NT * HC;
-    const int pl = nt ? tid / NT : 0, sub = tid % NT;
-    const int me = h0 + pl;  // this thread's neuron (the pre of its outgoing row)
+    const bool nt = tid < NB * HC;
+    const int pl = nt ? tid / NB : 0;                 // the thread's neuron
+    const int half = tid & 1, sub = (tid >> 1) % LS;  // in the link loops: its half of the samples, its share
+    const int own = LS * half + sub;                  // its sample
+    const int me = h0 + pl;                           // its neuron (the pre of its outgoing row)
     const int obase = a.out_grp[(size_t)h0 * (MAXD + 1)];
     const int on_all = a.out_grp[(size_t)(h0 + HC - 1) * (MAXD + 1) + MAXD] - obase;
     const int on = min(on_all, out_cta_max);  // a wrong out_cta_max: the links past it are skipped, counted
@@ -582,7 +922,7 @@ __global__ void __launch_bounds__(512) bwd_kernel(const __grid_constant__ Args a
         for (int d = 1; d <= MAXD; ++d) {
             const int gs = min(a.out_grp[(size_t)me * (MAXD + 1) + d - 1] - obase, on);
             const int ge = min(a.out_grp[(size_t)me * (MAXD + 1) + d] - obase, on);
-            for (int l = gs + sub; l < ge; l += NT) {
+            for (int l = gs + own; l < ge; l += NB) {
                 const uint32_t c = a.out_code[obase + l];
                 const bool bad = (int)(c >> 11) != d || (c & 0x7FFu) >= (uint32_t)H;
                 if (bad) atomicAdd(a.err + 0, 1);
@@ -599,74 +939,62 @@ __global__ void __launch_bounds__(512) bwd_kernel(const __grid_constant__ Args a
     __shared__ int aborted;
     if (tid == 0) aborted = 0;
     __syncthreads();
-    uint32_t *xcnt = a.xcnt + q;
-    uint32_t target = 0;
 
-    const size_t bq = (size_t)q * NS + SPT * sub;
-    const bool ro = tid < NS * R;
+    const size_t bq = (size_t)q * NS + own;  // this thread's sample
+    const bool ro = !FULL && tid < NS * R;
     const int rb = ro ? tid / R : 0, rr = ro ? tid % R : 0;
     const float dmv = ro ? a.dm[(size_t)(q * NS + rb) * R + rr] : 0.f;
     const int tsv = ro ? a.tstar_in[(size_t)(q * NS + rb) * R + rr] : -1;
     float o = (ro && !first) ? a.o_st[(size_t)(q * NS + rb) * R + rr] : 0.f;
-    float qp0 = 0.f, qp1 = 0.f;  // q[t + 1] of this thread's two samples
-    if (nt && !first) {
-        qp0 = a.q_st[bq * H + me];
-        qp1 = a.q_st[(bq + 1) * H + me];
-    }
-    const int R4 = (R + NT - 1) / NT;
+    float qp = (nt && !first) ? a.q_st[bq * H + me] : 0.f;  // q[t + 1] of this thread's sample
 
-    // this neuron's 8 samples' spikes at step tt (0 before step 0): a byte of bits, or floats in the smooth model
-    auto spikes_at = [&](int tt, float out[NS], uint32_t &byte) {
-        byte = 0;
+    // this neuron's spikes at step tt (0 before step 0): the 8 samples' bits, or (smooth) the floats of this lane's
+    // half of the samples
+    auto spikes_at = [&](int tt, float out[LS]) -> uint32_t {
         if constexpr (SMOOTH) {
 #pragma unroll
-            for (int b = 0; b < NS; ++b) out[b] = 0.f;
-            if (tt < 0 || !nt) return;
-            const float4 *src = reinterpret_cast<const float4 *>(a.s_f) + (((size_t)tt * a.NC + q) * H + me) * 2;
-            const float4 x = src[0], y = src[1];
+            for (int b = 0; b < LS; ++b) out[b] = 0.f;
+            if (tt < 0 || !nt) return 0u;
+            const float4 x = reinterpret_cast<const float4 *>(a.s_f)[(((size_t)tt * a.NC + q) * H + me) * 2 + half];
             out[0] = x.x; out[1] = x.y; out[2] = x.z; out[3] = x.w;
-            out[4] = y.x; out[5] = y.y; out[6] = y.z; out[7] = y.w;
-            byte = 0xffu;
+            return 0xffu;
         } else {
             (void)out;
-            if (tt < 0 || !nt) return;
-            byte = a.s_bits[((size_t)tt * a.NC + q) * H + me];
+            return (tt < 0 || !nt) ? 0u : a.s_bits[((size_t)tt * a.NC + q) * H + me];
         }
     };
     uint64_t hist = 0;      // spiking: byte d - 1 = the 8 samples' spikes at t - d
-    float histf[MAXD][NS];  // smooth: histf[d - 1] = spikes at t - d
+    float histf[MAXD][LS];  // smooth: histf[d - 1] = spikes at t - d
     for (int d = 1; d <= MAXD; ++d) {
-        uint32_t byte;
-        spikes_at(t1 - 1 - d, histf[d - 1], byte);
+        const uint32_t byte = spikes_at(t1 - 1 - d, histf[d - 1]);
         if constexpr (!SMOOTH) hist |= (uint64_t)byte << (8 * (d - 1));
     }
     // the surrogate derivatives and spikes of the next step down, loaded one step ahead
-    auto g_at = [&](int tt, int j) { return nt ? a.g_seg[((size_t)(tt - t0) * B + bq + j) * H + me] : 0.f; };
-    float gn0 = g_at(t1 - 1, 0), gn1 = g_at(t1 - 1, 1);
-    float stn[NS];
-    uint32_t sbn;
-    spikes_at(t1 - 1, stn, sbn);
+    auto g_at = [&](int tt) { return nt ? __ldcs(a.g_seg + ((size_t)(tt - t0) * B + bq) * H + me) : 0.f; };
+    float gn = g_at(t1 - 1);
+    auto y_at = [&](int tt) { return (FULL && nt) ? a.dU[((size_t)tt * B + bq) * H + me] : 0.f; };
+    float yn = y_at(t1 - 1);
+    float stn[LS];
+    uint32_t sbn = spikes_at(t1 - 1, stn);
     // outgoing rows of neuron me, delay group d, at step u (q[u] in pnew): partial[u - d] += w q[u][post];
     // dw += s[u - d][me] q[u][post] (sbyte, sf: the spikes at u - d). Every thread of the CTA calls it.
     auto out_rows = [&](int u, int d, uint32_t sbyte, const float *sf) {
-        float acc[NS];
+        float acc[LS];
 #pragma unroll
-        for (int b = 0; b < NS; ++b) acc[b] = 0.f;
+        for (int b = 0; b < LS; ++b) acc[b] = 0.f;
         const int gs = nt ? grp[pl * (MAXD + 1) + d - 1] : 0, ge = nt ? grp[pl * (MAXD + 1) + d] : 0;
         if (__any_sync(FULL, sbyte != 0u))  // the same branch for the whole warp
-            out_group<SMOOTH, true>(ocode, ow, pnew, dw, gs, ge, sub, sbyte != 0u, sbyte, sf, acc);
+            out_group<SMOOTH, true>(ocode, ow, pnew, dw, gs, ge, sub, half, sbyte != 0u, sbyte >> (LS * half), sf, acc);
         else
-            out_group<SMOOTH, false>(ocode, ow, pnew, dw, gs, ge, sub, false, 0u, sf, acc);
-#pragma unroll
-        for (int b = 0; b < NS; ++b) acc[b] = __fadd_rn(acc[b], __shfl_xor_sync(FULL, acc[b], 1));
-#pragma unroll
-        for (int b = 0; b < NS; ++b) acc[b] = __fadd_rn(acc[b], __shfl_xor_sync(FULL, acc[b], 2));
+            out_group<SMOOTH, false>(ocode, ow, pnew, dw, gs, ge, sub, half, false, 0u, sf, acc);
+        // the shares added pairwise, two samples fewer to carry each time: ends with the lane's sample 4 half + sub
+        const float k0 = (sub & 1) ? acc[1] : acc[0], k1 = (sub & 1) ? acc[3] : acc[2];
+        const float s0 = (sub & 1) ? acc[0] : acc[1], s1 = (sub & 1) ? acc[2] : acc[3];
+        const float e0 = __fadd_rn(k0, __shfl_xor_sync(FULL, s0, 2)), e1 = __fadd_rn(k1, __shfl_xor_sync(FULL, s1, 2));
+        const float x = __fadd_rn((sub & 2) ? e1 : e0, __shfl_xor_sync(FULL, (sub & 2) ? e0 : e1, 4));
         if (nt && u - d >= 0) {
-            float x0, x1;
-            mine(acc, sub, x0, x1);
-            float *pp = part + ((size_t)((u - d) % RING) * HC + pl) * NS + SPT * sub;
-            pp[0] = __fadd_rn(pp[0], x0);
-            pp[1] = __fadd_rn(pp[1], x1);
+            float *pp = part + ((size_t)((u - d) % RING) * HC + pl) * NS + LS * half + sub;
+            *pp = __fadd_rn(*pp, x);
         }
     };
     // the readout adjoint o[t] does not depend on q: it is made one step ahead, into the other half of obuf, so
@@ -675,46 +1003,58 @@ __global__ void __launch_bounds__(512) bwd_kernel(const __grid_constant__ Args a
         o = __fadd_rn(t1 - 1 == tsv ? dmv : 0.f, __fmul_rn(a.beta, o));
         obuf[(size_t)((t1 - 1) & 1) * NS * R + rb * R + rr] = o;
     }
-    __syncthreads();  // o[t1 - 1] ready
+    if (!FULL) __syncthreads();  // o[t1 - 1] ready
     for (int t = t1 - 1; t >= t0; --t) {
         const float *ob = obuf + (size_t)(t & 1) * NS * R;  // o[t]
-        float qv0 = 0.f, qv1 = 0.f;
-        float st[NS];
+        float st[LS];
 #pragma unroll
-        for (int b = 0; b < NS; ++b) st[b] = stn[b];
+        for (int b = 0; b < LS; ++b) st[b] = stn[b];
         const uint32_t sbyte_t = sbn;
-        const float gc0 = gn0, gc1 = gn1;
+        const float gc = gn, yc = yn;
         if (t > t0) {
-            gn0 = g_at(t - 1, 0);
-            gn1 = g_at(t - 1, 1);
-            spikes_at(t - 1, stn, sbn);
+            gn = g_at(t - 1);
+            yn = y_at(t - 1);
+            sbn = spikes_at(t - 1, stn);
         }
+        float *slot = a.qx + ((size_t)q * 2 + (t & 1)) * H * NS;
+        uint32_t *flags = a.qflag + ((size_t)q * 2 + (t & 1)) * (H / 4);
         if (nt) {
-#pragma unroll
-            for (int j = 0; j < SPT; ++j) {
-                const int bl = SPT * sub + j;
-                float *pp = part + ((size_t)(t % RING) * HC + pl) * NS + bl;
-                float sh = *pp;
-                for (int r = 0; r < R; ++r) sh = __fmaf_rn(__ldg(wout + pl * R + r), ob[bl * R + r], sh);
-                *pp = 0.f;
-                const float g = j ? gc1 : gc0;
-                const float ap = __fmul_rn(a.alpha, j ? qp1 : qp0);
-                const float qv = __fmaf_rn(g, __fmaf_rn(-a.theta, ap, sh), ap);
-                a.dU[((size_t)t * B + bq + j) * H + me] = qv;
-                if (j) qv1 = qv;
-                else qv0 = qv;
+            float *pp = part + ((size_t)(t % RING) * HC + pl) * NS + own;
+            float sh = *pp;
+            if constexpr (FULL) {
+                sh = __fadd_rn(sh, yc);
+            } else {
+#pragma unroll 4
+                for (int r = 0; r < R; ++r) sh = __fmaf_rn(__ldg(wout + pl * R + r), ob[own * R + r], sh);
             }
-            qp0 = qv0;
-            qp1 = qv1;
-            // dw_out: this neuron's spikes at t times o[t]; each of its NT threads takes a quarter of the readouts
-            if (sbyte_t) {
-                for (int r = sub * R4; r < min(R, (sub + 1) * R4); ++r) {
-                    float acc = dwo[pl * R + r];
-                    for (int b = 0; b < NS; ++b) {
-                        if constexpr (SMOOTH) acc = __fmaf_rn(st[b], ob[b * R + r], acc);
-                        else if ((sbyte_t >> b) & 1u) acc = __fadd_rn(acc, ob[b * R + r]);
+            *pp = 0.f;
+            const float ap = __fmul_rn(a.alpha, qp);
+            qp = __fmaf_rn(gc, __fmaf_rn(-a.theta, ap, sh), ap);
+            slot[(size_t)me * NS + own] = qp;
+        }
+        __syncwarp();
+        if (nt && (tid & 31) == 0)
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + me / 4), "r"((uint32_t)t + 1u) : "memory");
+        // while the group's other values arrive: what nothing waits for
+        if (nt) {
+            __stcs(a.dU + ((size_t)t * B + bq) * H + me, qp);
+            // dw_out: this neuron's spikes at t times o[t]; each of its NB threads takes an eighth of the readouts
+            if (!FULL && sbyte_t) {
+                if constexpr (SMOOTH) {
+                    // a lane holds half of the samples' spikes: its half's sum to the readout, the halves in turn
+                    for (int r = sub; r < R; r += LS) {
+                        float acc = 0.f;
+#pragma unroll
+                        for (int b = 0; b < LS; ++b) acc = __fmaf_rn(st[b], ob[(LS * half + b) * R + r], acc);
+                        acc = __fadd_rn(acc, __shfl_xor_sync(3u << (tid & 30), acc, 1));
+                        if (half == 0) dwo[pl * R + r] = __fadd_rn(dwo[pl * R + r], acc);
                     }
-                    dwo[pl * R + r] = acc;
+                } else {
+                    for (int r = own; r < R; r += NB) {
+                        float acc = dwo[pl * R + r];
+                        for (uint32_t m = sbyte_t; m; m &= m - 1) acc = __fadd_rn(acc, ob[(__ffs(m) - 1) * R + r]);
+                        dwo[pl * R + r] = acc;
+                    }
                 }
             }
         }
@@ -722,34 +1062,35 @@ __global__ void __launch_bounds__(512) bwd_kernel(const __grid_constant__ Args a
             o = __fadd_rn(t - 1 == tsv ? dmv : 0.f, __fmul_rn(a.beta, o));
             obuf[(size_t)((t - 1) & 1) * NS * R + rb * R + rr] = o;
         }
-        float *slot = a.qx + ((size_t)q * 2 + (t & 1)) * H * NS;
-        if (nt) reinterpret_cast<float2 *>(slot)[(size_t)me * (NS / 2) + sub] = make_float2(qv0, qv1);
-        __syncthreads();  // this CTA's q[t] written
-        target += CL;
-        if (tid == 0) group_arrive(xcnt);
-        // while the group's other CTAs arrive: step t + 1's delay groups 2..5 (pnew still holds q[t + 1]; their
-        // partials are for steps t - 1 and earlier, so only the delay-1 group waits for q[t])
+        // step t + 1's delay groups 2..5 (pnew still holds q[t + 1]; their partials are for steps t - 1 and earlier,
+        // so only the delay-1 group waits for q[t])
         if (t + 1 < t1) {
 #pragma unroll
             for (int d = 2; d <= MAXD; ++d)
                 out_rows(t + 1, d, SMOOTH ? 0xffu : (uint32_t)((hist >> (8 * (d - 2))) & 0xffu), histf[d - 2]);
         }
-        if (tid == 0) group_wait(xcnt, target, a.err, a.wait_polls, aborted);
-        __syncthreads();  // every CTA's q[t] written, every read of q[t + 1] done: copy q[t] (past L1) into pnew
+        if (tid < H / 4 && !*(volatile int *)&aborted) {
+            bool there = false;
+            for (int it = 0; it < a.wait_polls && !there; ++it) {
+                uint32_t v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flags + tid) : "memory");
+                there = v == (uint32_t)t + 1u;
+            }
+            if (!there) {
+                atomicAdd(a.err + 3, 1);
+                *(volatile int *)&aborted = 1;
+            }
+        }
+        __syncthreads();  // every CTA's q[t] written, every read of q[t + 1] done: q[t] (past L1) into pnew
         for (int j = tid; j < H * (NS / 4); j += nthr)
-            reinterpret_cast<float4 *>(pnew)[(size_t)(j >> 1) * (QROW / 4) + (j & 1)] =
-                __ldcg(reinterpret_cast<const float4 *>(slot) + j);
+            reinterpret_cast<float4 *>(pnew)[j] = __ldcg(reinterpret_cast<const float4 *>(slot) + j);
         __syncthreads();
         out_rows(t, 1, SMOOTH ? 0xffu : (uint32_t)(hist & 0xffu), histf[0]);
         // the spike history of step t - 1: delays 1..5 reach t - 2 .. t - 6
         if constexpr (SMOOTH) {
-            for (int d = 1; d <= MAXD; ++d) {
-                uint32_t byte;
-                spikes_at(t - 1 - d, histf[d - 1], byte);
-            }
+            for (int d = 1; d <= MAXD; ++d) spikes_at(t - 1 - d, histf[d - 1]);
         } else {
-            uint32_t byte;
-            spikes_at(t - 1 - MAXD, histf[0], byte);
+            const uint32_t byte = spikes_at(t - 1 - MAXD, histf[0]);
             hist = (hist >> 8) | ((uint64_t)byte << (8 * (MAXD - 1)));
         }
     }
@@ -759,14 +1100,96 @@ __global__ void __launch_bounds__(512) bwd_kernel(const __grid_constant__ Args a
         out_rows(t0, d, SMOOTH ? 0xffu : (uint32_t)((hist >> (8 * (d - 2))) & 0xffu), histf[d - 2]);
     // the state for the segment before this one
     __syncthreads();
-    for (int k = tid; k < RING * HC * NS; k += nthr) part_st[k] = part[k];
     for (int k = tid; k < on; k += nthr) a.dwp[(size_t)q * a.nnz + obase + k] = dw[k];
-    for (int k = tid; k < HC * R; k += nthr) a.dwo_p[((size_t)q * H + h0) * R + k] = dwo[k];
-    if (nt) {
-        a.q_st[bq * H + me] = qp0;
-        a.q_st[(bq + 1) * H + me] = qp1;
+    if constexpr (!FULL) {
+        for (int k = tid; k < RING * HC * NS; k += nthr) part_st[k] = part[k];
+        for (int k = tid; k < HC * R; k += nthr) a.dwo_p[((size_t)q * H + h0) * R + k] = dwo[k];
+        if (nt) a.q_st[bq * H + me] = qp;
+        if (ro && rank == 0) a.o_st[(size_t)(q * NS + rb) * R + rr] = o;
     }
-    if (ro && rank == 0) a.o_st[(size_t)(q * NS + rb) * R + rr] = o;
+}
+
+// FULL, before the adjoint: the readout adjoint of every step, a thread per (sample, readout), last step first.
+__global__ void __launch_bounds__(64) readout_adjoint_kernel(const __grid_constant__ Args a) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, n = a.B * a.R;
+    if (k >= n) return;
+    const float dm = a.dm[k];
+    const int ts = a.tstar_in[k];
+    float o = 0.f;
+    for (int t = a.T - 1; t >= 0; --t) {
+        o = __fadd_rn(t == ts ? dm : 0.f, __fmul_rn(a.beta, o));
+        a.o_all[(size_t)t * n + k] = o;
+    }
+}
+
+// FULL, before the adjoint: dU[t][b][i] = sum_r w_out[i][r] o[t][b][r], a thread per two neurons with their rows of w_out
+// in registers (R4 groups of four readouts), DV_ROWS (t, b) rows per block. Bound by the write of dU.
+constexpr int DV_ROWS = 32;
+template <int R4>
+__global__ void __launch_bounds__(256) readout_dV_kernel(const __grid_constant__ Args a) {
+    __shared__ float4 o[DV_ROWS][R4];
+    const int pairs = a.H / 2, i = blockIdx.y * blockDim.x + threadIdx.x, n = a.T * a.B;
+    const int r0 = blockIdx.x * DV_ROWS, rows = min(DV_ROWS, n - r0);
+    for (int k = threadIdx.x; k < DV_ROWS * R4 * 4; k += blockDim.x) {
+        const int row = k / (R4 * 4), r = k % (R4 * 4);
+        reinterpret_cast<float *>(o)[k] = (row < rows && r < a.R) ? a.o_all[(size_t)(r0 + row) * a.R + r] : 0.f;
+    }
+    float w[2][R4 * 4];
+#pragma unroll
+    for (int r = 0; r < R4 * 4; ++r) {
+        const bool in = i < pairs && r < a.R;
+        w[0][r] = in ? a.w_out[(size_t)(2 * i) * a.R + r] : 0.f;
+        w[1][r] = in ? a.w_out[(size_t)(2 * i + 1) * a.R + r] : 0.f;
+    }
+    __syncthreads();
+    if (i >= pairs) return;
+    for (int k = 0; k < rows; ++k) {
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int r = 0; r < R4; ++r) {
+            const float4 v = o[k][r];
+            s0 = __fmaf_rn(w[0][4 * r], v.x, s0);
+            s1 = __fmaf_rn(w[1][4 * r], v.x, s1);
+            s0 = __fmaf_rn(w[0][4 * r + 1], v.y, s0);
+            s1 = __fmaf_rn(w[1][4 * r + 1], v.y, s1);
+            s0 = __fmaf_rn(w[0][4 * r + 2], v.z, s0);
+            s1 = __fmaf_rn(w[1][4 * r + 2], v.z, s1);
+            s0 = __fmaf_rn(w[0][4 * r + 3], v.w, s0);
+            s1 = __fmaf_rn(w[1][4 * r + 3], v.w, s1);
+        }
+        __stcs(reinterpret_cast<float2 *>(a.dU + (size_t)(r0 + k) * a.H) + i, make_float2(s0, s1));
+    }
+}
+
+// FULL: dw_out's partial sums, chunk c of NC of the steps: dwo_p[c][i][r] = sum over the chunk's spikes of neuron i of
+// o[t][b][r]. A warp per four neurons (one word of spikes per step and group), a lane per readout.
+__global__ void __launch_bounds__(256) dwo_kernel(const __grid_constant__ Args a) {
+    const int lane = threadIdx.x & 31, word = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, c = blockIdx.y;
+    if (word >= a.H / 4) return;
+    const int t0 = (int)((long long)a.T * c / a.NC), t1 = (int)((long long)a.T * (c + 1) / a.NC);
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(a.s_bits) + word;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const int n = (t1 - t0) * a.NC;  // (step, group) pairs
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        // 32 pairs' words, a lane each; then those with a spike, in order
+        const uint32_t mine = k0 + lane < n ? src[((size_t)t0 * a.NC + k0 + lane) * (a.H / 4)] : 0u;
+        for (uint32_t some = __ballot_sync(FULL, mine != 0u); some; some &= some - 1) {
+            const int k = k0 + __ffs(some) - 1;
+            const uint32_t w = __shfl_sync(FULL, mine, k - k0);
+            const float *o = a.o_all + ((size_t)t0 * a.NC + k) * NS * a.R + lane;  // (t, q): samples 8q ..
+            for (uint32_t m = w; m; m &= m - 1) {
+                const int bit = __ffs(m) - 1;
+                const float v = lane < a.R ? __ldg(o + (bit & 7) * a.R) : 0.f;
+                if (bit < 8) acc[0] = __fadd_rn(acc[0], v);
+                else if (bit < 16) acc[1] = __fadd_rn(acc[1], v);
+                else if (bit < 24) acc[2] = __fadd_rn(acc[2], v);
+                else acc[3] = __fadd_rn(acc[3], v);
+            }
+        }
+    }
+    if (lane < a.R)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a.dwo_p[((size_t)c * a.H + 4 * word + j) * a.R + lane] = acc[j];
 }
 
 // dw_rec in the caller's (incoming, canonical) order: the clusters' partials added in cluster order.
@@ -885,8 +1308,13 @@ int bcuda(cudaError_t e, const char *what) {
         if (_e != cudaSuccess) return bcuda(_e, #call); \
     } while (0)
 
+// A taped forward keeps the surrogate derivatives of every step when they take at most this much (the workload's
+// 128 x 500 x 1024 are 262 MB): 0.04 ms of writes under the forward instead of 0.18 ms of recomputing per segment of
+// 50 steps, of which the adjoint hides half. Larger layers keep the membrane every `checkpoint` steps and recompute.
+constexpr size_t FULL_TAPE_BYTES = (size_t)4 << 30;
+
 struct WsLayout {
-    size_t spikes, vck, gseg, outw, dwp, dwo, part, qst, ost, qx, xcnt, err, total;
+    size_t spikes, plain, xw, tot, vck, gseg, outw, dwp, dwo, part, qst, ost, qx, qflag, err, total;
 };
 
 size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -909,14 +1337,27 @@ int check_desc(const n2b_bptt_desc *d) {
     return N2B_OK;
 }
 
+// The forward runs fwd_group_kernel: its rows fit shared memory.
+bool scans(const n2b_bptt_desc *d) {
+    return !d->smooth && scan_smem(d->hidden, d->hidden / CL, d->in_cta_max).total <= SMEM_MAX - 1024;
+}
+
+bool full_tape(const n2b_bptt_desc *d) {
+    return scans(d) && sizeof(float) * (size_t)d->steps * d->batch * d->hidden <= FULL_TAPE_BYTES;
+}
+
 WsLayout ws_layout(const n2b_bptt_desc *d) {
     WsLayout L{};
     const size_t T = d->steps, B = d->batch, H = d->hidden, R = d->readouts, NC = B / NS;
     const size_t nseg = (T + d->checkpoint - 1) / d->checkpoint, K = std::min<size_t>(d->checkpoint, T);
     size_t o = 0;
     L.spikes = o; o = a256(o + (d->smooth ? sizeof(float) * T * NC * H * NS : T * NC * H));
-    L.vck = o; o = a256(o + sizeof(float) * nseg * B * H);
-    L.gseg = o; o = a256(o + sizeof(float) * 2 * K * B * H);  // two segments: one recomputed, one run back
+    L.plain = o; o = a256(o + (scans(d) ? T * NC * H : 0));
+    L.xw = o; o = a256(o + (scans(d) ? sizeof(unsigned long long) * NC * XSLOTS * (H / 4) : 0));
+    L.tot = o; o = a256(o + (scans(d) ? sizeof(float) * T * B * R : 0));
+    L.vck = o; o = a256(o + (full_tape(d) ? 0 : sizeof(float) * nseg * B * H));
+    // every step, or two segments: one recomputed, one run back
+    L.gseg = o; o = a256(o + sizeof(float) * (full_tape(d) ? T : 2 * K) * B * H);
     L.outw = o; o = a256(o + sizeof(float) * std::max<size_t>(d->nnz, 1));
     L.dwp = o; o = a256(o + sizeof(float) * NC * std::max<size_t>(d->nnz, 1));
     L.dwo = o; o = a256(o + sizeof(float) * NC * H * R);
@@ -924,14 +1365,14 @@ WsLayout ws_layout(const n2b_bptt_desc *d) {
     L.qst = o; o = a256(o + sizeof(float) * B * H);
     L.ost = o; o = a256(o + sizeof(float) * B * R);
     L.qx = o; o = a256(o + sizeof(float) * NC * 2 * H * NS);
-    L.xcnt = o; o = a256(o + sizeof(uint32_t) * NC);
+    L.qflag = o; o = a256(o + sizeof(uint32_t) * NC * 2 * (H / 4));
     L.err = o; o = a256(o + sizeof(int32_t) * N2B_BPTT_ERR_WORDS);
     L.total = o;
     return L;
 }
 
-int threads_of(const n2b_bptt_desc *d) {
-    const int n = std::max(NT * (d->hidden / CL), NS * d->readouts);
+int threads_of(const n2b_bptt_desc *d, int per_neuron) {
+    const int n = std::max(per_neuron * (d->hidden / CL), NS * d->readouts);
     return (n + 31) / 32 * 32;
 }
 
@@ -956,8 +1397,12 @@ Args args_of(const n2b_bptt_desc *d, char *ws, const WsLayout &L) {
     a.out_code = d->out_code;
     a.s_bits = reinterpret_cast<uint8_t *>(ws + L.spikes);
     a.s_f = reinterpret_cast<float *>(ws + L.spikes);
+    a.s_plain = reinterpret_cast<uint8_t *>(ws + L.plain);
+    a.xw = reinterpret_cast<unsigned long long *>(ws + L.xw);
+    a.tot = reinterpret_cast<float *>(ws + L.tot);
     a.v_ckpt = reinterpret_cast<float *>(ws + L.vck);
     a.g_seg = reinterpret_cast<float *>(ws + L.gseg);
+    a.g_all = full_tape(d) ? a.g_seg : nullptr;
     a.out_w = reinterpret_cast<float *>(ws + L.outw);
     a.dwp = reinterpret_cast<float *>(ws + L.dwp);
     a.dwo_p = reinterpret_cast<float *>(ws + L.dwo);
@@ -965,7 +1410,8 @@ Args args_of(const n2b_bptt_desc *d, char *ws, const WsLayout &L) {
     a.q_st = reinterpret_cast<float *>(ws + L.qst);
     a.o_st = reinterpret_cast<float *>(ws + L.ost);
     a.qx = reinterpret_cast<float *>(ws + L.qx);
-    a.xcnt = reinterpret_cast<uint32_t *>(ws + L.xcnt);
+    a.qflag = reinterpret_cast<uint32_t *>(ws + L.qflag);
+    a.o_all = a.tot;
     a.err = reinterpret_cast<int32_t *>(ws + L.err);
     a.wait_polls = d->wait_polls > 0 ? d->wait_polls : XCHG_SPIN_LIMIT;
     return a;
@@ -1095,10 +1541,28 @@ int n2b_bptt_forward(const n2b_bptt_desc *d, const float *u, const float *w_rec,
     a.tstar = tstar;
     B_CUDA(cudaMemsetAsync(ws + L.err, 0, sizeof(int32_t) * N2B_BPTT_ERR_WORDS, s));
     const bool smooth = d->smooth != 0;
+    const int grid = (d->batch / NS) * CL, threads = threads_of(d, NT);
+    if (scans(d)) {
+        const int NC = d->batch / NS, gthreads = (NB * (d->hidden / CL) + 31) / 32 * 32;
+        const size_t smem = scan_smem(d->hidden, d->hidden / CL, d->in_cta_max).total;
+        int per_launch = 0;  // groups per cooperative launch
+        rc = coop_groups(fwd_group_kernel, gthreads, smem, per_launch);
+        if (rc) return rc;
+        B_CUDA(cudaMemsetAsync(a.xw, 0, sizeof(unsigned long long) * NC * XSLOTS * (d->hidden / 4), s));
+        for (int g0 = 0; g0 < NC; g0 += per_launch) {
+            rc = launch_coop(fwd_group_kernel, std::min(per_launch, NC - g0) * CL, gthreads, smem, s, a, d->in_cta_max,
+                             g0);
+            if (rc) return rc;
+        }
+        readout_kernel<<<dim3((unsigned)d->steps, (unsigned)NC), READOUT_THREADS, 0, s>>>(a);
+        B_CUDA(cudaGetLastError());
+        readout_max_kernel<<<(unsigned)((d->batch * d->readouts + 31) / 32), 32, 0, s>>>(a);
+        B_CUDA(cudaGetLastError());
+        return N2B_OK;
+    }
     FwdSmem S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, true, d->in_cta_max);
     a.csr_smem = S.total <= 200 * 1024;
     if (!a.csr_smem) S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, false, 0);
-    const int grid = (d->batch / NS) * CL, threads = threads_of(d);
     return smooth ? launch_cluster(fwd_kernel<true>, grid, threads, S.total, s, a, d->in_cta_max)
                   : launch_cluster(fwd_kernel<false>, grid, threads, S.total, s, a, d->in_cta_max);
 }
@@ -1126,14 +1590,16 @@ int n2b_bptt_backward(const n2b_bptt_desc *d, const float *u, const float *w_rec
         B_CUDA(cudaGetLastError());
     }
     const bool smooth = d->smooth != 0;
-    const BwdSmem S = bwd_smem(d->hidden, d->hidden / CL, d->readouts, d->out_cta_max);
-    const int NC = d->batch / NS, threads = threads_of(d);
-    const int K = d->checkpoint, nseg = a.nseg;
+    const int NC = d->batch / NS, threads = threads_of(d, NB);
+    const bool full = full_tape(d);  // the adjoint of all steps in one launch, nothing to recompute
+    const BwdSmem S = bwd_smem(d->hidden, d->hidden / CL, d->readouts, d->out_cta_max, full);
+    const int K = full ? d->steps : d->checkpoint, nseg = full ? 1 : a.nseg;
     const int rthreads = d->hidden % 64 == 0 ? 256 : 128;  // whole neurons of NT threads; hidden % 32 == 0
     const size_t rsmem = smooth ? 0 : (size_t)16 * d->hidden;  // the staged spike rows
     int per_launch = 0;  // groups per cooperative launch
-    rc = smooth ? coop_groups(bwd_kernel<true>, threads, S.total, per_launch)
-                : coop_groups(bwd_kernel<false>, threads, S.total, per_launch);
+    rc = smooth ? coop_groups(bwd_kernel<true, false>, threads, S.total, per_launch)
+         : full ? coop_groups(bwd_kernel<false, true>, threads, S.total, per_launch)
+                : coop_groups(bwd_kernel<false, false>, threads, S.total, per_launch);
     if (rc) return rc;
     SideStreams st;
     rc = side_streams(st);
@@ -1144,7 +1610,7 @@ int n2b_bptt_backward(const n2b_bptt_desc *d, const float *u, const float *w_rec
     B_CUDA(cudaEventRecord(fork, s));
     B_CUDA(cudaStreamWaitEvent(st.hi, fork, 0));
     B_CUDA(cudaStreamWaitEvent(st.lo, fork, 0));
-    float *gbuf[2] = {a.g_seg, a.g_seg + (size_t)std::min(K, d->steps) * d->batch * d->hidden};
+    float *gbuf[2] = {a.g_seg, full ? a.g_seg : a.g_seg + (size_t)std::min(K, d->steps) * d->batch * d->hidden};
     // segment seg recomputed from its checkpoint into gbuf[seg & 1] on the low-priority stream
     auto recompute = [&](int seg) -> int {
         const int t0 = seg * K, t1 = std::min(d->steps, t0 + K);
@@ -1165,21 +1631,47 @@ int n2b_bptt_backward(const n2b_bptt_desc *d, const float *u, const float *w_rec
     };
     // Segments run backwards. The recompute of segment seg - 1 overlaps the adjoint of seg; it reuses the buffer
     // of seg + 1, so it waits for that adjoint.
-    rc = recompute(nseg - 1);
+    B_CUDA(cudaMemsetAsync(a.qflag, 0, sizeof(uint32_t) * NC * 2 * (d->hidden / 4), st.hi));
+    if (full) {  // what does not depend on q: the readout's part of dU on this stream, dw_out beside the adjoint
+        readout_adjoint_kernel<<<(unsigned)((d->batch * d->readouts + 63) / 64), 64, 0, st.hi>>>(a);
+        B_CUDA(cudaGetLastError());
+        B_CUDA(cudaEventRecord(rec[0], st.hi));
+        B_CUDA(cudaStreamWaitEvent(st.lo, rec[0], 0));
+        dwo_kernel<<<dim3((unsigned)((d->hidden / 4 + 7) / 8), (unsigned)NC), 256, 0, st.lo>>>(a);
+        B_CUDA(cudaGetLastError());
+        B_CUDA(cudaEventRecord(rec[1], st.lo));
+        const int vthreads = std::min(256, d->hidden / 2);
+        const dim3 vgrid((unsigned)(((int64_t)d->steps * d->batch + DV_ROWS - 1) / DV_ROWS),
+                         (unsigned)((d->hidden / 2 + vthreads - 1) / vthreads));
+        switch ((d->readouts + 3) / 4) {
+            case 1: readout_dV_kernel<1><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+            case 2: readout_dV_kernel<2><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+            case 3: readout_dV_kernel<3><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+            case 4: readout_dV_kernel<4><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+            case 5: readout_dV_kernel<5><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+            case 6: readout_dV_kernel<6><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+            case 7: readout_dV_kernel<7><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+            default: readout_dV_kernel<8><<<vgrid, vthreads, 0, st.hi>>>(a); break;
+        }
+        B_CUDA(cudaGetLastError());
+    } else {
+        rc = recompute(nseg - 1);
+    }
     if (rc) return rc;
     for (int seg = nseg - 1; seg >= 0; --seg) {
         const int t0 = seg * K, t1 = std::min(d->steps, t0 + K);
         const int first = seg == nseg - 1;
         Args ba = a;
         ba.g_seg = gbuf[seg & 1];
-        B_CUDA(cudaStreamWaitEvent(st.hi, rec[seg & 1], 0));
-        B_CUDA(cudaMemsetAsync(a.xcnt, 0, sizeof(uint32_t) * NC, st.hi));
+        if (!full) B_CUDA(cudaStreamWaitEvent(st.hi, rec[seg & 1], 0));
         for (int g0 = 0; g0 < NC; g0 += per_launch) {
             const int grid = std::min(per_launch, NC - g0) * CL;
-            rc = smooth ? launch_coop(bwd_kernel<true>, grid, threads, S.total, st.hi, ba, d->out_cta_max, t0, t1,
+            rc = smooth ? launch_coop(bwd_kernel<true, false>, grid, threads, S.total, st.hi, ba, d->out_cta_max, t0,
+                                      t1, first, g0)
+                 : full ? launch_coop(bwd_kernel<false, true>, grid, threads, S.total, st.hi, ba, d->out_cta_max, t0, t1,
                                       first, g0)
-                        : launch_coop(bwd_kernel<false>, grid, threads, S.total, st.hi, ba, d->out_cta_max, t0, t1,
-                                      first, g0);
+                        : launch_coop(bwd_kernel<false, false>, grid, threads, S.total, st.hi, ba, d->out_cta_max, t0,
+                                      t1, first, g0);
             if (rc) return rc;
         }
         B_CUDA(cudaEventRecord(adj[seg & 1], st.hi));
@@ -1194,6 +1686,7 @@ int n2b_bptt_backward(const n2b_bptt_desc *d, const float *u, const float *w_rec
         B_CUDA(cudaGetLastError());
     }
     const int n = d->hidden * d->readouts;
+    if (full) B_CUDA(cudaStreamWaitEvent(st.hi, rec[1], 0));
     reduce_dwo_kernel<<<(n + 255) / 256, 256, 0, st.hi>>>(a.dwo_p, n, NC, dw_out);
     B_CUDA(cudaGetLastError());
     B_CUDA(cudaEventRecord(join, st.hi));

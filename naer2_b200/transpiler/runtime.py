@@ -105,10 +105,11 @@ def arrival_bytes(n_tgt: int, n_links: int, depth: int) -> int:
 
 def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -> dict:
     """The arrival bits of one connection, from its pull CSR: `wptr` int32 [n_tgt + 1], each row's first word in a
-    slot; `words` per slot; `depth`, the slots (the largest delay + 1: a slot is read
-    and cleared in the step before the first that can set it again); the outgoing rows `out_ptr`
-    int32 [n_src + 1], `pos` int32 (uint32 bits: the link's bit in a slot) and `dly` uint8, links of a source in
-    pull order -- with at most 2^24 bits to a slot the delay is in the top 8 bits of `pos` and `dly` is None; `bad`: links whose source or delay (1 .. mask) is out of range, in no outgoing row."""
+    slot; `words` per slot; `depth`, the slots (the largest delay + 1: a slot is read and cleared in the step before
+    the first that can set it again); the outgoing rows `out_ptr` int32 [n_src + 1], `pos` int32 (uint32 bits: the
+    link's bit in a slot) and `dly` uint8, links of a source in pull order -- with at most 2^24 bits to a slot the
+    delay is in the top 8 bits of `pos` and `dly` is None; `bad`: links whose source or delay (1 .. mask) is out of
+    range, in no outgoing row."""
     dev = link.device
     n_tgt = len(ptr) - 1
     ptr = ptr.to(torch.int64)

@@ -1045,7 +1045,8 @@ __device__ __forceinline__ void deliver_spikes(const StepArgs &a, const PopDev &
         // EARLY: the far items are listed while the first near links are in flight (the claim's answer comes about
         // when they do): with the groups' shifts and rec0 read once, 5.17 to 4.6-4.7 us a step at 12,500 neurons, 5.95
         // to 5.4 at 38,585. In the kernel with the pull path, at its limit of 128 registers, they are listed after
-        // (listed early there, the dense-input network steps in 16.2 us instead of 15.6).
+        // (listed early there, the dense-input network steps in 16.2 us instead of 15.6); so are the spikes of a
+        // block's later tiles (549,872 neurons in 2,148 tiles: 86.6 us a step early, 84.9 after).
         auto list_items = [&]() {
             base = __shfl_sync(FULL, base, 0);
             if (lane < m && items_c > 0) {
@@ -1245,7 +1246,8 @@ __device__ __forceinline__ void tile_phase(const StepArgs &a, const long long n,
     }
 
     // 4. the spikes' outgoing rows
-    if (n_out > 0) deliver_spikes<NPB, INL, !PULL>(a, P, tile.y, CACHED ? s_cache : nullptr, cnt, n, sc, s_conn, k);
+    if (n_out > 0)
+        deliver_spikes<NPB, INL, !PULL && CACHED>(a, P, tile.y, CACHED ? s_cache : nullptr, cnt, n, sc, s_conn, k);
     for (int c = MERGE_OUT; c < n_out; ++c) {
         const ConnDev &C = push_at<INL>(a, P.out_first + c);
         const Row r = fire ? row_of(C, j) : Row{0, 0, 0};

@@ -251,9 +251,20 @@ int n2b_bptt_workspace_bytes(const n2b_bptt_desc *d, size_t *bytes);
 /* Forward over all steps: u [T][B][H] input current, w_rec [nnz] (incoming
  * order), w_out [H][R]; writes m [B][R] (max over time of the readouts) and
  * tstar [B][R] (its first step). tape = 1 keeps what the backward needs in
- * the workspace; 0 is the plain forward. */
+ * the workspace; 0 is the plain forward, which writes the error words alone
+ * there (n2b_bptt_infer is faster). */
 int n2b_bptt_forward(const n2b_bptt_desc *d, const float *u, const float *w_rec, const float *w_out, int32_t tape,
                      float *m, int32_t *tstar, void *workspace, size_t workspace_bytes, void *stream);
+
+/* Scratch bytes of n2b_bptt_infer (0: it needs none). */
+int n2b_bptt_infer_bytes(const n2b_bptt_desc *d, size_t *bytes);
+
+/* The plain forward over scratch of the call's own (device, 256-byte aligned):
+ * m and tstar as n2b_bptt_forward writes them, bit for bit, the error words in
+ * err [N2B_BPTT_ERR_WORDS] (device). It touches no workspace. Calls that may
+ * overlap on the device each need their own scratch and err. */
+int n2b_bptt_infer(const n2b_bptt_desc *d, const float *u, const float *w_rec, const float *w_out, float *m,
+                   int32_t *tstar, int32_t *err, void *scratch, size_t scratch_bytes, void *stream);
 
 /* Backward of the last taped forward: dm [B][R] = dL/dm, tstar as the forward
  * wrote it; writes du [T][B][H] = dL/du, dw_rec [nnz], dw_out [H][R]. The work

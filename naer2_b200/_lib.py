@@ -79,6 +79,8 @@ SIGNATURES = {
     "n2b_bptt_workspace_bytes": (ctypes.c_int, [ctypes.POINTER(BpttDesc), ctypes.POINTER(ctypes.c_size_t)]),
     "n2b_bptt_forward": (ctypes.c_int, [ctypes.POINTER(BpttDesc), _P, _P, _P, ctypes.c_int32, _P, _P, _P,
                                         ctypes.c_size_t, _P]),
+    "n2b_bptt_infer_bytes": (ctypes.c_int, [ctypes.POINTER(BpttDesc), ctypes.POINTER(ctypes.c_size_t)]),
+    "n2b_bptt_infer": (ctypes.c_int, [ctypes.POINTER(BpttDesc), _P, _P, _P, _P, _P, _P, _P, ctypes.c_size_t, _P]),
     "n2b_bptt_backward": (ctypes.c_int, [ctypes.POINTER(BpttDesc), _P, _P, _P, _P, _P, _P, _P, _P, _P,
                                          ctypes.c_size_t, _P]),
     "n2b_bptt_status": (ctypes.c_int, [ctypes.POINTER(BpttDesc), _P, ctypes.c_size_t,

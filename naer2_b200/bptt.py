@@ -248,6 +248,7 @@ class RecurrentLIF(torch.nn.Module):
             (torch.randn(hidden, readouts, generator=gen) * s_out / math.sqrt(hidden)).to(dev))
         self._ws = None
         self._ws_key = None
+        self._plain = None  # the last call was a plain forward: its (batch, steps) and error words
         self.tape_id = 0
         # polls before a wait of the backward's per-step exchange gives up (0: the library's default, about a
         # second); tests set a few to make the wait give up without a hang
@@ -305,21 +306,33 @@ class RecurrentLIF(torch.nn.Module):
         if U.dtype != torch.float32 or not U.is_cuda:
             raise RuntimeError("the layer runs on a CUDA device with fp32 currents (no CPU fallback)")
         d = self.desc(B, T)
-        ws = self.workspace(d)
+        lib = _lib.load()
         m = torch.empty(B, self.readouts, dtype=torch.float32, device=U.device)
         ts = torch.empty(B, self.readouts, dtype=torch.int32, device=U.device)
         s = ctypes.c_void_p(torch.cuda.current_stream(U.device).cuda_stream)
-        _lib.check(_lib.load().n2b_bptt_forward(ctypes.byref(d), U.data_ptr(), self.w_rec.data_ptr(),
-                                                self.w_out.data_ptr(), int(tape), m.data_ptr(), ts.data_ptr(),
-                                                ws.data_ptr(), ws.numel(), s), "n2b_bptt_forward")
-        if tape:
-            self.tape_id += 1
+        if not tape:
+            # scratch of the call's own, on its stream: calls of several streams or threads, and a backward, may overlap
+            n = ctypes.c_size_t()
+            _lib.check(lib.n2b_bptt_infer_bytes(ctypes.byref(d), ctypes.byref(n)), "n2b_bptt_infer_bytes")
+            scratch = torch.empty(n.value, dtype=torch.uint8, device=U.device)
+            err = torch.empty(_lib.BPTT_ERR_WORDS, dtype=torch.int32, device=U.device)
+            _lib.check(lib.n2b_bptt_infer(ctypes.byref(d), U.data_ptr(), self.w_rec.data_ptr(), self.w_out.data_ptr(),
+                                          m.data_ptr(), ts.data_ptr(), err.data_ptr(), scratch.data_ptr(), n.value, s),
+                       "n2b_bptt_infer")
+            self._plain = ((B, T), err)
+            return m, ts
+        ws = self.workspace(d)
+        self._plain = None
+        _lib.check(lib.n2b_bptt_forward(ctypes.byref(d), U.data_ptr(), self.w_rec.data_ptr(), self.w_out.data_ptr(), 1,
+                                        m.data_ptr(), ts.data_ptr(), ws.data_ptr(), ws.numel(), s), "n2b_bptt_forward")
+        self.tape_id += 1
         return m, ts
 
     def run_backward(self, U, dm, ts):
         T, B, H = U.shape
         d = self.desc(B, T)
         ws = self.workspace(d)
+        self._plain = None
         du = torch.empty_like(U)
         dw_rec = torch.empty_like(self.w_rec)
         dw_out = torch.empty_like(self.w_out)
@@ -332,6 +345,9 @@ class RecurrentLIF(torch.nn.Module):
         return du, dw_rec, dw_out
 
     def status(self, batch: int, steps: int) -> list:
+        plain = self._plain
+        if plain is not None and plain[0] == (batch, steps):
+            return plain[1].tolist()
         d = self.desc(batch, steps)
         ws = self.workspace(d)
         words = (ctypes.c_int32 * _lib.BPTT_ERR_WORDS)()

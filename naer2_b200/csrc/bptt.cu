@@ -68,7 +68,6 @@ struct Args {
     float *s_f;         // [T][NC][H][8]   (smooth)
     float *v_ckpt;      // [nseg][B][H]
     float *g_seg;       // [K][B][H]: the segment's recurrent input, then its surrogate derivatives
-    uint8_t *s_plain;   // [T][NC][H]: the plain forward's spikes
     unsigned long long *xw;  // [NC][XSLOTS][H / 4]: the forward's published words
     float *tot;         // [T][B][R]: every step's readout sums
     float *g_all;       // [T][B][H]: every step's surrogate derivatives, or null (segments recomputed)
@@ -520,7 +519,6 @@ __global__ void __launch_bounds__(NB * 128) fwd_group_kernel(const __grid_consta
     }
     uint32_t *ring32 = reinterpret_cast<uint32_t *>(ring);
     unsigned long long *xw = a.xw + (size_t)q * XSLOTS * (H / 4);
-    uint8_t *bits_out = a.tape ? a.s_bits : a.s_plain;
     const float *u = a.U + ((size_t)q * NS + own) * H + post;
     const size_t ustep = (size_t)B * H;
     float V = 0.f, u0 = nt ? __ldcs(u) : 0.f, u1 = (nt && a.T > 1) ? __ldcs(u + ustep) : 0.f;
@@ -629,7 +627,7 @@ __global__ void __launch_bounds__(NB * 128) fwd_group_kernel(const __grid_consta
         const uint32_t word = __ballot_sync(FULL, sp != 0.f);
         if (lane == 0 && nt) {
             publish(xw + (size_t)(t % XSLOTS) * (H / 4) + (post >> 2), word, (uint32_t)t + 1u);
-            *reinterpret_cast<uint32_t *>(bits_out + ((size_t)t * a.NC + q) * H + post) = word;
+            *reinterpret_cast<uint32_t *>(a.s_bits + ((size_t)t * a.NC + q) * H + post) = word;
         }
         if (a.tape && a.g_all && nt)
             __stcs(a.g_all + ((size_t)t * B + (size_t)q * NS + own) * H + post, surrogate(__fadd_rn(vp, -a.theta), a.slope));
@@ -643,7 +641,7 @@ constexpr int READOUT_THREADS = 256;
 __global__ void __launch_bounds__(READOUT_THREADS) readout_kernel(const __grid_constant__ Args a) {
     __shared__ uint32_t bits[NS][32];
     const int t = blockIdx.x, q = blockIdx.y, lane = threadIdx.x & 31;
-    const uint8_t *src = (a.tape ? a.s_bits : a.s_plain) + ((size_t)t * a.NC + q) * a.H;
+    const uint8_t *src = a.s_bits + ((size_t)t * a.NC + q) * a.H;
     for (int g = threadIdx.x / 32; g < a.H / 32; g += READOUT_THREADS / 32) {
         const uint32_t byte = src[32 * g + lane];
 #pragma unroll
@@ -1314,7 +1312,7 @@ int bcuda(cudaError_t e, const char *what) {
 constexpr size_t FULL_TAPE_BYTES = (size_t)4 << 30;
 
 struct WsLayout {
-    size_t spikes, plain, xw, tot, vck, gseg, outw, dwp, dwo, part, qst, ost, qx, qflag, err, total;
+    size_t spikes, xw, tot, vck, gseg, outw, dwp, dwo, part, qst, ost, qx, qflag, err, total;
 };
 
 size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -1352,7 +1350,6 @@ WsLayout ws_layout(const n2b_bptt_desc *d) {
     const size_t nseg = (T + d->checkpoint - 1) / d->checkpoint, K = std::min<size_t>(d->checkpoint, T);
     size_t o = 0;
     L.spikes = o; o = a256(o + (d->smooth ? sizeof(float) * T * NC * H * NS : T * NC * H));
-    L.plain = o; o = a256(o + (scans(d) ? T * NC * H : 0));
     L.xw = o; o = a256(o + (scans(d) ? sizeof(unsigned long long) * NC * XSLOTS * (H / 4) : 0));
     L.tot = o; o = a256(o + (scans(d) ? sizeof(float) * T * B * R : 0));
     L.vck = o; o = a256(o + (full_tape(d) ? 0 : sizeof(float) * nseg * B * H));
@@ -1371,12 +1368,28 @@ WsLayout ws_layout(const n2b_bptt_desc *d) {
     return L;
 }
 
+// n2b_bptt_infer's scratch: what fwd_group_kernel and the readout's kernels hand on.
+struct PlainLayout {
+    size_t spikes, xw, tot, total;
+};
+PlainLayout plain_layout(const n2b_bptt_desc *d) {
+    PlainLayout L{};
+    if (!scans(d)) return L;  // fwd_kernel keeps nothing in memory
+    const size_t T = d->steps, B = d->batch, H = d->hidden, NC = B / NS;
+    size_t o = 0;
+    L.spikes = o; o = a256(o + T * NC * H);
+    L.xw = o; o = a256(o + sizeof(unsigned long long) * NC * XSLOTS * (H / 4));
+    L.tot = o; o = a256(o + sizeof(float) * T * B * d->readouts);
+    L.total = o;
+    return L;
+}
+
 int threads_of(const n2b_bptt_desc *d, int per_neuron) {
     const int n = std::max(per_neuron * (d->hidden / CL), NS * d->readouts);
     return (n + 31) / 32 * 32;
 }
 
-Args args_of(const n2b_bptt_desc *d, char *ws, const WsLayout &L) {
+Args sizes_of(const n2b_bptt_desc *d) {
     Args a{};
     a.B = d->batch;
     a.T = d->steps;
@@ -1395,9 +1408,14 @@ Args args_of(const n2b_bptt_desc *d, char *ws, const WsLayout &L) {
     a.in_code = d->in_code;
     a.out_grp = d->out_grp;
     a.out_code = d->out_code;
+    a.wait_polls = d->wait_polls > 0 ? d->wait_polls : XCHG_SPIN_LIMIT;
+    return a;
+}
+
+Args args_of(const n2b_bptt_desc *d, char *ws, const WsLayout &L) {
+    Args a = sizes_of(d);
     a.s_bits = reinterpret_cast<uint8_t *>(ws + L.spikes);
     a.s_f = reinterpret_cast<float *>(ws + L.spikes);
-    a.s_plain = reinterpret_cast<uint8_t *>(ws + L.plain);
     a.xw = reinterpret_cast<unsigned long long *>(ws + L.xw);
     a.tot = reinterpret_cast<float *>(ws + L.tot);
     a.v_ckpt = reinterpret_cast<float *>(ws + L.vck);
@@ -1413,7 +1431,6 @@ Args args_of(const n2b_bptt_desc *d, char *ws, const WsLayout &L) {
     a.qflag = reinterpret_cast<uint32_t *>(ws + L.qflag);
     a.o_all = a.tot;
     a.err = reinterpret_cast<int32_t *>(ws + L.err);
-    a.wait_polls = d->wait_polls > 0 ? d->wait_polls : XCHG_SPIN_LIMIT;
     return a;
 }
 
@@ -1512,6 +1529,37 @@ int launch_coop(Kern kern, int grid, int threads, size_t smem, cudaStream_t s, c
     return N2B_OK;
 }
 
+// The forward's launches. `group`: fwd_group_kernel and the readout's kernels, over a's spikes, words and readout sums;
+// else fwd_kernel, which without a tape writes m, tstar and the error words alone.
+int run_forward(const n2b_bptt_desc *d, Args a, bool group, cudaStream_t s) {
+    B_CUDA(cudaMemsetAsync(a.err, 0, sizeof(int32_t) * N2B_BPTT_ERR_WORDS, s));
+    if (group) {
+        const int NC = d->batch / NS, gthreads = (NB * (d->hidden / CL) + 31) / 32 * 32;
+        const size_t smem = scan_smem(d->hidden, d->hidden / CL, d->in_cta_max).total;
+        int per_launch = 0;  // groups per cooperative launch
+        int rc = coop_groups(fwd_group_kernel, gthreads, smem, per_launch);
+        if (rc) return rc;
+        B_CUDA(cudaMemsetAsync(a.xw, 0, sizeof(unsigned long long) * NC * XSLOTS * (d->hidden / 4), s));
+        for (int g0 = 0; g0 < NC; g0 += per_launch) {
+            rc = launch_coop(fwd_group_kernel, std::min(per_launch, NC - g0) * CL, gthreads, smem, s, a, d->in_cta_max,
+                             g0);
+            if (rc) return rc;
+        }
+        readout_kernel<<<dim3((unsigned)d->steps, (unsigned)NC), READOUT_THREADS, 0, s>>>(a);
+        B_CUDA(cudaGetLastError());
+        readout_max_kernel<<<(unsigned)((d->batch * d->readouts + 31) / 32), 32, 0, s>>>(a);
+        B_CUDA(cudaGetLastError());
+        return N2B_OK;
+    }
+    const bool smooth = d->smooth != 0;
+    const int grid = (d->batch / NS) * CL, threads = threads_of(d, NT);
+    FwdSmem S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, true, d->in_cta_max);
+    a.csr_smem = S.total <= 200 * 1024;
+    if (!a.csr_smem) S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, false, 0);
+    return smooth ? launch_cluster(fwd_kernel<true>, grid, threads, S.total, s, a, d->in_cta_max)
+                  : launch_cluster(fwd_kernel<false>, grid, threads, S.total, s, a, d->in_cta_max);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1530,41 +1578,48 @@ int n2b_bptt_forward(const n2b_bptt_desc *d, const float *u, const float *w_rec,
     int rc = check_ws(d, workspace, workspace_bytes, L);
     if (rc) return rc;
     if (!u || !w_out || !m || !tstar || (d->nnz > 0 && !w_rec)) return bfail(N2B_EINVAL, "missing arguments");
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    char *ws = static_cast<char *>(workspace);
-    Args a = args_of(d, ws, L);
+    Args a = args_of(d, static_cast<char *>(workspace), L);
     a.tape = tape != 0;
     a.U = u;
     a.in_w = w_rec;
     a.w_out = w_out;
     a.m = m;
     a.tstar = tstar;
-    B_CUDA(cudaMemsetAsync(ws + L.err, 0, sizeof(int32_t) * N2B_BPTT_ERR_WORDS, s));
-    const bool smooth = d->smooth != 0;
-    const int grid = (d->batch / NS) * CL, threads = threads_of(d, NT);
-    if (scans(d)) {
-        const int NC = d->batch / NS, gthreads = (NB * (d->hidden / CL) + 31) / 32 * 32;
-        const size_t smem = scan_smem(d->hidden, d->hidden / CL, d->in_cta_max).total;
-        int per_launch = 0;  // groups per cooperative launch
-        rc = coop_groups(fwd_group_kernel, gthreads, smem, per_launch);
-        if (rc) return rc;
-        B_CUDA(cudaMemsetAsync(a.xw, 0, sizeof(unsigned long long) * NC * XSLOTS * (d->hidden / 4), s));
-        for (int g0 = 0; g0 < NC; g0 += per_launch) {
-            rc = launch_coop(fwd_group_kernel, std::min(per_launch, NC - g0) * CL, gthreads, smem, s, a, d->in_cta_max,
-                             g0);
-            if (rc) return rc;
-        }
-        readout_kernel<<<dim3((unsigned)d->steps, (unsigned)NC), READOUT_THREADS, 0, s>>>(a);
-        B_CUDA(cudaGetLastError());
-        readout_max_kernel<<<(unsigned)((d->batch * d->readouts + 31) / 32), 32, 0, s>>>(a);
-        B_CUDA(cudaGetLastError());
-        return N2B_OK;
+    // without a tape nothing of the workspace but the error words is written (calls and a backward may overlap)
+    return run_forward(d, a, tape && scans(d), reinterpret_cast<cudaStream_t>(stream));
+}
+
+int n2b_bptt_infer_bytes(const n2b_bptt_desc *d, size_t *bytes) {
+    if (!bytes) return bfail(N2B_EINVAL, "bytes is NULL");
+    int rc = check_desc(d);
+    if (rc) return rc;
+    *bytes = plain_layout(d).total;
+    return N2B_OK;
+}
+
+int n2b_bptt_infer(const n2b_bptt_desc *d, const float *u, const float *w_rec, const float *w_out, float *m,
+                   int32_t *tstar, int32_t *err, void *scratch, size_t scratch_bytes, void *stream) {
+    int rc = check_desc(d);
+    if (rc) return rc;
+    if (!u || !w_out || !m || !tstar || !err || (d->nnz > 0 && !w_rec)) return bfail(N2B_EINVAL, "missing arguments");
+    const PlainLayout L = plain_layout(d);
+    if (L.total > 0 && (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 255)))
+        return bfail(N2B_EINVAL, "scratch must be 256-byte aligned");
+    if (scratch_bytes < L.total) return bfail(N2B_ESPACE, "scratch too small: need " + std::to_string(L.total) + " bytes");
+    char *at = static_cast<char *>(scratch);
+    Args a = sizes_of(d);
+    a.U = u;
+    a.in_w = w_rec;
+    a.w_out = w_out;
+    a.m = m;
+    a.tstar = tstar;
+    a.err = err;
+    if (L.total > 0) {
+        a.s_bits = reinterpret_cast<uint8_t *>(at + L.spikes);
+        a.xw = reinterpret_cast<unsigned long long *>(at + L.xw);
+        a.tot = reinterpret_cast<float *>(at + L.tot);
     }
-    FwdSmem S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, true, d->in_cta_max);
-    a.csr_smem = S.total <= 200 * 1024;
-    if (!a.csr_smem) S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, false, 0);
-    return smooth ? launch_cluster(fwd_kernel<true>, grid, threads, S.total, s, a, d->in_cta_max)
-                  : launch_cluster(fwd_kernel<false>, grid, threads, S.total, s, a, d->in_cta_max);
+    return run_forward(d, a, scans(d), reinterpret_cast<cudaStream_t>(stream));
 }
 
 int n2b_bptt_backward(const n2b_bptt_desc *d, const float *u, const float *w_rec, const float *w_out,

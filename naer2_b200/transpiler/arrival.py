@@ -509,6 +509,9 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
         src += [_exact_collect(c, inc) for c, inc in enumerate(incoming) if takes(inc)]
         if any(takes(inc) for inc in incoming):
             src += [_exact_times(incoming), _EXACT_SORT, _exact_deliver(pop_name, incoming, hooks)]
+        else:  # the send of a time group has call sites of its own: without groups the step's send keeps its numbers
+            fn, ctx = hooks["send"]
+            lower_hook(fn, ctx, f"{pop_name} send")
     else:
         for c, inc in enumerate(incoming):
             if takes(inc):

@@ -1141,6 +1141,7 @@ __global__ void __launch_bounds__(256) readout_dV_kernel(const __grid_constant__
     }
     __syncthreads();
     if (i >= pairs) return;
+    const bool wide = (reinterpret_cast<uintptr_t>(a.dU) & 7) == 0;  // the caller's buffer (H is even: so every row)
     for (int k = 0; k < rows; ++k) {
         float s0 = 0.f, s1 = 0.f;
 #pragma unroll
@@ -1155,7 +1156,13 @@ __global__ void __launch_bounds__(256) readout_dV_kernel(const __grid_constant__
             s0 = __fmaf_rn(w[0][4 * r + 3], v.w, s0);
             s1 = __fmaf_rn(w[1][4 * r + 3], v.w, s1);
         }
-        __stcs(reinterpret_cast<float2 *>(a.dU + (size_t)(r0 + k) * a.H) + i, make_float2(s0, s1));
+        float *at = a.dU + (size_t)(r0 + k) * a.H + 2 * i;
+        if (wide) {
+            __stcs(reinterpret_cast<float2 *>(at), make_float2(s0, s1));
+        } else {
+            __stcs(at, s0);
+            __stcs(at + 1, s1);
+        }
     }
 }
 

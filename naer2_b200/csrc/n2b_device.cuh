@@ -1491,6 +1491,13 @@ __device__ __forceinline__ bool grid_sync(const StepArgs &a, unsigned k) {
     return grid_wait(a, k);
 }
 
+// Whether an earlier window gave up (nothing runs then). One thread reads the word for the block: a block of this launch
+// may set it meanwhile, and a block of which some threads saw it and others not would wait and read what its first
+// thread never wrote.
+__device__ __forceinline__ bool stopped(const StepArgs &a) {
+    return __syncthreads_or(threadIdx.x == 0 && *(volatile unsigned *)(a.barrier + BAR_ABORT));
+}
+
 // The end of a chunked window, on every way out of it: the last block to get here advances the step counter and
 // clears the barrier for the next launch (every block has read the one and waits on the other no more).
 __device__ __forceinline__ void finish_window(const StepArgs &a, int n_steps) {
@@ -1509,7 +1516,7 @@ enum { WITH_PULL, PLAIN, DENSE };
 template <int NPB, bool INL, int KIND>
 __global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
     persistent_kernel(const __grid_constant__ StepArgs a, const int n_steps) {
-    if (*(volatile unsigned *)(a.barrier + BAR_ABORT)) return;  // an earlier window gave up: nothing runs
+    if (stopped(a)) return;
     const long long n0 = *a.step;
     __shared__ Scratch<NPB> sc;
     if (threadIdx.x == 0) sc.rec0 = *a.rec0;  // (read at each step it would miss the L1, in the step's chain)
@@ -1644,7 +1651,7 @@ __device__ __forceinline__ void chunk_deliver(const StepArgs &a, const PopDev &P
 template <int TN>
 __global__ void __launch_bounds__(CHUNK_THREADS, 2)
     chunk_kernel(const __grid_constant__ StepArgs a, const int n_steps, const int chunk, const int n_tiles) {
-    if (*(volatile unsigned *)(a.barrier + BAR_ABORT)) {  // an earlier window gave up: nothing runs
+    if (stopped(a)) {
         finish_window(a, n_steps);
         return;
     }

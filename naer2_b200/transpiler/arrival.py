@@ -603,7 +603,8 @@ def window_source(exact: bool, bodies: list, sizes: list, edges: int, per_sm: in
 
 extern "C" __global__ void __launch_bounds__({THREADS}, {per_sm}) n2b_user_window(const __grid_constant__ Window w) {{
     __shared__ N2Scratch s;
-    if (*(volatile u32 *)(w.grid.bar + 32)) return;  // an earlier window gave up: nothing runs
+    // an earlier window gave up: nothing runs (one thread reads for the block: another block may set it meanwhile)
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile u32 *)(w.grid.bar + 32))) return;
     const int b = (int)blockIdx.x;
 """)
     first = 0

@@ -93,11 +93,11 @@ __device__ __forceinline__ void n2_deliver(const N2Out &o, long long n, int r0, 
         }
 }
 
-// The grid barrier of a window: `bar[0]` counts arrivals, `bar[32]` is set when a wait gave up (bar[33]: how many).
+// The grid barrier of a window: `bar[0]` counts arrivals (from 0 in every launch: n2_finish), `bar[32]` is set when a
+// wait gave up (bar[33]: how many), `bar[48]` counts the blocks that are done with the launch.
 struct N2Grid {
     u32 *bar;
     u64 limit_ns;
-    u32 base, pad;  // the count before this window
 };
 
 __device__ __forceinline__ u64 n2_clock() {
@@ -110,7 +110,7 @@ __device__ __forceinline__ bool n2_grid_sync(const N2Grid &g, int k) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const u32 target = g.base + (u32)(k + 1) * gridDim.x;
+        const u32 target = (u32)(k + 1) * gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.bar) : "memory");
         int ok = 1;
         u64 t0 = 0;
@@ -133,6 +133,15 @@ __device__ __forceinline__ bool n2_grid_sync(const N2Grid &g, int k) {
     __syncthreads();
     return s_ok != 0;
 }
+
+// Every block's way out of a window: the last one clears the barrier (none waits at it any more) for the next launch,
+// which may be this one's replay.
+__device__ __forceinline__ void n2_finish(const N2Grid &g) {
+    if (threadIdx.x == 0 && atomicAdd(g.bar + 48, 1u) == gridDim.x - 1) {
+        g.bar[0] = 0u;
+        g.bar[48] = 0u;
+    }
+}
 '''
 
 _LISTS = {False: "    u32 words[NPB_C][CHUNK];",
@@ -149,8 +158,7 @@ class Out(ctypes.Structure):
 
 class Grid(ctypes.Structure):
     """A window's grid barrier (N2Grid)."""
-    _fields_ = [("bar", ctypes.c_void_p), ("limit_ns", ctypes.c_uint64), ("base", ctypes.c_uint32),
-                ("pad", ctypes.c_uint32)]
+    _fields_ = [("bar", ctypes.c_void_p), ("limit_ns", ctypes.c_uint64)]
 
 
 def common(exact: bool, edges: int) -> str:
@@ -604,7 +612,10 @@ def window_source(exact: bool, bodies: list, sizes: list, edges: int, per_sm: in
 extern "C" __global__ void __launch_bounds__({THREADS}, {per_sm}) n2b_user_window(const __grid_constant__ Window w) {{
     __shared__ N2Scratch s;
     // an earlier window gave up: nothing runs (one thread reads for the block: another block may set it meanwhile)
-    if (__syncthreads_or(threadIdx.x == 0 && *(volatile u32 *)(w.grid.bar + 32))) return;
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile u32 *)(w.grid.bar + 32))) {{
+        n2_finish(w.grid);
+        return;
+    }}
     const int b = (int)blockIdx.x;
 """)
     first = 0
@@ -613,7 +624,7 @@ extern "C" __global__ void __launch_bounds__({THREADS}, {per_sm}) n2b_user_windo
             src.append(f"    if (b >= {first} && b < {first + blocks_of(n)}) n2p{k}::n2_steps<true>(w.p{k}, s, b - {first}, "
                        "w.step0, (int)w.n_steps, w.dt, w.grid);\n")
         first += blocks_of(n)
-    src.append("}\n")
+    src.append("    n2_finish(w.grid);\n}\n")
     return "".join(src)
 
 

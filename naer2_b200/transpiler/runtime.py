@@ -241,7 +241,7 @@ def save_plan(plan: dict, path) -> None:
 
     arrays, meta = {}, {"dt": plan["dt"], "exact": plan["exact"], "pops": []}
     if "window" in plan:
-        meta["window"] = plan["window"]
+        meta["window_source"] = plan["window"]
     for k, p in enumerate(plan["pops"]):
         m = {key: p[key] for key in ("name", "n", "words", "depth", "seed", "source", "fields", "attrs", "outs")
              if key in p}
@@ -263,8 +263,8 @@ def load_plan(path) -> dict:
     z = np.load(path)
     meta = json.loads(bytes(z["plan_json"]).decode())
     plan = {"dt": meta["dt"], "exact": meta["exact"], "pops": []}
-    if "window" in meta:
-        plan["window"] = meta["window"]
+    if "window_source" in meta:  # (a plan whose window kernel counts on its caller, "window", steps without it)
+        plan["window"] = meta["window_source"]
     for k, m in enumerate(meta["pops"]):
         p = dict(m)
         p["fields"] = [tuple(f) for f in m["fields"]]
@@ -382,8 +382,7 @@ class JitRuntime:
                                         arr=f["arr"].data_ptr(), words=f["words"], depth=f["depth"])
         self.window = self.window_kernel = None  # the window kernel and its parameter block
         self.window_grid = sum(arrival.blocks_of(p["n"]) for p in plan["pops"])
-        self.bar = torch.zeros(64, dtype=torch.int32, device=dev)  # its grid barrier: arrivals, abort word, stops
-        self.bar_base = 0  # arrivals of the windows so far
+        self.bar = torch.zeros(64, dtype=torch.int32, device=dev)  # its grid barrier (N2Grid)
         if "window" in plan:
             self._window(plan["window"], dindex)
         if self.window is None:
@@ -432,14 +431,12 @@ class JitRuntime:
     def _advance_window(self, step: int, n_steps: int) -> None:
         lib, W = _lib.load(), self.window
         W.step0, W.n_steps = step, n_steps
-        W.grid.base = self.bar_base
         W.grid.limit_ns = int(getattr(self.net, "barrier_limit_ns", 0) or BARRIER_LIMIT_NS)
         for k, P in enumerate(self.params):
             setattr(W, f"p{k}", P)
         _lib.check(lib.n2b_jit_launch_cooperative(self.window_kernel, self.window_grid, arrival.THREADS,
                                                   ctypes.addressof(W), ctypes.sizeof(W), self._s),
                    "n2b_jit_launch_cooperative")
-        self.bar_base = (self.bar_base + (n_steps - 1) * self.window_grid) & 0xFFFFFFFF
         self.launches += 1
 
     def _advance_steps(self, step: int, n_steps: int) -> None:
@@ -538,7 +535,6 @@ class JitRuntime:
         self.counters_t.zero_()
         self.err.zero_()
         self.bar.zero_()
-        self.bar_base = 0
 
     def close(self) -> None:
         self.stream.synchronize()

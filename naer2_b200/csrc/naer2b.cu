@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -170,6 +171,7 @@ struct n2b_net {
     // steps without a grid barrier between them (chunk_kernel; 0: a barrier per step), its neurons per tile and tiles
     int32_t chunk = 0, chunk_tn = 0, chunk_tiles = 0;
     cudaEvent_t before = nullptr, after = nullptr;  // n2b_advance: the caller's stream and the net's, in order
+    std::mutex advancing;                           // ... of one call at a time: the events and the captured window
 };
 
 namespace {
@@ -651,6 +653,7 @@ int n2b_advance(n2b_net *net, int64_t n_steps, int32_t window_steps, void *strea
     DeviceGuard guard;
     if (!net) return fail(N2B_EINVAL, "net is NULL");
     if (n_steps < 0 || window_steps <= 0) return fail(N2B_EINVAL, "n_steps < 0 or window_steps <= 0");
+    std::lock_guard<std::mutex> lock(net->advancing);
     N2B_CUDA(cudaSetDevice(net->device));
     if (!net->before) N2B_CUDA(cudaEventCreateWithFlags(&net->before, cudaEventDisableTiming));
     if (!net->after) N2B_CUDA(cudaEventCreateWithFlags(&net->after, cudaEventDisableTiming));

@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(NB * 128) fwd_group_kernel(const __grid_consta
 constexpr int READOUT_THREADS = 256;
 __global__ void __launch_bounds__(READOUT_THREADS) readout_kernel(const __grid_constant__ Args a) {
     __shared__ uint32_t bits[NS][32];
-    const int t = blockIdx.x, q = blockIdx.y, lane = threadIdx.x & 31;
+    const int t = blockIdx.x / a.NC, q = blockIdx.x % a.NC, lane = threadIdx.x & 31;
     const uint8_t *src = a.s_bits + ((size_t)t * a.NC + q) * a.H;
     for (int g = threadIdx.x / 32; g < a.H / 32; g += READOUT_THREADS / 32) {
         const uint32_t byte = src[32 * g + lane];
@@ -1552,7 +1552,7 @@ int run_forward(const n2b_bptt_desc *d, Args a, bool group, cudaStream_t s) {
                              g0);
             if (rc) return rc;
         }
-        readout_kernel<<<dim3((unsigned)d->steps, (unsigned)NC), READOUT_THREADS, 0, s>>>(a);
+        readout_kernel<<<(unsigned)(d->steps * NC), READOUT_THREADS, 0, s>>>(a);  // (below 2^26: check_desc)
         B_CUDA(cudaGetLastError());
         readout_max_kernel<<<(unsigned)((d->batch * d->readouts + 31) / 32), 32, 0, s>>>(a);
         B_CUDA(cudaGetLastError());

@@ -71,3 +71,15 @@ def test_a_forward_without_a_tape_leaves_the_workspace(cuda):
                                             ws.numel(), s), "n2b_bptt_forward")
     assert torch.equal(m, m2) and torch.equal(ts, ts2)
     assert int((ws != 0x5A).sum()) == 4 * _lib.BPTT_ERR_WORDS
+
+
+def test_a_batch_of_more_groups_than_a_grid_has_rows(cuda):
+    """65,544 groups of 8 samples: the last samples are those of a small batch, bit for bit."""
+    B, T, H = 8 * 65544, 2, 32
+    layer = RecurrentLIF(n_in=4, hidden=H, readouts=1, density=0.5, checkpoint=7, seed=H, device=cuda)
+    g = torch.Generator(device=cuda).manual_seed(1)
+    U = 0.6 + 0.5 * torch.randn(T, B, H, generator=g, device=cuda)
+    m, ts = layer.run_forward(U, tape=False)
+    want, want_ts = layer.run_forward(U[:, -16:].contiguous(), tape=False)
+    assert torch.equal(m[-16:], want) and torch.equal(ts[-16:], want_ts)
+    assert int((m != 0).sum()) > B // 4

@@ -239,8 +239,8 @@ typedef struct n2b_bptt_desc {
     const int32_t *out_grp;   /* [H][6] outgoing rows: start of the delay-1..5 links, then the row end */
     const uint16_t *out_code; /* [nnz] target | delay << 11, outgoing order */
     const int32_t *out_perm;  /* [nnz] incoming-order index of each outgoing link */
-    int32_t wait_polls;       /* polls before a backward exchange wait gives up with error word 3 (0: about a
-                                 second); tests set a few, so that the wait gives up without a hang */
+    int32_t wait_polls;       /* polls before a wait of the per-step exchange (the spiking forward's or the
+                                 backward's) gives up with error word 3 (0: about a second); tests set a few, so that the wait gives up without a hang */
     int32_t reserved;
 } n2b_bptt_desc;
 

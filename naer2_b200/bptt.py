@@ -250,7 +250,7 @@ class RecurrentLIF(torch.nn.Module):
         self._ws_key = None
         self._plain = None  # the last call was a plain forward: its (batch, steps) and error words
         self.tape_id = 0
-        # polls before a wait of the backward's per-step exchange gives up (0: the library's default, about a
+        # polls before a wait of the per-step exchange (forward or backward) gives up (0: the library's default, about a
         # second); tests set a few to make the wait give up without a hang
         self.wait_polls = 0
 

@@ -86,7 +86,7 @@ struct Args {
     uint32_t *qflag;    // [NC][2][H / 4] its flags, one per warp (cleared before a call's first launch)
     float *o_all;       // [T][B][R]: every step's readout adjoint (all steps in one launch)
     int32_t *err;       // [N2B_BPTT_ERR_WORDS]
-    int wait_polls;     // polls before a wait of the adjoint's exchange gives up
+    int wait_polls;     // polls before a wait of the per-step exchange gives up
 };
 
 __device__ __forceinline__ float surrogate(float x, float slope) {
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(NB * 128) fwd_group_kernel(const __grid_consta
             if (tid < H / 4) {
                 uint32_t word = 0u;
                 if (!*(volatile int *)&aborted &&
-                    !await(xw + (size_t)((t - 1) % XSLOTS) * (H / 4) + tid, (uint32_t)t, XCHG_SPIN_LIMIT, word)) {
+                    !await(xw + (size_t)((t - 1) % XSLOTS) * (H / 4) + tid, (uint32_t)t, a.wait_polls, word)) {
                     atomicAdd(a.err + 3, 1);
                     *(volatile int *)&aborted = 1;
                 }

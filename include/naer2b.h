@@ -212,10 +212,10 @@ int n2b_destroy(n2b_net *net);
  * The backward uses g = 1 / (1 + slope |Vpre - theta|)^2 for ds/dVpre (the
  * fast-sigmoid surrogate; the exact derivative of the smooth f), the reset
  * included. The forward keeps the spikes of every step (one bit per neuron,
- * sample and step), the membrane every `checkpoint` steps and, where that
- * takes 4 GiB at most, g of every step; the backward runs it backwards (else
- * it recomputes each segment's g from its checkpoint first) over
- * the transposed (outgoing) rows. */
+ * sample and step) and g of every step, where that takes 4 GiB at most and
+ * `segments` is 0, else the membrane every `checkpoint` steps, from which the
+ * backward recomputes each segment's g; the backward runs over the transposed
+ * (outgoing) rows. */
 
 /* error words: 0 links with a bad code (skipped); 1 recomputed spikes that
  * differ from the forward's; 2 in_cta_max / out_cta_max below the rows' counts;
@@ -241,7 +241,8 @@ typedef struct n2b_bptt_desc {
     const int32_t *out_perm;  /* [nnz] incoming-order index of each outgoing link */
     int32_t wait_polls;       /* polls before a wait of the per-step exchange (the spiking forward's or the
                                  backward's) gives up with error word 3 (0: about a second); tests set a few, so that the wait gives up without a hang */
-    int32_t reserved;
+    int32_t segments;         /* 1: keep the membrane every `checkpoint` steps instead of g of every step, whatever
+                                 it takes (a smaller workspace; the same value in every call over one) */
 } n2b_bptt_desc;
 
 /* Device workspace bytes of the layer (spike tape, checkpoints, the surrogate

@@ -52,7 +52,7 @@ class BpttDesc(ctypes.Structure):
         ("alpha", ctypes.c_float), ("beta", ctypes.c_float), ("theta", ctypes.c_float), ("slope", ctypes.c_float),
         ("in_ptr", ctypes.c_void_p), ("in_code", ctypes.c_void_p), ("out_grp", ctypes.c_void_p),
         ("out_code", ctypes.c_void_p), ("out_perm", ctypes.c_void_p), ("wait_polls", ctypes.c_int32),
-        ("reserved", ctypes.c_int32),
+        ("segments", ctypes.c_int32),
     ]
 
 

@@ -6,9 +6,9 @@ sparse delayed recurrence (w_rec, delays 1..5 steps) -> R leaky non-spiking read
 over time of each readout, m [B, R], for a cross-entropy loss.
 The recurrence and its adjoint run in `n2b_bptt_forward` / `n2b_bptt_backward` (naer2_b200/csrc/bptt.cu)
 behind `torch.autograd.Function`: the forward keeps the spikes of every step (one bit per neuron, sample and
-step), the membrane every `checkpoint` steps and, where that takes 4 GiB at most, the surrogate's derivative of
-every step; the backward runs it backwards over the transposed (outgoing) rows, else it recomputes each segment
-from its checkpoint first. The model equations are stated in include/naer2b.h.
+step) and the surrogate's derivative of every step, where that takes 4 GiB and half of the free memory at most, else
+the membrane every `checkpoint` steps, from which the backward recomputes each segment; the backward runs over the
+transposed (outgoing) rows. The model equations are stated in include/naer2b.h.
 
 naer2 itself has no differentiable path; this layer follows the BPTT workload's description (700 input
 channels, 1024 hidden neurons at 10% recurrent density, delays of 1-5 steps, 20 readouts, fast-sigmoid
@@ -248,6 +248,10 @@ class RecurrentLIF(torch.nn.Module):
             (torch.randn(hidden, readouts, generator=gen) * s_out / math.sqrt(hidden)).to(dev))
         self._ws = None
         self._ws_key = None
+        # the tape of a taped forward: the surrogate's derivative of every step (False), the membrane every `checkpoint`
+        # steps, recomputed segment by segment (True; slower, smaller), or (None) the first where memory allows
+        self.segments: bool | None = None
+        self._ws_segments = 0
         self._plain = None  # the last call was a plain forward: its (batch, steps) and error words
         self.tape_id = 0
         # polls before a wait of the per-step exchange (forward or backward) gives up (0: the library's default, about a
@@ -269,13 +273,32 @@ class RecurrentLIF(torch.nn.Module):
         return d
 
     def workspace(self, d: _lib.BpttDesc) -> torch.Tensor:
-        key = (d.batch, d.steps, d.checkpoint, d.smooth)
+        """The layer's workspace at d's sizes; sets d.segments to the form that it holds."""
+        key = (d.batch, d.steps, d.checkpoint, d.smooth, self.segments)
         if self._ws_key != key:
-            n = ctypes.c_size_t()
-            lib = _lib.load()
-            _lib.check(lib.n2b_bptt_workspace_bytes(ctypes.byref(d), ctypes.byref(n)), "n2b_bptt_workspace_bytes")
-            self._ws = torch.empty(n.value, dtype=torch.uint8, device=self.w_in.device)
-            self._ws_key = key
+            self._ws = None
+            dev, bytes_of = self.w_in.device, []
+            for segments in (0, 1):
+                d.segments, n = segments, ctypes.c_size_t()
+                _lib.check(_lib.load().n2b_bptt_workspace_bytes(ctypes.byref(d), ctypes.byref(n)),
+                           "n2b_bptt_workspace_bytes")
+                bytes_of.append(n.value)
+            forms = [int(self.segments)] if self.segments is not None else [0, 1]
+            if len(forms) > 1 and not torch.cuda.is_current_stream_capturing():
+                # the derivatives of every step take half of what is free at most: the rest is the program's
+                free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+                if bytes_of[0] - bytes_of[1] > free // 2:
+                    forms = [1]
+            for segments in forms:
+                try:
+                    self._ws = torch.empty(bytes_of[segments], dtype=torch.uint8, device=dev)
+                except torch.cuda.OutOfMemoryError:
+                    if segments == forms[-1]:
+                        raise
+                    continue
+                break
+            self._ws_segments, self._ws_key = segments, key
+        d.segments = self._ws_segments
         return self._ws
 
     def current(self, x, steps: int | None = None) -> torch.Tensor:

@@ -1315,7 +1315,8 @@ int bcuda(cudaError_t e, const char *what) {
 
 // A taped forward keeps the surrogate derivatives of every step when they take at most this much (the workload's
 // 128 x 500 x 1024 are 262 MB): 0.04 ms of writes under the forward instead of 0.18 ms of recomputing per segment of
-// 50 steps, of which the adjoint hides half. Larger layers keep the membrane every `checkpoint` steps and recompute.
+// 50 steps, of which the adjoint hides half. Larger layers, and those asked for it (desc.segments: their tape would leave
+// the program too little memory), keep the membrane every `checkpoint` steps and recompute.
 constexpr size_t FULL_TAPE_BYTES = (size_t)4 << 30;
 
 struct WsLayout {
@@ -1348,7 +1349,7 @@ bool scans(const n2b_bptt_desc *d) {
 }
 
 bool full_tape(const n2b_bptt_desc *d) {
-    return scans(d) && sizeof(float) * (size_t)d->steps * d->batch * d->hidden <= FULL_TAPE_BYTES;
+    return !d->segments && scans(d) && sizeof(float) * (size_t)d->steps * d->batch * d->hidden <= FULL_TAPE_BYTES;
 }
 
 WsLayout ws_layout(const n2b_bptt_desc *d) {

@@ -37,10 +37,10 @@ EDGE_CAP = {False: 16, True: MAX_ARRIVALS}  # arrivals whose edge values are loa
 EDGE_ATTRS = {False: 8, True: 2}  # ... of at most so many edge attributes
 OUT_CACHED = 8  # outgoing connections whose row bounds a block holds in shared memory
 PIECE = 256  # links of a row that a warp delivers at once, eight loads a lane in flight
-WORDS_AHEAD = 4  # incoming connections whose arrival words are loaded together at a step's start
-ROWS_AHEAD = 8  # incoming connections whose row bounds a thread holds
+AHEAD = (8, 4)  # incoming connections whose row bounds a thread holds, those whose arrival words are loaded together
 WINDOW_PARAMS = 16384  # bytes of a window kernel's parameter block at most
-WINDOW_POPS = 16  # populations of a window kernel at most (each is a copy of the step's code)
+WINDOW_POPS = 16  # populations of a window kernel at most
+WINDOW_INTAKES = 8  # connections that the code of a window kernel takes in at most, over its distinct populations
 
 _COMMON = r'''
 struct N2Out {
@@ -191,13 +191,13 @@ def _row_bounds(c: int) -> str:
             f"c{c}_w1 = live ? p.c{c}_wptr[j + 1] : 0;\n")
 
 
-def _chunk_head(c: int) -> str:
+def _chunk_head(c: int, ahead: tuple) -> str:
     """The loop over a row's words in chunks (the same number of them for the whole warp): word kb + SCAN i + sc is
     x[i] of the neuron's thread sc, four loads in flight; the first connections' first chunk is loaded already."""
-    again = "" if c < ROWS_AHEAD else f"            const int {_row_bounds(c)}"
-    if c >= ROWS_AHEAD:
+    again = "" if c < ahead[0] else f"            const int {_row_bounds(c)}"
+    if c >= ahead[0]:
         again += f"            const int c{c}_rounds = {_rounds(c)};\n"
-    first = f"x{c}[i]" if c < WORDS_AHEAD else "w0 + SCAN * i + sc < w1 ? __ldcg(arr + w0 + SCAN * i + sc) : 0u"
+    first = f"x{c}[i]" if c < ahead[1] else "w0 + SCAN * i + sc < w1 ? __ldcg(arr + w0 + SCAN * i + sc) : 0u"
     return f"""{again}            const int r0 = c{c}_r0, w0 = c{c}_w0, w1 = c{c}_w1;
             u32 *arr = p.c{c}_arr + (size_t)slot{c} * p.c{c}_arr_words;
             u32 x[4];
@@ -217,7 +217,7 @@ def _rounds(c: int) -> str:
     return f"(int)(__reduce_max_sync(0xffffffffu, (u32)(c{c}_w1 - c{c}_w0)) + CHUNK - 1) / CHUNK"
 
 
-def _words_ahead(incoming: list) -> str:
+def _words_ahead(incoming: list, ahead: tuple) -> str:
     """The first connections' first words, loaded together: their latencies overlap."""
     return "".join(f"""        u32 x{c}[4];
         {{
@@ -225,7 +225,7 @@ def _words_ahead(incoming: list) -> str:
             #pragma unroll
             for (int i = 0; i < 4; ++i) x{c}[i] = SCAN * i + sc < c{c}_w1 - c{c}_w0 ? __ldcg(arr + SCAN * i + sc) : 0u;
         }}
-""" for c, inc in enumerate(incoming[:WORDS_AHEAD]) if takes(inc))
+""" for c, inc in enumerate(incoming[:ahead[1]]) if takes(inc))
 
 
 # Each thread's first arrival (start[i]) of its word i among the neuron's arrivals of the chunk, in word order, and
@@ -251,7 +251,7 @@ def _stage_edges(c: int, inc: dict, exact: bool, at: str, pad: int) -> str:
                    for a, e in enumerate(inc["edge_dynamic"][:EDGE_ATTRS[exact]]))
 
 
-def _clocked_intake(c: int, inc: dict, body: str) -> str:
+def _clocked_intake(c: int, inc: dict, body: str, ahead: tuple) -> str:
     """Connection c's arrivals: the neuron's threads put their words with a set bit into shared memory and clear
     them; the neuron's first thread (the owner) runs the hooks over the words' bits, i.e. in link order. Edge values
     are loaded by the threads together, ahead of the owner's chain of hooks (of the chunk's first EDGE_CAP arrivals)."""
@@ -271,7 +271,7 @@ def _clocked_intake(c: int, inc: dict, body: str) -> str:
                       else f"float e_{e} = p.c{c}_e_{e}[l];\n")
     run = loads + ("++at;\n" if edges else "") + "link_k = arrived++;\n{\n" + body + "}\n"
     return f"""        {{  // connection {c}
-{_chunk_head(c)}{stage}                u32 some = 0u;  // the neuron's words of the chunk with a set bit
+{_chunk_head(c, ahead)}{stage}                u32 some = 0u;  // the neuron's words of the chunk with a set bit
                 #pragma unroll
                 for (int i = 0; i < 4; ++i) {{
                     some |= ((__ballot_sync(0xffffffffu, x[i] != 0u) >> (threadIdx.x & 31 & ~(SCAN - 1))) & ((1u << SCAN) - 1)) << (SCAN * i);
@@ -294,11 +294,11 @@ def _clocked_intake(c: int, inc: dict, body: str) -> str:
 """
 
 
-def _exact_collect(c: int, inc: dict) -> str:
+def _exact_collect(c: int, inc: dict, ahead: tuple) -> str:
     """Connection c's arrivals of the step into the neuron's list, in link order; past MAX_ARRIVALS they are counted
     and dropped."""
     return f"""        {{  // connection {c}
-{_chunk_head(c)}{_RANKS}                #pragma unroll
+{_chunk_head(c, ahead)}{_RANKS}                #pragma unroll
                 for (int i = 0; i < 4; ++i) {{
                     int at = na + start[i];
                     for (u32 v = x[i]; v; v &= v - 1, ++at) {{
@@ -462,7 +462,8 @@ def params_fields(attrs: dict, incoming: list, n_out: int, exact: bool) -> list:
     return fields
 
 
-def population(pop_name: str, attrs: dict, hooks: dict, incoming: list, n_out: int, exact: bool, fields: list) -> str:
+def population(pop_name: str, attrs: dict, hooks: dict, incoming: list, n_out: int, exact: bool, fields: list,
+               ahead: tuple) -> str:
     """A population's Params and its steps: `n2_steps`, n_steps of them from step n for the block `blk` (WINDOW: a
     grid barrier between them). Edge backward hooks that assign nothing of the destination run for a fired neuron's
     links on a group of warps (a link's hook touches that link alone), the others on the owner, link by link."""
@@ -481,7 +482,7 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
     # and the row bounds loaded while it is still running
     src.append('    if (!WINDOW) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");\n')
     src += [f"    const int {_row_bounds(c)}    const int c{c}_rounds = {_rounds(c)};\n"
-            for c, inc in enumerate(incoming[:ROWS_AHEAD]) if takes(inc)]
+            for c, inc in enumerate(incoming[:ahead[0]]) if takes(inc)]
     if n_out:
         src.append(f"""    for (int k = threadIdx.x; k < {min(n_out, OUT_CACHED)} * (NPB_C + 1); k += {THREADS}) {{
         const int q = k % (NPB_C + 1);
@@ -511,10 +512,10 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
             if (p.bad && blk == 0) atomicAdd(p.err, p.bad);
         }
         __syncthreads();
-""".replace("@WORDS@", _words_ahead(incoming)))
+""".replace("@WORDS@", _words_ahead(incoming, ahead)))
     if exact:
         src.append("        int na = 0;  // the neuron's arrivals of the step\n")
-        src += [_exact_collect(c, inc) for c, inc in enumerate(incoming) if takes(inc)]
+        src += [_exact_collect(c, inc, ahead) for c, inc in enumerate(incoming) if takes(inc)]
         if any(takes(inc) for inc in incoming):
             src += [_exact_times(incoming), _EXACT_SORT, _exact_deliver(pop_name, incoming, hooks)]
         else:  # the send of a time group has call sites of its own: without groups the step's send keeps its numbers
@@ -523,7 +524,7 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
     else:
         for c, inc in enumerate(incoming):
             if takes(inc):
-                src.append(_clocked_intake(c, inc, _arrival_body(pop_name, c, inc)))
+                src.append(_clocked_intake(c, inc, _arrival_body(pop_name, c, inc), ahead))
     src.append("        if (live && own) {\n")
     for name in ("update", "send"):
         fn, ctx = hooks[name]
@@ -587,12 +588,13 @@ extern "C" __global__ void __launch_bounds__({THREADS}) n2b_user_step(const __gr
 """
 
 
-def build(pop_name: str, attrs: dict, hooks: dict, incoming: list, n_out: int, exact: bool) -> tuple[str, list, str]:
+def build(pop_name: str, attrs: dict, hooks: dict, incoming: list, n_out: int, exact: bool,
+          ahead: tuple = AHEAD) -> tuple[str, list, str]:
     """(step kernel source, params fields, `population` text) of one population; the arguments are build_source's
     (template.py), with "backward_writes" per incoming connection: whether its backward hook assigns the
-    destination's state, and n_out: the population's outgoing connections."""
+    destination's state, n_out: the population's outgoing connections, and `ahead` (AHEAD)."""
     fields = params_fields(attrs, incoming, n_out, exact)
-    body = population(pop_name, attrs, hooks, incoming, n_out, exact, fields)
+    body = population(pop_name, attrs, hooks, incoming, n_out, exact, fields, ahead)
     return _PRELUDE + common(exact, staged(incoming, exact)) + body + STEP_KERNEL, fields, body
 
 
@@ -600,13 +602,16 @@ def blocks_of(n: int) -> int:
     return (n + NPB_C - 1) // NPB_C
 
 
-def window_source(exact: bool, bodies: list, sizes: list, edges: int, per_sm: int) -> str:
-    """The window kernel over every population: `bodies` their `population` texts, `sizes` their neurons, `edges` the
-    most edge attributes that one of them stages."""
+def window_source(exact: bool, kinds: list, edges: int, per_sm: int) -> str:
+    """The window kernel: `kinds` its distinct `population` texts and how many populations run each, in the order of the
+    parameter block (populations of one kind share its code); `edges` the most edge attributes that one of them stages;
+    `per_sm` the blocks that an SM holds at once. The populations' sizes are parameters: networks that differ in them
+    alone share the kernel."""
     src = [_PRELUDE, common(exact, edges)]
-    src += [f"namespace n2p{k} {{\n{body}}}\n\n" for k, body in enumerate(bodies)]
+    src += [f"namespace n2p{g} {{\n{body}}}\n\n" for g, (body, _) in enumerate(kinds)]
     src.append("struct Window {\n    long long step0;\n    double dt;\n    N2Grid grid;\n    long long n_steps;\n")
-    src += [f"    n2p{k}::Params p{k};\n" for k in range(len(bodies))]
+    src.append(f"    int first[{sum(count for _, count in kinds) + 1}];  // each population's first block, then their number\n")
+    src += [f"    n2p{g}::Params p{g}[{count}];\n" for g, (_, count) in enumerate(kinds)]
     src.append(f"""}};
 
 extern "C" __global__ void __launch_bounds__({THREADS}, {per_sm}) n2b_user_window(const __grid_constant__ Window w) {{
@@ -616,20 +621,22 @@ extern "C" __global__ void __launch_bounds__({THREADS}, {per_sm}) n2b_user_windo
         n2_finish(w.grid);
         return;
     }}
-    const int b = (int)blockIdx.x;
+    int k = 0;
+    while ((int)blockIdx.x >= w.first[k + 1]) ++k;
+    const int b = (int)blockIdx.x - w.first[k];
 """)
-    first = 0
-    for k, n in enumerate(sizes):
-        if n:
-            src.append(f"    if (b >= {first} && b < {first + blocks_of(n)}) n2p{k}::n2_steps<true>(w.p{k}, s, b - {first}, "
-                       "w.step0, (int)w.n_steps, w.dt, w.grid);\n")
-        first += blocks_of(n)
+    before = 0
+    for g, (_, count) in enumerate(kinds):
+        src.append(f"    if (k >= {before} && k < {before + count}) n2p{g}::n2_steps<true>(w.p{g}[{f'k - {before}' if count > 1 else 0}], "
+                   "s, b, w.step0, (int)w.n_steps, w.dt, w.grid);\n")
+        before += count
     src.append("    n2_finish(w.grid);\n}\n")
     return "".join(src)
 
 
-def window_type(params: list):
-    """The ctypes structure of a Window over the populations' Params types."""
+def window_type(kinds: list):
+    """The ctypes structure of a Window: per kind its Params type and its number of populations."""
     return type("Window", (ctypes.Structure,), {
-        "_fields_": [("step0", ctypes.c_int64), ("dt", ctypes.c_double), ("grid", Grid), ("n_steps", ctypes.c_int64)]
-                    + [(f"p{k}", t) for k, t in enumerate(params)]})
+        "_fields_": [("step0", ctypes.c_int64), ("dt", ctypes.c_double), ("grid", Grid), ("n_steps", ctypes.c_int64),
+                     ("first", ctypes.c_int32 * (sum(count for _, count in kinds) + 1))]
+                    + [(f"p{g}", t * count) for g, (t, count) in enumerate(kinds)]})

@@ -171,6 +171,8 @@ def plan_of(net) -> dict:
             outs[index[id(c._source)]].append([k, ci])
     arrivals = sum(arrival_bytes(len(p.shape), len(c.fabric.topology), depth[index[id(c._source)]])
                    for p, conns in zip(pops, incoming_of) for c in conns) <= ARRIVAL_BYTES
+    total = sum(arrival.blocks_of(len(p.shape)) for p in pops)
+    per_sm = -(-total // WINDOW_SMS)
     bodies, edges = [], 0  # arrival bits: the populations' part of the window kernel, edge attributes they stage
     for k, p in enumerate(pops):
         node = p.node
@@ -227,10 +229,13 @@ def plan_of(net) -> dict:
                                    "link": link.to(torch.int32).cpu(), "perm": perm.cpu(), "per_link": per_link,
                                    "written": list(ep.written), "conn_id": id(c)})
         plan["pops"].append(entry)
-    sizes = [len(p.shape) for p in pops]
-    total = sum(arrival.blocks_of(n) for n in sizes)
     if arrivals and 0 < total <= WINDOW_BLOCKS and len(pops) <= arrival.WINDOW_POPS:
-        plan["window"] = arrival.window_source(exact, bodies, sizes, edges, -(-total // WINDOW_SMS))
+        kinds = sorted(set(bodies), key=bodies.index)  # populations of one text share its code
+        if sum(len(incoming_of[bodies.index(b)]) for b in kinds) <= arrival.WINDOW_INTAKES:
+            order = sorted(range(len(pops)), key=lambda k: (kinds.index(bodies[k]), k))
+            counts = [bodies.count(b) for b in kinds]
+            plan["window"] = {"source": arrival.window_source(exact, list(zip(kinds, counts)), edges, per_sm),
+                              "order": order, "counts": counts}
     plan["device"] = dev
     return plan
 
@@ -241,7 +246,7 @@ def save_plan(plan: dict, path) -> None:
 
     arrays, meta = {}, {"dt": plan["dt"], "exact": plan["exact"], "pops": []}
     if "window" in plan:
-        meta["window_source"] = plan["window"]
+        meta["window_kernel"] = plan["window"]
     for k, p in enumerate(plan["pops"]):
         m = {key: p[key] for key in ("name", "n", "words", "depth", "seed", "source", "fields", "attrs", "outs")
              if key in p}
@@ -263,8 +268,8 @@ def load_plan(path) -> dict:
     z = np.load(path)
     meta = json.loads(bytes(z["plan_json"]).decode())
     plan = {"dt": meta["dt"], "exact": meta["exact"], "pops": []}
-    if "window_source" in meta:  # (a plan whose window kernel counts on its caller, "window", steps without it)
-        plan["window"] = meta["window_source"]
+    if "window_kernel" in meta:  # (an older plan's, under "window", takes other parameters: it steps without)
+        plan["window"] = meta["window_kernel"]
     for k, m in enumerate(meta["pops"]):
         p = dict(m)
         p["fields"] = [tuple(f) for f in m["fields"]]
@@ -321,12 +326,13 @@ class JitRuntime:
         self.raster_offs = [torch.zeros(max(1, self.record_rows) * max(1, p["n"]), dtype=torch.float32,
                                         device=dev) for p in plan["pops"]]
         self.kernels, self.params, self.sources = [], [], []
+        types: dict = {}  # Params fields -> their structure
         forms = []  # per population, its incoming connections' arrival forms
         self.edge_arrays = {}  # (connection id, edge name) -> (per-link values in pull order, pull permutation)
         tdtype = {"bool": torch.bool, "int": torch.int32, "float": torch.float32}
         for k, (p, pp) in enumerate(zip(pops, plan["pops"])):
             self.sources.append(pp["source"])
-            P = _params_struct(pp["fields"])()
+            P = types.setdefault(tuple(pp["fields"]), _params_struct(pp["fields"]))()
             P.n, P.words, P.bit_mask = pp["n"], words[k], depth[k] - 1
             P.seed_lo, P.seed_hi = pp["seed"] & 0xFFFFFFFF, (pp["seed"] >> 32) & 0xFFFFFFFF
             for a, ty in pp["attrs"].items():
@@ -391,17 +397,24 @@ class JitRuntime:
         self._s = ctypes.c_void_p(self.stream.cuda_stream)
         self.launches = 0
 
-    def _window(self, source: str, dindex: int) -> None:
+    def _window(self, plan: dict, dindex: int) -> None:
         """The window kernel, where its parameters fit and the device holds all its blocks at once."""
-        W = arrival.window_type([type(P) for P in self.params])
+        slots, kinds, at = [], [], 0  # per population in the block's order: (its kind, its place among them)
+        for g, count in enumerate(plan["counts"]):
+            kinds.append((type(self.params[plan["order"][at]]), count))
+            slots += [(plan["order"][at + i], g, i) for i in range(count)]
+            at += count
+        W = arrival.window_type(kinds)
         if ctypes.sizeof(W) > arrival.WINDOW_PARAMS:
             return
-        lib, kern, blocks = _lib.load(), compile_source(source, dindex, b"n2b_user_window"), ctypes.c_int32()
+        lib, kern, blocks = _lib.load(), compile_source(plan["source"], dindex, b"n2b_user_window"), ctypes.c_int32()
         _lib.check(lib.n2b_jit_resident_blocks(kern, arrival.THREADS, ctypes.byref(blocks)), "n2b_jit_resident_blocks")
         if blocks.value >= self.window_grid:
-            self.window_kernel, self.window = kern, W()
+            self.window_kernel, self.window, self.window_slots = kern, W(), slots
             self.window.dt = self.dt
             self.window.grid.bar = self.bar.data_ptr()
+            for at, (k, _, _) in enumerate(slots):
+                self.window.first[at + 1] = self.window.first[at] + arrival.blocks_of(self.plan["pops"][k]["n"])
 
     def _dev(self, t):
         t = t.to(self.device).contiguous()
@@ -432,8 +445,8 @@ class JitRuntime:
         lib, W = _lib.load(), self.window
         W.step0, W.n_steps = step, n_steps
         W.grid.limit_ns = int(getattr(self.net, "barrier_limit_ns", 0) or BARRIER_LIMIT_NS)
-        for k, P in enumerate(self.params):
-            setattr(W, f"p{k}", P)
+        for k, g, i in self.window_slots:
+            getattr(W, f"p{g}")[i] = self.params[k]
         _lib.check(lib.n2b_jit_launch_cooperative(self.window_kernel, self.window_grid, arrival.THREADS,
                                                   ctypes.addressof(W), ctypes.sizeof(W), self._s),
                    "n2b_jit_launch_cooperative")

@@ -42,7 +42,7 @@ def test_one_thread_reads_the_stop_word():
     for at in reads:
         line = text[text.rindex("\n", 0, at):text.index("\n", at)]
         assert "__syncthreads_or(threadIdx.x == 0 && " in line or "(spin & 15) == 15" in line, line
-    window = plan_of(_user_net())["window"]
+    window = plan_of(_user_net())["window"]["source"]
     kernel = window[window.index("n2b_user_window"):]
     assert re.search(r"if \(__syncthreads_or\(threadIdx\.x == 0 && \*\(volatile u32 \*\)\(w\.grid\.bar \+ 32\)\)\)",
                      kernel)

@@ -37,7 +37,10 @@ EDGE_CAP = {False: 16, True: MAX_ARRIVALS}  # arrivals whose edge values are loa
 EDGE_ATTRS = {False: 8, True: 2}  # ... of at most so many edge attributes
 OUT_CACHED = 8  # outgoing connections whose row bounds a block holds in shared memory
 PIECE = 256  # links of a row that a warp delivers at once, eight loads a lane in flight
-AHEAD = (8, 4)  # incoming connections whose row bounds a thread holds, those whose arrival words are loaded together
+# (incoming connections whose row bounds a thread holds, those of them whose arrival words are loaded together at a
+# step's start). Four blocks on an SM leave a thread 64 registers, three 80: with (8, 4), 4 connections spill 56 bytes at
+# 64 and 8 connections 224, with (2, 2) none.
+AHEAD, AHEAD_FEW = (8, 4), (2, 2)
 WINDOW_PARAMS = 16384  # bytes of a window kernel's parameter block at most
 WINDOW_POPS = 16  # populations of a window kernel at most
 WINDOW_INTAKES = 8  # connections that the code of a window kernel takes in at most, over its distinct populations

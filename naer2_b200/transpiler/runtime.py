@@ -173,6 +173,7 @@ def plan_of(net) -> dict:
                    for p, conns in zip(pops, incoming_of) for c in conns) <= ARRIVAL_BYTES
     total = sum(arrival.blocks_of(len(p.shape)) for p in pops)
     per_sm = -(-total // WINDOW_SMS)
+    ahead = arrival.AHEAD_FEW if 2 * WINDOW_SMS < total <= WINDOW_BLOCKS else arrival.AHEAD
     bodies, edges = [], 0  # arrival bits: the populations' part of the window kernel, edge attributes they stage
     for k, p in enumerate(pops):
         node = p.node
@@ -204,7 +205,7 @@ def plan_of(net) -> dict:
                  "send": (node.send.ast, hook_context(p, node.send, site_base=site + 32))}
         if arrivals:
             src, fields, body = arrival.build(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
-                                              len(outs[k]), exact)
+                                              len(outs[k]), exact, ahead)
             bodies.append(body)
             edges = max(edges, arrival.staged(incoming, exact))
         else:

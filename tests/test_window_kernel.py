@@ -5,12 +5,14 @@ scanning intake's results bit for bit."""
 
 import itertools
 import re
+import subprocess
 
 import numpy as np
 import pytest
 import torch
 
 from naer2_b200 import population
+from naer2_b200.build import ARCH, nvcc
 from naer2_b200.patterns import fixed_indegree
 from naer2_b200.transpiler import JitRuntime, plan_of
 from naer2_b200.transpiler import runtime as jit_runtime
@@ -93,3 +95,14 @@ def test_populations_that_share_code_match_the_scanning_intake(cuda, monkeypatch
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
     assert sum(int(np.unpackbits(w.view(np.uint8)).sum()) for w in want[:len(sizes)]) > 50
+
+
+@pytest.mark.parametrize("pops, per", [(4, 4500), (8, 2300), (8, 1700)])
+def test_full_networks_spill_no_registers(tmp_path, pops, per):
+    """At three and four blocks per SM, with as many connections as a window kernel takes in."""
+    plan = plan_of(_net((per,) * pops, (1.0,) * pops, k=1))
+    src = tmp_path / "window.cu"
+    src.write_text(plan["window"]["source"])
+    out = subprocess.run([nvcc(), *ARCH, "-std=c++17", "--fmad=false", "-Xptxas", "-v", "-cubin", "-o",
+                          str(tmp_path / "window.cubin"), str(src)], capture_output=True, text=True, check=True)
+    assert "0 bytes spill stores, 0 bytes spill loads" in out.stderr, out.stderr

@@ -125,3 +125,11 @@ def check(rc: int, what: str) -> None:
     if rc != 0:
         msg = load().n2b_last_error().decode(errors="replace")
         raise RuntimeError(f"{what} failed ({rc}): {msg}")
+
+
+def free_bytes(device) -> int:
+    """Device memory that an allocation can still have: the device's free memory and what torch's allocator holds free."""
+    import torch
+
+    return (torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device)
+            - torch.cuda.memory_allocated(device))

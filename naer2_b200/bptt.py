@@ -286,8 +286,7 @@ class RecurrentLIF(torch.nn.Module):
             forms = [int(self.segments)] if self.segments is not None else [0, 1]
             if len(forms) > 1 and not torch.cuda.is_current_stream_capturing():
                 # the derivatives of every step take half of what is free at most: the rest is the program's
-                free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-                if bytes_of[0] - bytes_of[1] > free // 2:
+                if bytes_of[0] - bytes_of[1] > _lib.free_bytes(dev) // 2:
                     forms = [1]
             for segments in forms:
                 try:

@@ -25,10 +25,12 @@ from .template import NPB_C, build_source, ctype_of, edge_hook_context, hook_con
 
 BLOCK = 128  # exact-time intake without arrival bits: one thread per neuron
 # A network's intake reads arrival bits (one bit per link and arrival slot, set by the spikes' deliveries) as long
-# as they and the outgoing rows take at most this much; past it, every neuron looks its whole incoming row up in
-# its sources' spike rings, which needs no more memory than the links. At 12,500 neurons of 1,250 links and 32
-# slots the bits are 64 MB, the rows 78 MB.
+# as they and the outgoing rows take at most this much, and half of the device's free memory with what making them
+# holds at once (BUILD_BYTES per link of a connection: int64 columns and a sort, 52 measured); past it, every neuron
+# looks its whole incoming row up in its sources' spike rings, which needs no more memory than the links. At 12,500
+# neurons of 1,250 links and 32 slots the bits are 64 MB, the rows 78 MB.
 ARRIVAL_BYTES = 32 << 30
+BUILD_BYTES = 72
 # A window kernel holds every block of the network at once: 592 blocks (18,944 neurons) are four per SM, 64 registers
 # a thread, which the step's code needs (five per SM would be 51). Larger networks, those of more than
 # arrival.WINDOW_POPS populations, and devices that hold fewer blocks step by one launch per population.
@@ -139,6 +141,21 @@ def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -
             "dly": None if packed else dly.to(torch.uint8), "bad": bad}
 
 
+def scan_form(plan: dict) -> dict:
+    """A plan of arrival bits as one of the scanning intake, which needs no memory beside the links."""
+    out = {key: v for key, v in plan.items() if key != "window"}
+    out["pops"] = [{**{key: v for key, v in p.items() if key not in ("outs", "scan")}, **p["scan"]} for p in plan["pops"]]
+    return out
+
+
+def arrivals_need(plan: dict) -> int:
+    """Device bytes of a plan's arrival bits and outgoing rows, and of building the largest connection's."""
+    pops = plan["pops"]
+    sizes = [(arrival_bytes(p["n"], len(c["link"]), pops[c["src"]]["depth"]), BUILD_BYTES * len(c["link"]))
+             for p in pops for c in p["conns"]]
+    return sum(t for t, _ in sizes) + max((b for _, b in sizes), default=0)
+
+
 def plan_of(net) -> dict:
     """The transpiled form of a network, everything its step kernels need and nothing of its Python model classes:
     per population its CUDA source, the Params fields with the values of the scalar ones, its state attributes
@@ -176,47 +193,49 @@ def plan_of(net) -> dict:
     ahead = arrival.AHEAD_FEW if 2 * WINDOW_SMS < total <= WINDOW_BLOCKS else arrival.AHEAD
     bodies, edges = [], 0  # arrival bits: the populations' part of the window kernel, edge attributes they stage
     for k, p in enumerate(pops):
-        node = p.node
-        incoming = []
-        conns = incoming_of[k]
-        site = 0
-        for c in conns:
-            port = c._target_port or "receive"
-            hook = node.receive.get(port)
-            if hook is None:
-                raise ValueError(f"{p!r} has no receive port {port!r}")
-            ep = EdgePlan(c, hook)
-            dyn = [h for h, real in ep.recv.items() if real in ep.per_link]
-            stat = {h: ep.static[real] for h, real in ep.recv.items() if real not in ep.per_link}
-            ctx = hook_context(p, hook, dyn, stat, site_base=site)
-            site += 32
-            inc = {"receive": (hook.ast, ctx), "edge_dynamic": ep.per_link, "edge_written": ep.written,
-                   "alias": {h: real for h, real in ep.recv.items() if real in ep.per_link and h != real},
-                   "forward": None, "backward": None, "conn": c, "plan": ep}
-            for kind in ("forward", "backward"):
-                eh = getattr(ep, kind)
-                if eh is not None:
-                    inc[kind] = (eh.ast, edge_hook_context(p, eh, ep.per_link, ep.static))
-            if ep.backward is not None:
-                dst = ep.backward.parameter_type_to_name.get(receives.destination)
-                inc["backward_writes"] = dst is not None and bool(assigned_members(ep.backward.ast, dst))
-            incoming.append(inc)
-        hooks = {"update": (node.update.ast, hook_context(p, node.update, site_base=site)),
-                 "send": (node.send.ast, hook_context(p, node.send, site_base=site + 32))}
+        node, conns, name = p.node, incoming_of[k], type(p.instance).__name__
+
+        def lowered() -> tuple[list, dict]:
+            """The incoming connections and the hooks as a source takes them (their draws' call sites count from here)."""
+            incoming, site = [], 0
+            for c in conns:
+                port = c._target_port or "receive"
+                hook = node.receive.get(port)
+                if hook is None:
+                    raise ValueError(f"{p!r} has no receive port {port!r}")
+                ep = EdgePlan(c, hook)
+                dyn = [h for h, real in ep.recv.items() if real in ep.per_link]
+                stat = {h: ep.static[real] for h, real in ep.recv.items() if real not in ep.per_link}
+                ctx = hook_context(p, hook, dyn, stat, site_base=site)
+                site += 32
+                inc = {"receive": (hook.ast, ctx), "edge_dynamic": ep.per_link, "edge_written": ep.written,
+                       "alias": {h: real for h, real in ep.recv.items() if real in ep.per_link and h != real},
+                       "forward": None, "backward": None, "conn": c, "plan": ep}
+                for kind in ("forward", "backward"):
+                    eh = getattr(ep, kind)
+                    if eh is not None:
+                        inc[kind] = (eh.ast, edge_hook_context(p, eh, ep.per_link, ep.static))
+                if ep.backward is not None:
+                    dst = ep.backward.parameter_type_to_name.get(receives.destination)
+                    inc["backward_writes"] = dst is not None and bool(assigned_members(ep.backward.ast, dst))
+                incoming.append(inc)
+            return incoming, {"update": (node.update.ast, hook_context(p, node.update, site_base=site)),
+                              "send": (node.send.ast, hook_context(p, node.send, site_base=site + 32))}
+
+        incoming, hooks = lowered()
+        src, fields = build_source(name, dict(p.dynamic_attrs), hooks, incoming, exact=exact, n=len(p.shape))
+        scanning = {"source": src, "fields": [(f, ctype) for f, ctype, _ in fields]}
         if arrivals:
-            src, fields, body = arrival.build(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
-                                              len(outs[k]), exact, ahead)
+            incoming, hooks = lowered()
+            src, fields, body = arrival.build(name, dict(p.dynamic_attrs), hooks, incoming, len(outs[k]), exact, ahead)
             bodies.append(body)
             edges = max(edges, arrival.staged(incoming, exact))
-        else:
-            src, fields = build_source(type(p.instance).__name__, dict(p.dynamic_attrs), hooks, incoming,
-                                       exact=exact, n=len(p.shape))
         attrs = {a: ("bool" if py is bool else "int" if py is int else "float") for a, py in p.dynamic_attrs.items()}
-        entry = {"name": type(p.instance).__name__, "n": len(p.shape), "words": words[k], "depth": depth[k],
+        entry = {"name": name, "n": len(p.shape), "words": words[k], "depth": depth[k],
                  "seed": int(p.seed) & 0xFFFFFFFFFFFFFFFF, "source": src,
                  "fields": [(name, ctype) for name, ctype, _ in fields], "attrs": attrs, "conns": []}
         if arrivals:
-            entry["outs"] = outs[k]
+            entry["outs"], entry["scan"] = outs[k], scanning
         for inc in incoming:
             c = inc["conn"]
             topo = c.fabric.topology
@@ -249,8 +268,8 @@ def save_plan(plan: dict, path) -> None:
     if "window" in plan:
         meta["window_kernel"] = plan["window"]
     for k, p in enumerate(plan["pops"]):
-        m = {key: p[key] for key in ("name", "n", "words", "depth", "seed", "source", "fields", "attrs", "outs")
-             if key in p}
+        m = {key: p[key] for key in ("name", "n", "words", "depth", "seed", "source", "fields", "attrs", "outs",
+                                      "scan") if key in p}
         m["conns"] = []
         for ci, c in enumerate(p["conns"]):
             for key in ("ptr", "link", "perm"):
@@ -274,6 +293,8 @@ def load_plan(path) -> dict:
     for k, m in enumerate(meta["pops"]):
         p = dict(m)
         p["fields"] = [tuple(f) for f in m["fields"]]
+        if "scan" in m:
+            p["scan"] = {"source": m["scan"]["source"], "fields": [tuple(f) for f in m["scan"]["fields"]]}
         p["conns"] = []
         for ci, c in enumerate(m["conns"]):
             p["conns"].append({"src": c["src"], "written": c["written"], "conn_id": None,
@@ -308,6 +329,10 @@ class JitRuntime:
         dindex = dev.index if dev.index is not None else 0
         if plan is None:
             plan = plan_of(net)
+        # arrival bits where they, and making them, take half of what is free on the device at most (plans of an older
+        # version have no other form)
+        if any("scan" in p for p in plan["pops"]) and arrivals_need(plan) > _lib.free_bytes(dev) // 2:
+            plan = scan_form(plan)
         self.plan = plan
         dt = self.dt = float(plan["dt"])
         pops = self.pops = list(net.populations)

@@ -13,6 +13,7 @@ from __future__ import annotations
 import ast
 import ctypes
 import hashlib
+import warnings
 
 import numpy as np
 import torch
@@ -31,9 +32,11 @@ BLOCK = 128  # exact-time intake without arrival bits: one thread per neuron
 # neurons of 1,250 links and 32 slots the bits are 64 MB, the rows 78 MB.
 ARRIVAL_BYTES = 32 << 30
 BUILD_BYTES = 72
+PARAMS_BYTES = 32764  # a kernel's parameters at most (48 bytes per outgoing connection, 40 to 64 per incoming one)
 # A window kernel holds every block of the network at once: 592 blocks (18,944 neurons) are four per SM, 64 registers
 # a thread, which the step's code needs (five per SM would be 51). Larger networks, those of more than
-# arrival.WINDOW_POPS populations, and devices that hold fewer blocks step by one launch per population.
+# arrival.WINDOW_POPS populations or, over the distinct ones, arrival.WINDOW_INTAKES connections, and devices that hold
+# fewer blocks step by one launch per population.
 WINDOW_BLOCKS, WINDOW_SMS = 592, 148
 BARRIER_LIMIT_NS = 2_000_000_000  # how long a window's block waits at its grid barrier before it gives up
 _CACHE: dict = {}  # (source hash, device) -> n2b_jit_kernel handle, for the process's lifetime
@@ -319,6 +322,12 @@ def _params_struct(fields: list):
     return params_type([(name, ct, ctype(ct)) for name, ct in fields])
 
 
+def _kinds(window: dict, types: list) -> list:
+    """arrival.window_type's kinds of a plan's window, `types` the populations' Params."""
+    first = np.cumsum([0] + window["counts"])
+    return [(types[window["order"][at]], count) for at, count in zip(first, window["counts"])]
+
+
 class JitRuntime:
     """The step kernels of a transpiled network: built from `net` (its plan made on the spot), or from a saved
     plan (`plan`; `net` then a PlannedNetwork holding the plan's state)."""
@@ -333,6 +342,7 @@ class JitRuntime:
         # version have no other form)
         if any("scan" in p for p in plan["pops"]) and arrivals_need(plan) > _lib.free_bytes(dev) // 2:
             plan = scan_form(plan)
+        plan, window_kernel, self.kernels = self._compiled(plan, dindex)
         self.plan = plan
         dt = self.dt = float(plan["dt"])
         pops = self.pops = list(net.populations)
@@ -351,7 +361,7 @@ class JitRuntime:
         self.rasters = [torch.zeros(max(1, self.record_rows) * w, dtype=torch.int32, device=dev) for w in words]
         self.raster_offs = [torch.zeros(max(1, self.record_rows) * max(1, p["n"]), dtype=torch.float32,
                                         device=dev) for p in plan["pops"]]
-        self.kernels, self.params, self.sources = [], [], []
+        self.params, self.sources = [], []
         types: dict = {}  # Params fields -> their structure
         forms = []  # per population, its incoming connections' arrival forms
         self.edge_arrays = {}  # (connection id, edge name) -> (per-link values in pull order, pull permutation)
@@ -415,32 +425,47 @@ class JitRuntime:
         self.window = self.window_kernel = None  # the window kernel and its parameter block
         self.window_grid = sum(arrival.blocks_of(p["n"]) for p in plan["pops"])
         self.bar = torch.zeros(64, dtype=torch.int32, device=dev)  # its grid barrier (N2Grid)
-        if "window" in plan:
-            self._window(plan["window"], dindex)
-        if self.window is None:
-            self.kernels = [compile_source(src, dindex) for src in self.sources]
+        if window_kernel is not None:
+            self._window(plan["window"], window_kernel)
         self.stream = torch.cuda.Stream(device=dev)
         self._s = ctypes.c_void_p(self.stream.cuda_stream)
         self.launches = 0
 
-    def _window(self, plan: dict, dindex: int) -> None:
-        """The window kernel, where its parameters fit and the device holds all its blocks at once."""
-        slots, kinds, at = [], [], 0  # per population in the block's order: (its kind, its place among them)
+    def _compiled(self, plan: dict, dindex: int) -> tuple:
+        """(the plan's form to run, its window kernel or None, else its step kernels). The window kernel where it
+        compiles, its parameters fit and the device holds all its blocks at once; else a kernel per population, of the
+        scanning intake where those of the arrival bits do not compile or their parameters do not fit."""
+        types = [_params_struct(p["fields"]) for p in plan["pops"]]
+        scans = any("scan" in p for p in plan["pops"])
+        if scans and any(ctypes.sizeof(t) > PARAMS_BYTES for t in types):
+            return self._compiled(scan_form(plan), dindex)
+        if "window" in plan and ctypes.sizeof(arrival.window_type(_kinds(plan["window"], types))) <= arrival.WINDOW_PARAMS:
+            try:
+                kern, blocks = compile_source(plan["window"]["source"], dindex, b"n2b_user_window"), ctypes.c_int32()
+                _lib.check(_lib.load().n2b_jit_resident_blocks(kern, arrival.THREADS, ctypes.byref(blocks)),
+                           "n2b_jit_resident_blocks")
+                if blocks.value >= sum(arrival.blocks_of(p["n"]) for p in plan["pops"]):
+                    return plan, kern, []
+            except RuntimeError as e:
+                warnings.warn(f"no window kernel ({e}): one launch per population and step", stacklevel=4)
+        try:
+            return plan, None, [compile_source(p["source"], dindex) for p in plan["pops"]]
+        except RuntimeError as e:
+            if not scans:
+                raise
+            warnings.warn(f"no arrival bits ({e}): every link's source is looked up", stacklevel=4)
+            return self._compiled(scan_form(plan), dindex)
+
+    def _window(self, plan: dict, kern: ctypes.c_void_p) -> None:
+        """The window kernel's parameter block."""
+        self.window_kernel, self.window = kern, arrival.window_type(_kinds(plan, [type(P) for P in self.params]))()
+        self.window.dt = self.dt
+        self.window.grid.bar = self.bar.data_ptr()
+        self.window_slots = []  # per population in the block's order: (its index, its kind, its place among them)
         for g, count in enumerate(plan["counts"]):
-            kinds.append((type(self.params[plan["order"][at]]), count))
-            slots += [(plan["order"][at + i], g, i) for i in range(count)]
-            at += count
-        W = arrival.window_type(kinds)
-        if ctypes.sizeof(W) > arrival.WINDOW_PARAMS:
-            return
-        lib, kern, blocks = _lib.load(), compile_source(plan["source"], dindex, b"n2b_user_window"), ctypes.c_int32()
-        _lib.check(lib.n2b_jit_resident_blocks(kern, arrival.THREADS, ctypes.byref(blocks)), "n2b_jit_resident_blocks")
-        if blocks.value >= self.window_grid:
-            self.window_kernel, self.window, self.window_slots = kern, W(), slots
-            self.window.dt = self.dt
-            self.window.grid.bar = self.bar.data_ptr()
-            for at, (k, _, _) in enumerate(slots):
-                self.window.first[at + 1] = self.window.first[at] + arrival.blocks_of(self.plan["pops"][k]["n"])
+            self.window_slots += [(plan["order"][len(self.window_slots) + i], g, i) for i in range(count)]
+        for at, (k, _, _) in enumerate(self.window_slots):
+            self.window.first[at + 1] = self.window.first[at] + arrival.blocks_of(self.plan["pops"][k]["n"])
 
     def _dev(self, t):
         t = t.to(self.device).contiguous()

@@ -32,6 +32,7 @@ BLOCK = 128  # exact-time intake without arrival bits: one thread per neuron
 # neurons of 1,250 links and 32 slots the bits are 64 MB, the rows 78 MB.
 ARRIVAL_BYTES = 32 << 30
 BUILD_BYTES = 72
+PACKED_BITS = 1 << 24  # bits of a slot whose places leave a link word's top 8 bits to the delay
 PARAMS_BYTES = 32764  # a kernel's parameters at most (48 bytes per outgoing connection, 40 to 64 per incoming one)
 # A window kernel holds every block of the network at once: 592 blocks (18,944 neurons) are four per SM, 64 registers
 # a thread, which the step's code needs (five per SM would be 51). Larger networks, those of more than
@@ -135,7 +136,7 @@ def arrival_form(ptr: torch.Tensor, link: torch.Tensor, n_src: int, mask: int) -
     dly = dly[order]
     top = int(dly.max()) if dly.numel() else 1
     pos, words = pos[order], int(wptr[-1])
-    packed = 32 * words <= 1 << 24
+    packed = 32 * words <= PACKED_BITS
     if packed:
         pos = pos | (dly.to(torch.int64) << 24)
     return {"wptr": wptr.to(torch.int32), "words": words, "depth": top + 1,

@@ -177,7 +177,8 @@ int n2b_replay(n2b_net *net, int64_t n_windows, void *stream);
 int n2b_advance(n2b_net *net, int64_t n_steps, int32_t window_steps, void *stream, void *caller);
 
 /* Set the step counter (asynchronously, on `stream`); work of the previous
- * step still in the work list is dropped. */
+ * step still in the work list is dropped (a network whose steps run without a
+ * barrier between them has none: what its steps sent is in the arrival slots). */
 int n2b_set_step(n2b_net *net, int64_t step, void *stream);
 
 /* Start recording: raster row r of every population holds step step0 + r

@@ -111,6 +111,10 @@ int validate(const n2b_population *pops, int32_t n_pops, const n2b_connection *c
     const int32_t block = block_of(opt);
     if (block != 64 && block != 128 && block != 256) return fail(N2B_EINVAL, "block must be 64, 128 or 256");
     if (opt && opt->barrier_limit_ns < 0) return fail(N2B_EINVAL, "barrier_limit_ns < 0");
+    if (opt && opt->chunk < 0) return fail(N2B_EINVAL, "chunk < 0");
+    if (opt && opt->chunk_block != 0 && opt->chunk_block != 32 && opt->chunk_block != 64 && opt->chunk_block != 128 &&
+        opt->chunk_block != 256)
+        return fail(N2B_EINVAL, "chunk_block must be 0, 32, 64, 128 or 256");
     for (int32_t p = 0; p < n_pops; ++p) {
         const n2b_population &P = pops[p];
         const std::string at = "population " + std::to_string(p) + ": ";
@@ -263,11 +267,13 @@ int coresident_blocks(int32_t block, bool inl, int kind, int device, size_t dyn,
 
 // How many steps of a network of push connections need no grid barrier between them: the smallest delay of its
 // links, as far as every population's slots hold that many steps past its largest incoming delay; below 2, 0 (a
-// barrier per step, the deliveries of delay >= 2 spread over the grid). Reads the links once; the room of the push table,
-// not yet written, holds the ranges.
+// barrier per step, the deliveries of delay >= 2 spread over the grid).
+// Reads the links once; the room of the push table, not yet written, holds the ranges.
 int chunk_steps(const n2b_population *pops, int32_t n_pops, const std::vector<n2b::ConnDev> &push,
-                const std::vector<int32_t> &push_tgt, char *ws, const Layout &L, cudaStream_t s, int32_t *out) {
+                const std::vector<int32_t> &push_tgt, char *ws, const Layout &L, cudaStream_t s, int32_t most,
+                int32_t *out) {
     *out = 0;
+    if (most == 1) return N2B_OK;  // n2b_options.chunk
     std::vector<int32_t> range(2 * push.size());
     for (size_t c = 0; c < push.size(); ++c) {
         range[2 * c] = 255;
@@ -290,6 +296,7 @@ int chunk_steps(const n2b_population *pops, int32_t n_pops, const std::vector<n2
     for (size_t c = 0; c < push.size(); ++c)
         if (push[c].n_links > 0 && pops[push_tgt[c]].n > 0)
             k = std::min(k, std::min(range[2 * c], pops[push_tgt[c]].acc_depth - range[2 * c + 1]));
+    if (most > 0) k = std::min(k, most);
     if (k >= 2) *out = k;
     return N2B_OK;
 }
@@ -469,7 +476,7 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
                      (int32_t)pull.size() <= n2b::INLINE_PULL;
     int32_t chunk = 0;
     if (persistent && inl && pull.empty() && L.n_tiles > 0) {
-        rc = chunk_steps(pops, n_pops, push, push_tgt, ws, L, s, &chunk);
+        rc = chunk_steps(pops, n_pops, push, push_tgt, ws, L, s, opt ? opt->chunk : 0, &chunk);
         if (rc) return rc;
     }
     if (n_pops) N2B_CUDA(cudaMemcpyAsync(ws + L.pops, pd.data(), sizeof(n2b::PopDev) * n_pops, cudaMemcpyHostToDevice, s));
@@ -534,7 +541,7 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
         for (chunk_tn = 32;; chunk_tn *= 2) {
             chunk_tiles = 0;
             for (int32_t p = 0; p < n_pops; ++p) chunk_tiles += (pops[p].n + chunk_tn - 1) / chunk_tn;
-            if (chunk_tiles <= 2 * sms || chunk_tn == 256) break;
+            if (opt && opt->chunk_block ? chunk_tn == opt->chunk_block : (chunk_tiles <= 2 * sms || chunk_tn == 256)) break;
         }
         chunk = std::min(chunk, n2b::chunk_most(chunk_tn));
         int per_sm = 0;

@@ -29,6 +29,9 @@ class Network:
         # a window of steps as one persistent cooperative launch (steps separated by a grid barrier), or one
         # launch per step
         self.persistent: bool = True
+        # persistent windows: steps that run without a grid barrier between them at most, where every delay allows it
+        # (None: the library's choice; 1: a barrier per step)
+        self.steps_per_barrier: int | None = None
         # persistent windows: how long a block may wait at a grid barrier before the window stops with an error
         # word (0: the library's 2 s); tests set a few ns to make the wait give up without a hang
         self.barrier_limit_ns: int = 0

@@ -36,6 +36,7 @@ from .topology import delay_steps, pack_links, pull_split_form, push_form
 
 MAX_SHIFT = 40
 MAX_LOOKAHEAD = 32  # steps without a grid barrier between them, at most (csrc/n2b_device.cuh, CHUNK_MAX)
+INLINE_POPS, INLINE_PUSH = 32, 64  # populations and push connections of a network that may (csrc/n2b_device.cuh)
 
 
 def next_pow2(x: int) -> int:
@@ -222,6 +223,14 @@ def describe(net, modes: dict | None = None, forms: bool = True) -> NetDesc:
                    max_in_delay=max_in_delay)
 
 
+def lookahead(net, desc: NetDesc) -> int:
+    """Steps that the library may run without a grid barrier between them, slots permitting (1: none)."""
+    k = desc.lookahead if net.persistent and len(desc.pops) <= INLINE_POPS and len(desc.conns) <= INLINE_PUSH else 1
+    if net.steps_per_barrier:
+        return min(k, int(net.steps_per_barrier))
+    return k
+
+
 class NetworkRuntime:
     """Device buffers + libnaer2b handle of one network (built by Network.runtime)."""
 
@@ -292,7 +301,8 @@ class NetworkRuntime:
         block = net.block or min([p.group_size for p in pops] + [256])
         block = 64 if block <= 64 else 128 if block <= 128 else 256
         self.opt = _lib.Options(block=block, device=dev.index if dev.index is not None else 0, grid=int(net.grid or 0),
-                                persistent=int(bool(net.persistent)),
+                                persistent=int(bool(net.persistent)), chunk=int(net.steps_per_barrier or 0),
+                                chunk_block=block if net.block else 0,
                                 barrier_limit_ns=int(getattr(net, "barrier_limit_ns", 0) or 0))
         nbytes = ctypes.c_size_t()
         _lib.check(lib.n2b_workspace_bytes(self.cpop, len(pops), self.cconn, len(desc.conns), ctypes.byref(self.opt),

@@ -1,7 +1,8 @@
 """The autotuner: picks a network's launch configuration by measuring it.
 
 Candidates differ in neurons per block (128 / 256), in how a window is launched (one persistent cooperative
-launch, or one launch per step), in the grid (the library's default, or every co-resident block for a
+launch, or one launch per step), in how many of its steps run without a grid barrier between them (networks whose
+delays allow it: the library's choice, also with its own block size, or none), in the grid (the library's default, or every co-resident block for a
 persistent launch: RESIDENT), and in push or pull per connection. The push/pull split comes
 from a cost model fitted on a short all-push run: per connection, push moves (spikes of its source per step)
 x (its mean row length) link words, scattered into the target's arrival slots, while pull streams every one
@@ -9,7 +10,7 @@ of its links every step against the source's spike bits; pull is a candidate for
 bytes per step are below push's times `pull_factor`. Every candidate runs from the same initial state (the
 population tensors are restored after each trial, and every trial builds its runtime anew, its rings empty),
 for `steps` steps after `warmup`, timed with CUDA events; the fastest is kept (net.block, net.grid,
-net.persistent, net.tuned) and the network is left at its initial state with no runtime.
+net.persistent, net.steps_per_barrier, net.tuned) and the network is left at its initial state with no runtime.
 """
 
 from __future__ import annotations
@@ -18,6 +19,8 @@ import itertools
 import time
 
 import torch
+
+from .runtime import NetworkRuntime, lookahead
 
 
 def _snapshot(net) -> dict:
@@ -87,51 +90,55 @@ def autotune(net, steps: int = 300, warmup: int = 100, blocks=(128, 256), persis
     if net.device is None or net.device.type != "cuda":
         raise RuntimeError("autotune needs the network on a CUDA device")
     snap = _snapshot(net)
-    saved = (net.block, net.grid, net.persistent, dict(net.tuned), net.window, net.record_steps)
+    saved = (net.block, net.grid, net.persistent, dict(net.tuned), net.window, net.record_steps, net.steps_per_barrier)
     net.record_steps = 0
     net.window = max(net.window, steps)
     report = {"trials": []}
     try:
         # the all-push baseline first: it also measures the rates the cost model needs
         net.tuned = {}
-        net.block, net.grid, net.persistent = 256, None, True
+        net.block, net.grid, net.persistent, net.steps_per_barrier = 256, None, True, None
         us, stats = _trial(net, steps, warmup)
+        chunks = isinstance(net.runtime, NetworkRuntime) and lookahead(net, net.runtime.desc) > 1
         _restore(net, snap)
         spikes_per_step = [s / steps for s in stats["spikes"]]
         pulls = pull_candidates(net, spikes_per_step, pull_factor)
         report["trials"].append({"block": 256, "grid": None, "persistent": True, "pull": 0, "us_per_step": us})
         mode_sets = [{}] + ([pulls] if pulls else [])
-        best = (us, 256, None, True, {})
+        best = (us, 256, None, True, {}, None)
         t0 = time.perf_counter()
         # pull sets also try 64-neuron tiles: a pulled row is walked by its tile's warps, so smaller tiles spread
         # the pulls over more SMs
-        cands = [(b, g, p, m) for m in mode_sets for b in (tuple(blocks) + ((64,) if m and 64 not in blocks else ()))
+        cands = [(b, g, p, m, None) for m in mode_sets for b in (tuple(blocks) + ((64,) if m and 64 not in blocks else ()))
                  for g in grids for p in persistent if p or g != RESIDENT]  # (per-step launches: not RESIDENT)
-        for block, grid, pers, modes in cands:
-            if (block, grid, pers, len(modes)) == (256, None, True, 0):
+        if chunks:  # in chunks on the library's blocks; with a barrier per step as the networks that have no choice
+            cands += [(None, None, True, {}, None)] + [(b, g, True, {}, 1) for b in blocks for g in grids]
+        for block, grid, pers, modes, spb in cands:
+            if (block, grid, pers, len(modes), spb) == (256, None, True, 0, None):
                 continue
-            net.block, net.grid, net.persistent, net.tuned = block, grid, pers, dict(modes)
+            net.block, net.grid, net.persistent, net.tuned, net.steps_per_barrier = block, grid, pers, dict(modes), spb
             try:
                 us, _ = _trial(net, steps, warmup)
             finally:
                 _restore(net, snap)
             report["trials"].append({"block": block, "grid": grid, "persistent": pers, "pull": len(modes),
-                                     "us_per_step": us})
+                                     "steps_per_barrier": spb, "us_per_step": us})
             if verbose:
                 print(report["trials"][-1], flush=True)
             if us < best[0]:
-                best = (us, block, grid, pers, dict(modes))
+                best = (us, block, grid, pers, dict(modes), spb)
         report["seconds"] = time.perf_counter() - t0
     except BaseException:
-        net.block, net.grid, net.persistent, net.tuned, net.window, net.record_steps = saved
+        (net.block, net.grid, net.persistent, net.tuned, net.window, net.record_steps, net.steps_per_barrier) = saved
         raise
     finally:
         net.close()
         net.step_count, net.t = 0, 0.0
         _restore(net, snap)
-    us, block, grid, pers, modes = best
-    net.block, net.grid, net.persistent, net.tuned = block, grid, pers, modes
+    us, block, grid, pers, modes, spb = best
+    net.block, net.grid, net.persistent, net.tuned, net.steps_per_barrier = block, grid, pers, modes, spb
     net.window, net.record_steps = saved[4], saved[5]
-    report["chosen"] = {"block": block, "grid": grid, "persistent": pers, "pull": len(modes), "us_per_step": us}
+    report["chosen"] = {"block": block, "grid": grid, "persistent": pers, "pull": len(modes),
+                        "steps_per_barrier": spb, "us_per_step": us}
     net.tune_report = report
     return report

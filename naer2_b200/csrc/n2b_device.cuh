@@ -1545,7 +1545,8 @@ __global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
 
 // ------------------------------------------------------------------ chunks of steps
 
-// Networks whose every link has a delay of at least K >= 2 steps (a single transmission delay of 1.5 ms is 15): what
+// Networks whose every link has a delay of at least K >= 2 steps (a single transmission delay of 1.5 ms is 15; which
+// of them run in chunks: chunk_steps, naer2b.cu): what
 // a step reads was sent at least K steps earlier, so K steps need no grid barrier between them. A block runs K
 // steps of its tile of TN neurons straight through (phase 1: slots read and cleared, update, spikes listed; no
 // barrier of any kind, one thread per neuron, its random draws made beforehand by the whole block), then delivers

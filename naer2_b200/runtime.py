@@ -36,6 +36,7 @@ from .topology import delay_steps, pack_links, pull_split_form, push_form
 
 MAX_SHIFT = 40
 MAX_LOOKAHEAD = 32  # steps without a grid barrier between them, at most (csrc/n2b_device.cuh, CHUNK_MAX)
+PAIR_ROW = 640  # links per neuron up to which they may be two (csrc/naer2b.cu)
 INLINE_POPS, INLINE_PUSH = 32, 64  # populations and push connections of a network that may (csrc/n2b_device.cuh)
 
 
@@ -228,7 +229,7 @@ def lookahead(net, desc: NetDesc) -> int:
     k = desc.lookahead if net.persistent and len(desc.pops) <= INLINE_POPS and len(desc.conns) <= INLINE_PUSH else 1
     if net.steps_per_barrier:
         return min(k, int(net.steps_per_barrier))
-    return k
+    return k if k != 2 or desc.n_links <= PAIR_ROW * sum(p.n for p in desc.pops) else 1
 
 
 class NetworkRuntime:
@@ -254,12 +255,13 @@ class NetworkRuntime:
         self.words, self.rasters = [], []
         self.record_rows = int(net.record_steps)
         self.rec_step0 = net.step_count
+        ahead = lookahead(net, desc)
         for k, (p, d) in enumerate(zip(pops, desc.pops)):
             n, words = d.n, (d.n + 31) // 32
             self.words.append(words)
             cp = self.cpop[k]
             # slots for the steps that run between two grid barriers as well (at most twice the depth)
-            depth = max(d.acc_depth, min(256, next_pow2(desc.max_in_delay[k] + desc.lookahead))) if d.acc_depth else 0
+            depth = max(d.acc_depth, min(256, next_pow2(desc.max_in_delay[k] + ahead))) if d.acc_depth else 0
             cp.model, cp.n, cp.acc_depth, cp.bit_depth = d.model, n, depth, d.bit_depth
             cp.shift, cp.ref_steps, cp.fire_threshold = d.shift, d.ref_steps, d.fire_threshold
             cp.ext_len, cp.seed, cp.ext_wfx = len(d.ext_table), d.seed, d.ext_wfx

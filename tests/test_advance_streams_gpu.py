@@ -1,14 +1,22 @@
 """n2b_advance orders a network's steps with the stream they are asked for on: after what is already there, before what
 comes next, on any stream and from several threads, each call whole."""
 
+import itertools
 import threading
 
 import pytest
 import torch
 
+from naer2_b200 import population
 from naer2_b200.networks import brunel
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _own_seeds(monkeypatch):
+    """Populations made here draw their default seeds from a count of their own."""
+    monkeypatch.setattr(population, "_SEEDS", itertools.count(1 << 20))
 
 
 def _net(delay):

@@ -39,6 +39,7 @@ PARAMS_BYTES = 32764  # a kernel's parameters at most (48 bytes per outgoing con
 # arrival.WINDOW_POPS populations or, over the distinct ones, arrival.WINDOW_INTAKES connections, and devices that hold
 # fewer blocks step by one launch per population.
 WINDOW_BLOCKS, WINDOW_SMS = 592, 148
+WINDOW_STEPS = 1024  # steps of one launch of it at most (8 ms at 7.5 us a step): other streams' launches come in between
 BARRIER_LIMIT_NS = 2_000_000_000  # how long a window's block waits at its grid barrier before it gives up
 _CACHE: dict = {}  # (source hash, device) -> n2b_jit_kernel handle, for the process's lifetime
 
@@ -476,7 +477,7 @@ class JitRuntime:
     # ------------------------------------------------------------------ stepping
 
     def advance(self, n_steps: int) -> None:
-        """Steps step_count .. step_count + n_steps - 1: one launch of the window kernel or, without it, per step one
+        """Steps step_count .. step_count + n_steps - 1: a launch of the window kernel per WINDOW_STEPS or, without it, per step one
         launch per population, in order, the whole window in one library call (n2b_jit_launch_window writes each
         launch's step and times)."""
         n_steps = int(n_steps)
@@ -495,14 +496,15 @@ class JitRuntime:
 
     def _advance_window(self, step: int, n_steps: int) -> None:
         lib, W = _lib.load(), self.window
-        W.step0, W.n_steps = step, n_steps
         W.grid.limit_ns = int(getattr(self.net, "barrier_limit_ns", 0) or BARRIER_LIMIT_NS)
         for k, g, i in self.window_slots:
             getattr(W, f"p{g}")[i] = self.params[k]
-        _lib.check(lib.n2b_jit_launch_cooperative(self.window_kernel, self.window_grid, arrival.THREADS,
-                                                  ctypes.addressof(W), ctypes.sizeof(W), self._s),
-                   "n2b_jit_launch_cooperative")
-        self.launches += 1
+        for first in range(0, n_steps, WINDOW_STEPS):
+            W.step0, W.n_steps = step + first, min(WINDOW_STEPS, n_steps - first)
+            _lib.check(lib.n2b_jit_launch_cooperative(self.window_kernel, self.window_grid, arrival.THREADS,
+                                                      ctypes.addressof(W), ctypes.sizeof(W), self._s),
+                       "n2b_jit_launch_cooperative")
+            self.launches += 1
 
     def _advance_steps(self, step: int, n_steps: int) -> None:
         k = len(self.kernels)

@@ -83,3 +83,32 @@ def test_a_batch_of_more_groups_than_a_grid_has_rows(cuda):
     want, want_ts = layer.run_forward(U[:, -16:].contiguous(), tape=False)
     assert torch.equal(m[-16:], want) and torch.equal(ts[-16:], want_ts)
     assert int((m != 0).sum()) > B // 4
+
+
+@pytest.mark.parametrize("smooth", [False, True])
+def test_captured_calls_replay(cuda, smooth):
+    """A plain forward, and a taped one with its backward, captured into graphs and replayed on other currents."""
+    B, T, H = 16, 60, 128
+    layer, us, g = _layer(cuda, H, B, T)
+    layer.smooth, layer._ws_key = smooth, None
+    dm = torch.randn(B, 5, generator=g, device=cuda)
+    want = []
+    for U in us:
+        plain = layer.run_forward(U, tape=False)
+        m, ts = layer.run_forward(U, tape=True)
+        want.append([*plain, m, ts, *layer.run_backward(U, dm, ts)])
+    torch.cuda.synchronize()
+    static = us[0].clone()
+    plain_graph, graph = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(plain_graph):
+        plain = layer.run_forward(static, tape=False)
+    with torch.cuda.graph(graph):
+        m, ts = layer.run_forward(static, tape=True)
+        grads = layer.run_backward(static, dm, ts)
+    for U, w in zip(us, want):
+        static.copy_(U)
+        plain_graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip([*plain, m, ts, *grads], w):
+            assert torch.equal(a, b)

@@ -61,3 +61,26 @@ def test_captured_steps_replay(cuda, monkeypatch, replays):
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
     assert sum(int(np.unpackbits(w.view(np.uint8)).sum()) for w in got[:2]) > 100
+
+
+def test_long_runs_are_several_launches(cuda, monkeypatch):
+    def run(net_steps):
+        population._SEEDS = itertools.count(1 << 20)
+        src, tgt = Pacemaker(period=7) * 50, TraceLIF(theta=1.2) * 60
+        src.seed, tgt.seed = 1, 2
+        c = src >> PairSTDP() @ fixed_indegree(12, seed=10) >> tgt
+        c.weight, c.delay = 0.2, 0.3
+        net = src.network
+        net.resolution = 0.1
+        for n in net_steps:
+            net.run_steps(n)
+        rt = net.runtime
+        return [t.cpu().numpy() for p in net.populations for _, t in sorted(p._state.items())] + [
+            rt.edge_state(c, "weight").cpu().numpy(), np.array(rt.counters()["events"])], rt
+
+    got, rt = run([2100])
+    assert rt.window is not None and rt.launches == 3
+    want, _ = run([700] * 3)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
+    assert int(want[-1]) > 1000

@@ -130,8 +130,8 @@ typedef struct n2b_options {
     int32_t persistent; /* 1: a window of steps is one cooperative launch, steps separated by a grid
                            barrier; 0: one launch per step */
     int32_t chunk;   /* persistent push-only networks whose every delay allows it: steps without a grid barrier
-                        between them at most (0: the library's choice, 1: a barrier per step) */
-    int32_t chunk_block; /* ... and the neurons per block then: 32, 64, 128 or 256 (0: the library's choice) */
+                        between them at most (0: the library's choice, 1: a barrier per step), and above bit 16
+                        the neurons per block then: 32, 64, 128 or 256 (0: the library's choice) */
     int64_t barrier_limit_ns; /* persistent windows: the longest a block waits at a grid barrier before the
                                  window stops with N2B_ERR_BARRIER (0: 2 s). Tests set a few ns: the wait
                                  then gives up at once although every block arrives, without a hang */

@@ -38,7 +38,7 @@ class Connection(ctypes.Structure):
 
 class Options(ctypes.Structure):
     _fields_ = [("block", ctypes.c_int32), ("device", ctypes.c_int32), ("grid", ctypes.c_int32),
-                ("persistent", ctypes.c_int32), ("chunk", ctypes.c_int32), ("chunk_block", ctypes.c_int32),
+                ("persistent", ctypes.c_int32), ("chunk", ctypes.c_int32),
                 ("barrier_limit_ns", ctypes.c_int64)]
 
 

@@ -67,6 +67,8 @@ struct Layout {
     int32_t n_push, n_pull, n_tiles, item_cap;
 };
 
+int32_t chunk_block(const n2b_options *opt) { return opt ? opt->chunk >> 16 : 0; }
+
 int32_t block_of(const n2b_options *opt) {
     int32_t b = opt && opt->block ? opt->block : 128;
     return b;
@@ -112,9 +114,9 @@ int validate(const n2b_population *pops, int32_t n_pops, const n2b_connection *c
     if (block != 64 && block != 128 && block != 256) return fail(N2B_EINVAL, "block must be 64, 128 or 256");
     if (opt && opt->barrier_limit_ns < 0) return fail(N2B_EINVAL, "barrier_limit_ns < 0");
     if (opt && opt->chunk < 0) return fail(N2B_EINVAL, "chunk < 0");
-    if (opt && opt->chunk_block != 0 && opt->chunk_block != 32 && opt->chunk_block != 64 && opt->chunk_block != 128 &&
-        opt->chunk_block != 256)
-        return fail(N2B_EINVAL, "chunk_block must be 0, 32, 64, 128 or 256");
+    const int32_t tn = chunk_block(opt);
+    if (tn != 0 && tn != 32 && tn != 64 && tn != 128 && tn != 256)
+        return fail(N2B_EINVAL, "chunk: the block must be 0, 32, 64, 128 or 256");
     for (int32_t p = 0; p < n_pops; ++p) {
         const n2b_population &P = pops[p];
         const std::string at = "population " + std::to_string(p) + ": ";
@@ -486,7 +488,7 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
                      (int32_t)pull.size() <= n2b::INLINE_PULL;
     int32_t chunk = 0;
     if (persistent && inl && pull.empty() && L.n_tiles > 0) {
-        rc = chunk_steps(pops, n_pops, push, push_tgt, ws, L, s, opt ? opt->chunk : 0, &chunk);
+        rc = chunk_steps(pops, n_pops, push, push_tgt, ws, L, s, opt ? opt->chunk & 0xFFFF : 0, &chunk);
         if (rc) return rc;
     }
     if (n_pops) N2B_CUDA(cudaMemcpyAsync(ws + L.pops, pd.data(), sizeof(n2b::PopDev) * n_pops, cudaMemcpyHostToDevice, s));
@@ -551,7 +553,7 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
         for (chunk_tn = 32;; chunk_tn *= 2) {
             chunk_tiles = 0;
             for (int32_t p = 0; p < n_pops; ++p) chunk_tiles += (pops[p].n + chunk_tn - 1) / chunk_tn;
-            if (opt && opt->chunk_block ? chunk_tn == opt->chunk_block : (chunk_tiles <= 2 * sms || chunk_tn == 256)) break;
+            if (chunk_block(opt) ? chunk_tn == chunk_block(opt) : (chunk_tiles <= 2 * sms || chunk_tn == 256)) break;
         }
         chunk = std::min(chunk, n2b::chunk_most(chunk_tn));
         int per_sm = 0;

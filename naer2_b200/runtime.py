@@ -303,8 +303,8 @@ class NetworkRuntime:
         block = net.block or min([p.group_size for p in pops] + [256])
         block = 64 if block <= 64 else 128 if block <= 128 else 256
         self.opt = _lib.Options(block=block, device=dev.index if dev.index is not None else 0, grid=int(net.grid or 0),
-                                persistent=int(bool(net.persistent)), chunk=int(net.steps_per_barrier or 0),
-                                chunk_block=block if net.block else 0,
+                                persistent=int(bool(net.persistent)),
+                                chunk=min(int(net.steps_per_barrier or 0), 0xFFFF) | (block << 16 if net.block else 0),
                                 barrier_limit_ns=int(getattr(net, "barrier_limit_ns", 0) or 0))
         nbytes = ctypes.c_size_t()
         _lib.check(lib.n2b_workspace_bytes(self.cpop, len(pops), self.cconn, len(desc.conns), ctypes.byref(self.opt),

@@ -1,4 +1,4 @@
-"""n2b_options.chunk and chunk_block are checked on the host, by the size query already."""
+"""n2b_options.chunk, its steps and its block, is checked on the host, by the size query already."""
 
 import ctypes
 
@@ -7,8 +7,8 @@ import pytest
 from naer2_b200 import _lib
 
 
-@pytest.mark.parametrize("kw, msg", [(dict(chunk=-1), "chunk < 0"), (dict(chunk_block=48), "chunk_block"),
-                                     (dict(chunk_block=-32), "chunk_block"), (dict(chunk=7, chunk_block=64), None)])
+@pytest.mark.parametrize("kw, msg", [(dict(chunk=-1), "chunk < 0"), (dict(chunk=48 << 16), "block"),
+                                     (dict(chunk=512 << 16 | 3), "block"), (dict(chunk=7 | 64 << 16), None)])
 def test_chunk_options(kw, msg):
     lib = _lib.load()
     p = _lib.Population()

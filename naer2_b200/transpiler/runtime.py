@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ast
 import ctypes
+import functools
 import hashlib
 import warnings
 
@@ -32,6 +33,7 @@ BLOCK = 128  # exact-time intake without arrival bits: one thread per neuron
 # neurons of 1,250 links and 32 slots the bits are 64 MB, the rows 78 MB.
 ARRIVAL_BYTES = 32 << 30
 BUILD_BYTES = 72
+SMALL_BYTES = 64 << 20  # less than this is taken without asking the device (0.7 ms)
 PACKED_BITS = 1 << 24  # bits of a slot whose places leave a link word's top 8 bits to the delay
 PARAMS_BYTES = 32764  # a kernel's parameters at most (48 bytes per outgoing connection, 40 to 64 per incoming one)
 # A window kernel holds every block of the network at once: 592 blocks (18,944 neurons) are four per SM, 64 registers
@@ -161,14 +163,15 @@ def arrivals_need(plan: dict) -> int:
     return sum(t for t, _ in sizes) + max((b for _, b in sizes), default=0)
 
 
-def plan_of(net) -> dict:
+def plan_of(net, intake: str | None = None) -> dict:
     """The transpiled form of a network, everything its step kernels need and nothing of its Python model classes:
     per population its CUDA source, the Params fields with the values of the scalar ones, its state attributes
     (name -> "float" / "int" / "bool"), size, seed and spike-ring depth, and (networks whose intake reads arrival
     bits) its outgoing connections; per incoming connection (in order) its
     source population, pull CSR (int32 ptr, uint32 link words) and per-link edge arrays (pull order) with the
     pull permutation. JitRuntime builds from it; save_plan / load_plan keep it in a file, so that a network can
-    be transpiled where its model classes are and stepped where only the plan is."""
+    be transpiled where its model classes are and stepped where only the plan is. A plan of arrival bits carries the
+    scanning intake's sources along ("scan"), but with intake "arrivals"; "scan" is a plan of the latter alone."""
     dev = net.device if net.device is not None else torch.device("cpu")
     dt = float(net.resolution)
     pops = list(net.populations)
@@ -192,7 +195,7 @@ def plan_of(net) -> dict:
         for ci, c in enumerate(conns):
             outs[index[id(c._source)]].append([k, ci])
     arrivals = sum(arrival_bytes(len(p.shape), len(c.fabric.topology), depth[index[id(c._source)]])
-                   for p, conns in zip(pops, incoming_of) for c in conns) <= ARRIVAL_BYTES
+                   for p, conns in zip(pops, incoming_of) for c in conns) <= ARRIVAL_BYTES and intake != "scan"
     total = sum(arrival.blocks_of(len(p.shape)) for p in pops)
     per_sm = -(-total // WINDOW_SMS)
     ahead = arrival.AHEAD_FEW if 2 * WINDOW_SMS < total <= WINDOW_BLOCKS else arrival.AHEAD
@@ -227,9 +230,10 @@ def plan_of(net) -> dict:
             return incoming, {"update": (node.update.ast, hook_context(p, node.update, site_base=site)),
                               "send": (node.send.ast, hook_context(p, node.send, site_base=site + 32))}
 
-        incoming, hooks = lowered()
-        src, fields = build_source(name, dict(p.dynamic_attrs), hooks, incoming, exact=exact, n=len(p.shape))
-        scanning = {"source": src, "fields": [(f, ctype) for f, ctype, _ in fields]}
+        if not arrivals or intake is None:
+            incoming, hooks = lowered()
+            src, fields = build_source(name, dict(p.dynamic_attrs), hooks, incoming, exact=exact, n=len(p.shape))
+            scanning = {"source": src, "fields": [(f, ctype) for f, ctype, _ in fields]}
         if arrivals:
             incoming, hooks = lowered()
             src, fields, body = arrival.build(name, dict(p.dynamic_attrs), hooks, incoming, len(outs[k]), exact, ahead)
@@ -240,7 +244,9 @@ def plan_of(net) -> dict:
                  "seed": int(p.seed) & 0xFFFFFFFFFFFFFFFF, "source": src,
                  "fields": [(name, ctype) for name, ctype, _ in fields], "attrs": attrs, "conns": []}
         if arrivals:
-            entry["outs"], entry["scan"] = outs[k], scanning
+            entry["outs"] = outs[k]
+            if intake is None:
+                entry["scan"] = scanning
         for inc in incoming:
             c = inc["conn"]
             topo = c.fabric.topology
@@ -314,7 +320,8 @@ def load_plan(path) -> dict:
 _CTYPES = {"long long": ctypes.c_int64, "float": ctypes.c_float, "int": ctypes.c_int32, "u32": ctypes.c_uint32}
 
 
-def _params_struct(fields: list):
+@functools.lru_cache(maxsize=256)
+def _params_struct(fields: tuple):
     """The ctypes Params structure of a plan's fields (pointers as void *)."""
     def ctype(ct):
         if ct.startswith("N2Out["):
@@ -324,10 +331,13 @@ def _params_struct(fields: list):
     return params_type([(name, ct, ctype(ct)) for name, ct in fields])
 
 
-def _kinds(window: dict, types: list) -> list:
-    """arrival.window_type's kinds of a plan's window, `types` the populations' Params."""
-    first = np.cumsum([0] + window["counts"])
-    return [(types[window["order"][at]], count) for at, count in zip(first, window["counts"])]
+def _window_type(window: dict, types: list):
+    """The parameter block of a plan's window kernel, `types` the populations' Params."""
+    kinds, at = [], 0
+    for count in window["counts"]:
+        kinds.append((types[window["order"][at]], count))
+        at += count
+    return arrival.window_type(tuple(kinds))
 
 
 class JitRuntime:
@@ -338,13 +348,17 @@ class JitRuntime:
         self.net = net
         dev = self.device = net.device
         dindex = dev.index if dev.index is not None else 0
+        scanning = None  # the plan's other form (plans of an older version have none)
         if plan is None:
-            plan = plan_of(net)
-        # arrival bits where they, and making them, take half of what is free on the device at most (plans of an older
-        # version have no other form)
-        if any("scan" in p for p in plan["pops"]) and arrivals_need(plan) > _lib.free_bytes(dev) // 2:
-            plan = scan_form(plan)
-        plan, window_kernel, self.kernels = self._compiled(plan, dindex)
+            plan, scanning = plan_of(net, "arrivals"), lambda: plan_of(net, "scan")
+        elif any("scan" in p for p in plan["pops"]):
+            scanning = functools.partial(scan_form, plan)
+        # arrival bits where they, and making them, take half of what is free on the device at most
+        if scanning and any("outs" in p for p in plan["pops"]):
+            need = arrivals_need(plan)
+            if need > SMALL_BYTES and need > _lib.free_bytes(dev) // 2:
+                plan, scanning = scanning(), None
+        plan, window_kernel, self.kernels = self._compiled(plan, scanning, dindex)
         self.plan = plan
         dt = self.dt = float(plan["dt"])
         pops = self.pops = list(net.populations)
@@ -364,13 +378,12 @@ class JitRuntime:
         self.raster_offs = [torch.zeros(max(1, self.record_rows) * max(1, p["n"]), dtype=torch.float32,
                                         device=dev) for p in plan["pops"]]
         self.params, self.sources = [], []
-        types: dict = {}  # Params fields -> their structure
         forms = []  # per population, its incoming connections' arrival forms
         self.edge_arrays = {}  # (connection id, edge name) -> (per-link values in pull order, pull permutation)
         tdtype = {"bool": torch.bool, "int": torch.int32, "float": torch.float32}
         for k, (p, pp) in enumerate(zip(pops, plan["pops"])):
             self.sources.append(pp["source"])
-            P = types.setdefault(tuple(pp["fields"]), _params_struct(pp["fields"]))()
+            P = _params_struct(tuple(pp["fields"]))()
             P.n, P.words, P.bit_mask = pp["n"], words[k], depth[k] - 1
             P.seed_lo, P.seed_hi = pp["seed"] & 0xFFFFFFFF, (pp["seed"] >> 32) & 0xFFFFFFFF
             for a, ty in pp["attrs"].items():
@@ -433,15 +446,14 @@ class JitRuntime:
         self._s = ctypes.c_void_p(self.stream.cuda_stream)
         self.launches = 0
 
-    def _compiled(self, plan: dict, dindex: int) -> tuple:
+    def _compiled(self, plan: dict, scanning, dindex: int) -> tuple:
         """(the plan's form to run, its window kernel or None, else its step kernels). The window kernel where it
         compiles, its parameters fit and the device holds all its blocks at once; else a kernel per population, of the
         scanning intake where those of the arrival bits do not compile or their parameters do not fit."""
-        types = [_params_struct(p["fields"]) for p in plan["pops"]]
-        scans = any("scan" in p for p in plan["pops"])
-        if scans and any(ctypes.sizeof(t) > PARAMS_BYTES for t in types):
-            return self._compiled(scan_form(plan), dindex)
-        if "window" in plan and ctypes.sizeof(arrival.window_type(_kinds(plan["window"], types))) <= arrival.WINDOW_PARAMS:
+        types = [_params_struct(tuple(p["fields"])) for p in plan["pops"]]
+        if scanning and any(ctypes.sizeof(t) > PARAMS_BYTES for t in types):
+            return self._compiled(scanning(), None, dindex)
+        if "window" in plan and ctypes.sizeof(_window_type(plan["window"], types)) <= arrival.WINDOW_PARAMS:
             try:
                 kern, blocks = compile_source(plan["window"]["source"], dindex, b"n2b_user_window"), ctypes.c_int32()
                 _lib.check(_lib.load().n2b_jit_resident_blocks(kern, arrival.THREADS, ctypes.byref(blocks)),
@@ -453,14 +465,14 @@ class JitRuntime:
         try:
             return plan, None, [compile_source(p["source"], dindex) for p in plan["pops"]]
         except RuntimeError as e:
-            if not scans:
+            if not scanning or not any("outs" in p for p in plan["pops"]):
                 raise
             warnings.warn(f"no arrival bits ({e}): every link's source is looked up", stacklevel=4)
-            return self._compiled(scan_form(plan), dindex)
+            return self._compiled(scanning(), None, dindex)
 
     def _window(self, plan: dict, kern: ctypes.c_void_p) -> None:
         """The window kernel's parameter block."""
-        self.window_kernel, self.window = kern, arrival.window_type(_kinds(plan, [type(P) for P in self.params]))()
+        self.window_kernel, self.window = kern, _window_type(plan, [type(P) for P in self.params])()
         self.window.dt = self.dt
         self.window.grid.bar = self.bar.data_ptr()
         self.window_slots = []  # per population in the block's order: (its index, its kind, its place among them)

@@ -62,6 +62,7 @@ def test_little_free_memory_scans(cuda, monkeypatch, tmp_path, make, through_fil
     want, rt = run()
     assert rt.window is not None
     need = arrivals_need(rt.plan)
+    monkeypatch.setattr(jit_runtime, "SMALL_BYTES", 0)
     monkeypatch.setattr(_lib, "free_bytes", lambda device: 2 * need)
     _, rt = run()
     assert rt.window is not None

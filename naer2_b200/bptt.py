@@ -25,6 +25,7 @@ import torch
 
 from . import _lib
 
+SMALL_TAPE = 1 << 30  # more than this is taken by the device's free memory (asking for it costs 0.7 ms)
 MAX_DELAY = 5
 
 
@@ -276,7 +277,7 @@ class RecurrentLIF(torch.nn.Module):
         """The layer's workspace at d's sizes; sets d.segments to the form that it holds."""
         key = (d.batch, d.steps, d.checkpoint, d.smooth, self.segments)
         if self._ws_key != key:
-            self._ws = None
+            self._ws = self._ws_key = None
             dev, bytes_of = self.w_in.device, []
             for segments in (0, 1):
                 d.segments, n = segments, ctypes.c_size_t()
@@ -286,7 +287,8 @@ class RecurrentLIF(torch.nn.Module):
             forms = [int(self.segments)] if self.segments is not None else [0, 1]
             if len(forms) > 1 and not torch.cuda.is_current_stream_capturing():
                 # the derivatives of every step take half of what is free at most: the rest is the program's
-                if bytes_of[0] - bytes_of[1] > _lib.free_bytes(dev) // 2:
+                more = bytes_of[0] - bytes_of[1]
+                if more > SMALL_TAPE and more > _lib.free_bytes(dev) // 2:
                     forms = [1]
             for segments in forms:
                 try:

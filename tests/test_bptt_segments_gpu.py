@@ -8,6 +8,7 @@ reference it is held to the tolerances of test_bptt_gpu.py."""
 import pytest
 import torch
 
+from naer2_b200 import bptt
 from naer2_b200.bptt import RecurrentLIF
 from naer2_b200.networks import bptt_task
 from test_bptt_gpu import kernel_grads, make, reference, rel
@@ -105,8 +106,29 @@ def test_little_free_memory_takes_the_segments(cuda, monkeypatch):
     _run(layer, x, y)
     assert layer._ws.numel() > small
     layer._ws = layer._ws_key = None
+    monkeypatch.setattr(bptt, "SMALL_TAPE", 0)
     monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev=None: (0, 1 << 37))
     monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev=None: torch.cuda.memory_allocated(dev) + (1 << 16))
+    got = _run(layer, x, y)
+    assert layer._ws.numel() == small
+    for a, b in zip(got[0] + got[1], want[0] + want[1]):
+        assert torch.equal(a, b)
+
+
+def test_no_memory_for_the_whole_tape_takes_the_segments(cuda, monkeypatch):
+    layer, x, y = make(cuda, B=16, T=60, K=7, seed=4)
+    layer.segments = True
+    want = _run(layer, x, y)
+    small = layer._ws.numel()
+    layer.segments, layer._ws, layer._ws_key = None, None, None
+    empty = torch.empty
+
+    def refuse(*size, **kw):
+        if kw.get("dtype") is torch.uint8 and size[0] > small:
+            raise torch.cuda.OutOfMemoryError("refused")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", refuse)
     got = _run(layer, x, y)
     assert layer._ws.numel() == small
     for a, b in zip(got[0] + got[1], want[0] + want[1]):

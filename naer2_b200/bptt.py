@@ -253,6 +253,7 @@ class RecurrentLIF(torch.nn.Module):
         # steps, recomputed segment by segment (True; slower, smaller), or (None) the first where memory allows
         self.segments: bool | None = None
         self._ws_segments = 0
+        self._plain_bytes = (None, 0)  # a plain forward's scratch, by its sizes
         self._plain = None  # the last call was a plain forward: its (batch, steps) and error words
         self.tape_id = 0
         # polls before a wait of the per-step exchange (forward or backward) gives up (0: the library's default, about a
@@ -336,13 +337,18 @@ class RecurrentLIF(torch.nn.Module):
         s = ctypes.c_void_p(torch.cuda.current_stream(U.device).cuda_stream)
         if not tape:
             # scratch of the call's own, on its stream: calls of several streams or threads, and a backward, may overlap
-            n = ctypes.c_size_t()
-            _lib.check(lib.n2b_bptt_infer_bytes(ctypes.byref(d), ctypes.byref(n)), "n2b_bptt_infer_bytes")
-            scratch = torch.empty(n.value, dtype=torch.uint8, device=U.device)
+            key = (B, T, d.smooth, d.in_cta_max)
+            known, nbytes = self._plain_bytes
+            if known != key:
+                n = ctypes.c_size_t()
+                _lib.check(lib.n2b_bptt_infer_bytes(ctypes.byref(d), ctypes.byref(n)), "n2b_bptt_infer_bytes")
+                nbytes = n.value
+                self._plain_bytes = (key, nbytes)
+            scratch = torch.empty(nbytes, dtype=torch.uint8, device=U.device) if nbytes else None
             err = torch.empty(_lib.BPTT_ERR_WORDS, dtype=torch.int32, device=U.device)
             _lib.check(lib.n2b_bptt_infer(ctypes.byref(d), U.data_ptr(), self.w_rec.data_ptr(), self.w_out.data_ptr(),
-                                          m.data_ptr(), ts.data_ptr(), err.data_ptr(), scratch.data_ptr(), n.value, s),
-                       "n2b_bptt_infer")
+                                          m.data_ptr(), ts.data_ptr(), err.data_ptr(),
+                                          scratch.data_ptr() if nbytes else None, nbytes, s), "n2b_bptt_infer")
             self._plain = ((B, T), err)
             return m, ts
         ws = self.workspace(d)

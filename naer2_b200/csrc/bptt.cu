@@ -247,7 +247,8 @@ __device__ __forceinline__ float lif_step(const Args &a, float &V, float u, floa
 
 // ------------------------------------------------------------------------------------------------ forward
 
-template <bool SMOOTH>
+// DERIV: it keeps the surrogate derivatives of every step (a.g_all; a kernel of its own: 4% of the plain forward).
+template <bool SMOOTH, bool DERIV>
 __global__ void __launch_bounds__(512) fwd_kernel(const __grid_constant__ Args a, int in_cta_max) {
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(512) fwd_kernel(const __grid_constant__ Args a
     const size_t bq = (size_t)q * NS + SPT * sub;  // this thread's first sample
 
     for (int t = 0; t < a.T; ++t) {
-        if (a.tape && t % a.K == 0 && nt) {
+        if (!DERIV && a.tape && t % a.K == 0 && nt) {
             a.v_ckpt[((size_t)(t / a.K) * B + bq) * H + post] = V0;
             a.v_ckpt[((size_t)(t / a.K) * B + bq + 1) * H + post] = V1;
         }
@@ -311,8 +312,14 @@ __global__ void __launch_bounds__(512) fwd_kernel(const __grid_constant__ Args a
         if (nt) {
             const float u0 = __ldg(a.U + ((size_t)t * B + bq) * H + post);
             const float u1 = __ldg(a.U + ((size_t)t * B + bq + 1) * H + post);
+            float vp1;
             s0 = lif_step<SMOOTH>(a, V0, u0, r0, vp);
-            s1 = lif_step<SMOOTH>(a, V1, u1, r1, vp);
+            s1 = lif_step<SMOOTH>(a, V1, u1, r1, vp1);
+            if constexpr (DERIV) {
+                float *g = a.g_all + ((size_t)t * B + bq) * H + post;
+                __stcs(g, surrogate(__fadd_rn(vp, -a.theta), a.slope));
+                __stcs(g + H, surrogate(__fadd_rn(vp1, -a.theta), a.slope));
+            }
         }
         const int slot = t % RING;
         if constexpr (SMOOTH) {
@@ -1343,13 +1350,26 @@ int check_desc(const n2b_bptt_desc *d) {
     return N2B_OK;
 }
 
-// The forward runs fwd_group_kernel: its rows fit shared memory.
-bool scans(const n2b_bptt_desc *d) {
+// A spiking layer whose incoming rows fit a CTA's shared memory.
+bool rows_fit(const n2b_bptt_desc *d) {
     return !d->smooth && scan_smem(d->hidden, d->hidden / CL, d->in_cta_max).total <= SMEM_MAX - 1024;
 }
 
+// The forward runs fwd_group_kernel, else fwd_kernel (the same results). Its launches and set-up cost 13 us more, and its
+// CTAs lose against fwd_kernel's clusters where several of them share an SM. Measured, fwd_kernel over it, plain forwards
+// at 5% / 10% of the neurons spiking a step:
+//   steps: 5 0.3-0.7, 12 0.7-1.2, 16 0.9-1.3 / 0.7-1.15, 24 1.04-1.55 / 1.0-1.36, 50 1.2-1.9, 300 1.3-2.1;
+//   a CTA per SM (18 groups of 8 samples) 1.04-2.1 at 1,024 neurons, 19 groups 0.89-1.09 / 0.80-0.96; at 512 neurons 16
+//   groups 1.33-1.88, 19 groups 1.02-1.26 / 0.98-1.16, 64 groups 0.66-0.75; at 256 neurons 32 groups 1.06-1.34 / 1.01-1.28,
+//   64 groups 0.78-1.01; at 64 neurons 64 groups 1.04-1.33.
+constexpr int SMS = 148, GROUP_STEPS = 24, GROUP_THREADS = 512;  // (threads of its CTAs per SM, where there are several)
+bool scans(const n2b_bptt_desc *d) {
+    const int64_t ctas = (int64_t)(d->batch / NS) * CL;
+    return rows_fit(d) && d->steps >= GROUP_STEPS && (ctas <= SMS || ctas * d->hidden <= (int64_t)GROUP_THREADS * SMS);
+}
+
 bool full_tape(const n2b_bptt_desc *d) {
-    return !d->segments && scans(d) && sizeof(float) * (size_t)d->steps * d->batch * d->hidden <= FULL_TAPE_BYTES;
+    return !d->segments && rows_fit(d) && sizeof(float) * (size_t)d->steps * d->batch * d->hidden <= FULL_TAPE_BYTES;
 }
 
 WsLayout ws_layout(const n2b_bptt_desc *d) {
@@ -1359,7 +1379,7 @@ WsLayout ws_layout(const n2b_bptt_desc *d) {
     size_t o = 0;
     L.spikes = o; o = a256(o + (d->smooth ? sizeof(float) * T * NC * H * NS : T * NC * H));
     L.xw = o; o = a256(o + (scans(d) ? sizeof(unsigned long long) * NC * XSLOTS * (H / 4) : 0));
-    L.tot = o; o = a256(o + (scans(d) ? sizeof(float) * T * B * R : 0));
+    L.tot = o; o = a256(o + (scans(d) || full_tape(d) ? sizeof(float) * T * B * R : 0));
     L.vck = o; o = a256(o + (full_tape(d) ? 0 : sizeof(float) * nseg * B * H));
     // every step, or two segments: one recomputed, one run back
     L.gseg = o; o = a256(o + sizeof(float) * (full_tape(d) ? T : 2 * K) * B * H);
@@ -1564,8 +1584,9 @@ int run_forward(const n2b_bptt_desc *d, Args a, bool group, cudaStream_t s) {
     FwdSmem S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, true, d->in_cta_max);
     a.csr_smem = S.total <= 200 * 1024;
     if (!a.csr_smem) S = fwd_smem(d->hidden, d->hidden / CL, d->readouts, smooth, false, 0);
-    return smooth ? launch_cluster(fwd_kernel<true>, grid, threads, S.total, s, a, d->in_cta_max)
-                  : launch_cluster(fwd_kernel<false>, grid, threads, S.total, s, a, d->in_cta_max);
+    return smooth              ? launch_cluster(fwd_kernel<true, false>, grid, threads, S.total, s, a, d->in_cta_max)
+           : a.tape && a.g_all ? launch_cluster(fwd_kernel<false, true>, grid, threads, S.total, s, a, d->in_cta_max)
+                               : launch_cluster(fwd_kernel<false, false>, grid, threads, S.total, s, a, d->in_cta_max);
 }
 
 }  // namespace

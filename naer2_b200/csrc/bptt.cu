@@ -1173,22 +1173,22 @@ __global__ void __launch_bounds__(256) readout_dV_kernel(const __grid_constant__
     }
 }
 
-// FULL: dw_out's partial sums, chunk c of NC of the steps: dwo_p[c][i][r] = sum over the chunk's spikes of neuron i of
-// o[t][b][r]. A warp per four neurons (one word of spikes per step and group), a lane per readout.
+// FULL: dw_out's partial sums, chunk c of NC of the (step, group) pairs: dwo_p[c][i][r] = sum over the chunk's spikes of
+// neuron i of o[t][b][r]. A warp per four neurons (one word of spikes per step and group), a lane per readout. T pairs to
+// a chunk: chunks of whole steps left all but T of the NC of them empty in short sequences of large batches.
 __global__ void __launch_bounds__(256) dwo_kernel(const __grid_constant__ Args a) {
     const int lane = threadIdx.x & 31, word = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, c = blockIdx.y;
     if (word >= a.H / 4) return;
-    const int t0 = (int)((long long)a.T * c / a.NC), t1 = (int)((long long)a.T * (c + 1) / a.NC);
+    const size_t p0 = (size_t)c * a.T;  // the chunk's first pair
     const uint32_t *src = reinterpret_cast<const uint32_t *>(a.s_bits) + word;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const int n = (t1 - t0) * a.NC;  // (step, group) pairs
-    for (int k0 = 0; k0 < n; k0 += 32) {
+    for (int k0 = 0; k0 < a.T; k0 += 32) {
         // 32 pairs' words, a lane each; then those with a spike, in order
-        const uint32_t mine = k0 + lane < n ? src[((size_t)t0 * a.NC + k0 + lane) * (a.H / 4)] : 0u;
+        const uint32_t mine = k0 + lane < a.T ? src[(p0 + k0 + lane) * (a.H / 4)] : 0u;
         for (uint32_t some = __ballot_sync(FULL, mine != 0u); some; some &= some - 1) {
             const int k = k0 + __ffs(some) - 1;
             const uint32_t w = __shfl_sync(FULL, mine, k - k0);
-            const float *o = a.o_all + ((size_t)t0 * a.NC + k) * NS * a.R + lane;  // (t, q): samples 8q ..
+            const float *o = a.o_all + (p0 + k) * NS * a.R + lane;  // (t, q): samples 8q ..
             for (uint32_t m = w; m; m &= m - 1) {
                 const int bit = __ffs(m) - 1;
                 const float v = lane < a.R ? __ldg(o + (bit & 7) * a.R) : 0.f;
@@ -1676,7 +1676,14 @@ int n2b_bptt_backward(const n2b_bptt_desc *d, const float *u, const float *w_rec
     const bool smooth = d->smooth != 0;
     const int NC = d->batch / NS, threads = threads_of(d, NB);
     const bool full = full_tape(d);  // the adjoint of all steps in one launch, nothing to recompute
-    const BwdSmem S = bwd_smem(d->hidden, d->hidden / CL, d->readouts, d->out_cta_max, full);
+    BwdSmem S = bwd_smem(d->hidden, d->hidden / CL, d->readouts, d->out_cta_max, full);
+    // Other kernels run beside the adjoint (dw_out's, the next segment's recomputation). Where several of its CTAs fit an
+    // SM it would be placed around theirs, two and more to one SM and none to the next, at the pace of the fullest: it
+    // asks for so much shared memory that an SM holds just its share. 50 steps of 128 samples: 256 neurons 403 -> 285 us,
+    // 512 neurons 505 -> 375.
+    const int share = (NC * CL + SMS - 1) / SMS;
+    const bool spread = full && d->hidden <= 512 && share <= 3;
+    if (spread) S.total = std::max(S.total, SMEM_MAX / (share + 1) + 2048);
     const int K = full ? d->steps : d->checkpoint, nseg = full ? 1 : a.nseg;
     const int rthreads = d->hidden % 64 == 0 ? 256 : 128;  // whole neurons of NT threads; hidden % 32 == 0
     const size_t rsmem = smooth ? 0 : (size_t)16 * d->hidden;  // the staged spike rows
@@ -1721,8 +1728,17 @@ int n2b_bptt_backward(const n2b_bptt_desc *d, const float *u, const float *w_rec
         B_CUDA(cudaGetLastError());
         B_CUDA(cudaEventRecord(rec[0], st.hi));
         B_CUDA(cudaStreamWaitEvent(st.lo, rec[0], 0));
-        dwo_kernel<<<dim3((unsigned)((d->hidden / 4 + 7) / 8), (unsigned)NC), 256, 0, st.lo>>>(a);
-        B_CUDA(cudaGetLastError());
+        // (with the adjoint's partition of shared memory and L1: an SM that runs it takes the adjoint's CTA at once)
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)((d->hidden / 4 + 7) / 8), (unsigned)NC);
+        cfg.blockDim = dim3(256);
+        cfg.stream = st.lo;
+        cudaLaunchAttribute carveout[1];
+        carveout[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        carveout[0].val.sharedMemCarveout = 100;
+        cfg.attrs = carveout;
+        cfg.numAttrs = spread ? 1 : 0;
+        B_CUDA(cudaLaunchKernelEx(&cfg, dwo_kernel, a));
         B_CUDA(cudaEventRecord(rec[1], st.lo));
         const int vthreads = std::min(256, d->hidden / 2);
         const dim3 vgrid((unsigned)(((int64_t)d->steps * d->batch + DV_ROWS - 1) / DV_ROWS),

@@ -268,16 +268,8 @@ int coresident_blocks(int32_t block, bool inl, int kind, int device, size_t dyn,
 }
 
 // How many steps of a network of push connections need no grid barrier between them: the smallest delay of its
-// links, as far as every population's slots hold that many steps past its largest incoming delay; below 2, 0 (a
-// barrier per step, the deliveries of delay >= 2 spread over the grid). Two steps are worth it for short rows alone: a
-// spike's links are its block's to deliver in a chunk, and a chunk of two steps has few spikes to share its latencies.
-// Measured against a barrier per step, us per step of networks of model A, 1,000 to 500,000 neurons: three steps are
-// 1.09 to 2.01 times as fast with rows of 100 to 1,250 links, 15 steps 1.8 to 4.1 times; two steps 1.05 to 1.7 times
-// with rows of up to 625 links, 0.90 to 1.1 times with 1,250 (12,500 neurons firing densely 5.56 against 5.83, 75,000
-// neurons 7.8 against 8.6, 100,000 8.5 against 9.3). Tiles past the resident blocks change nothing: 150,000 neurons 13.1
-// against 10.4 with three steps, 500,000 27.2 against 18.8.
-// Reads the links once; the room of the push table, not yet written, holds the ranges.
-constexpr int64_t PAIR_ROW = 640;  // links per neuron up to which a chunk may be of two steps
+// links, as far as every population's slots hold that many steps past its largest incoming delay and `most` allows;
+// below 2, 0. Reads the links once; the room of the push table, not yet written, holds the ranges.
 int chunk_steps(const n2b_population *pops, int32_t n_pops, const std::vector<n2b::ConnDev> &push,
                 const std::vector<int32_t> &push_tgt, char *ws, const Layout &L, cudaStream_t s, int32_t most,
                 int32_t *out) {
@@ -306,11 +298,42 @@ int chunk_steps(const n2b_population *pops, int32_t n_pops, const std::vector<n2
         if (push[c].n_links > 0 && pops[push_tgt[c]].n > 0)
             k = std::min(k, std::min(range[2 * c], pops[push_tgt[c]].acc_depth - range[2 * c + 1]));
     if (most > 0) k = std::min(k, most);
-    int64_t links = 0, neurons = 0;
-    for (size_t c = 0; c < push.size(); ++c) links += push[c].n_links;
-    for (int32_t p = 0; p < n_pops; ++p) neurons += pops[p].n;
-    if (k >= 3 || (k == 2 && (most > 0 || links <= PAIR_ROW * neurons))) *out = k;
+    if (k >= 2) *out = k;
     return N2B_OK;
+}
+
+int32_t chunk_tiles_of(const n2b_population *pops, int32_t n_pops, int32_t tn) {
+    int32_t tiles = 0;
+    for (int32_t p = 0; p < n_pops; ++p) tiles += (pops[p].n + tn - 1) / tn;
+    return tiles;
+}
+
+// The smallest tiles that two blocks per SM still hold at once (1,000 neurons: 32 blocks of 32), 256 at most: a tile's
+// spikes are its block's to deliver.
+int32_t chunk_tile(const n2b_population *pops, int32_t n_pops, int sms) {
+    int32_t tn = 32;
+    while (tn < 256 && chunk_tiles_of(pops, n_pops, tn) > 2 * sms) tn *= 2;
+    return tn;
+}
+
+// Whether chunks of k steps are faster than a barrier per step. A chunk saves k - 1 barriers, but a spike's row is its
+// own block's to deliver where a barrier's step spreads its links of delay >= 2 over the grid: the longer the rows
+// (links per neuron) for the steps of a chunk, and the more neurons to a block, the more it loses. Measured (model A at
+// several rates, the microcircuit and eight unequal populations with their delays raised; barrier over chunk):
+//   tiles of at most 128 neurons (37,888 in all): rows of up to 390 k links 1.05 to 4.1, of 400 k 0.95 to 1.12, more
+//   0.6 to 1.6;
+//   tiles of 256 that two blocks per SM hold (75,776): up to 128 k links and 1,300 in all 1.09 to 2.8; the microcircuit at
+//   129 k to 200 k 0.37 to 0.8;
+//   more tiles than that, several to a block: up to 50 k links and 640 in all 1.02 to 1.9; at 78 k 0.94, 208 k 0.72 to 1.13.
+bool chunks_pay(const n2b_population *pops, int32_t n_pops, const std::vector<n2b::ConnDev> &push, int32_t k, int sms) {
+    int64_t links = 0, neurons = 0;
+    for (const n2b::ConnDev &c : push) links += c.n_links;
+    for (int32_t p = 0; p < n_pops; ++p) neurons += pops[p].n;
+    const int32_t tn = chunk_tile(pops, n_pops, sms);
+    if (tn <= 128) return links <= 390 * k * neurons;
+    k = std::min(k, n2b::chunk_most(tn));
+    return chunk_tiles_of(pops, n_pops, tn) <= 2 * sms ? links <= std::min<int64_t>(128 * k, 1300) * neurons
+                                                       : links <= std::min<int64_t>(50 * k, 640) * neurons;
 }
 
 void drop_graph(n2b_net *net) {
@@ -547,14 +570,10 @@ int n2b_create(const n2b_population *pops, int32_t n_pops, const n2b_connection 
         grid = std::max(grid, 1);
     }
     int32_t chunk_tn = 0, chunk_tiles = 0;
+    if (chunk && !(opt && opt->chunk & 0xFFFF) && !chunks_pay(pops, n_pops, push, chunk, sms)) chunk = 0;
     if (chunk) {
-        // the smallest tiles that two blocks per SM still hold at once: a tile's spikes are its block's to deliver
-        // (1,000 neurons: 32 blocks of 32)
-        for (chunk_tn = 32;; chunk_tn *= 2) {
-            chunk_tiles = 0;
-            for (int32_t p = 0; p < n_pops; ++p) chunk_tiles += (pops[p].n + chunk_tn - 1) / chunk_tn;
-            if (chunk_block(opt) ? chunk_tn == chunk_block(opt) : (chunk_tiles <= 2 * sms || chunk_tn == 256)) break;
-        }
+        chunk_tn = chunk_block(opt) ? chunk_block(opt) : chunk_tile(pops, n_pops, sms);
+        chunk_tiles = chunk_tiles_of(pops, n_pops, chunk_tn);
         chunk = std::min(chunk, n2b::chunk_most(chunk_tn));
         int per_sm = 0;
         N2B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chunk_kernel_of(chunk_tn), n2b::CHUNK_THREADS, 0));

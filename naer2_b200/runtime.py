@@ -36,7 +36,6 @@ from .topology import delay_steps, pack_links, pull_split_form, push_form
 
 MAX_SHIFT = 40
 MAX_LOOKAHEAD = 32  # steps without a grid barrier between them, at most (csrc/n2b_device.cuh, CHUNK_MAX)
-PAIR_ROW = 640  # links per neuron up to which they may be two (csrc/naer2b.cu)
 INLINE_POPS, INLINE_PUSH = 32, 64  # populations and push connections of a network that may (csrc/n2b_device.cuh)
 
 
@@ -229,7 +228,27 @@ def lookahead(net, desc: NetDesc) -> int:
     k = desc.lookahead if net.persistent and len(desc.pops) <= INLINE_POPS and len(desc.conns) <= INLINE_PUSH else 1
     if net.steps_per_barrier:
         return min(k, int(net.steps_per_barrier))
-    return k if k != 2 or desc.n_links <= PAIR_ROW * sum(p.n for p in desc.pops) else 1
+    sizes = [p.n for p in desc.pops]
+    return k if k > 1 and chunks_pay(sizes, desc.n_links, k, blocks_at_once(net.device)) else 1
+
+
+def blocks_at_once(device) -> int:
+    return 2 * torch.cuda.get_device_properties(device).multi_processor_count
+
+
+def chunks_pay(sizes: list, links: int, k: int, at_once: int) -> bool:
+    """The library's rule (csrc/naer2b.cu, chunks_pay): whether k steps between two barriers are faster than one, for
+    populations of these sizes and `links` links in all; at_once: two blocks per SM."""
+    tile = 32
+    while tile < 256 and sum(-(-n // tile) for n in sizes) > at_once:
+        tile *= 2
+    if tile <= 128:
+        row = 390 * k
+    elif sum(-(-n // tile) for n in sizes) <= at_once:
+        row = min(128 * min(k, 16), 1300)
+    else:
+        row = min(50 * min(k, 16), 640)
+    return links <= row * sum(sizes)
 
 
 class NetworkRuntime:

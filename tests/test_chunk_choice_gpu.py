@@ -51,7 +51,7 @@ def test_slots_are_kept_for_chunks_alone(cuda, change):
         for i in range(60):
             c = a >> fixed_indegree(2, seed=i) >> a
             c.weight, c.delay = 0.01, 1.5
-    if change == "rows":  # two steps between barriers, rows past the rule's line
+    if change == "rows":  # two steps between barriers, 1,300 links per neuron: past the rule's line
         a = net.populations[1]
         c = a >> fixed_indegree(2400, seed=1) >> a
         c.weight, c.delay = 0.0005, 0.2

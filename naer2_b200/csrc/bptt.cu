@@ -17,9 +17,10 @@
 // Layout: a group of 8 CTAs runs 8 samples; CTA `rank` owns hidden neurons [rank*HC, rank*HC + HC), HC = H/8.
 // Spiking forward (fwd_group_kernel) and adjoint (bwd_kernel): eight threads per neuron, groups of one cooperative
 // launch (one CTA per SM: at that size only 15 clusters of 8 are resident on 148 SMs, but every group must be) that
-// exchange a step's spikes, or its q, through the L2. The smooth model, and rows that do not fit a CTA's shared
-// memory, take fwd_kernel: four threads per neuron (two samples each), the group a thread-block cluster, every CTA
-// writing its neurons' entries into all 8 CTAs' spike rings (distributed shared memory) before one cluster barrier.
+// exchange a step's spikes, or its q, through the L2. The smooth model, rows that do not fit a CTA's shared memory, short
+// sequences and many groups (scans) take fwd_kernel: four threads per neuron (two samples each), the group a
+// thread-block cluster, every CTA writing its neurons' entries into all 8 CTAs' spike rings (distributed shared memory)
+// before one cluster barrier.
 // The forward keeps the last spikes of all H neurons for its 8 samples in shared memory (one byte of 8 sample bits per
 // neuron, or 8 floats in the smooth model). Backward: what it needs of the forward is the surrogate's derivative of
 // every step. Up to FULL_TAPE_BYTES the forward keeps them; past that each K-step segment is first recomputed from its

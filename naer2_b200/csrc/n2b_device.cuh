@@ -1491,11 +1491,11 @@ __device__ __forceinline__ bool grid_sync(const StepArgs &a, unsigned k) {
     return grid_wait(a, k);
 }
 
-// Whether an earlier window gave up (nothing runs then). One thread reads the word for the block: a block of this launch
-// may set it meanwhile, and a block of which some threads saw it and others not would wait and read what its first
-// thread never wrote.
-__device__ __forceinline__ bool stopped(const StepArgs &a) {
-    return __syncthreads_or(threadIdx.x == 0 && *(volatile unsigned *)(a.barrier + BAR_ABORT));
+// Whether an earlier window gave up (nothing runs then), to be voted on by the block (__syncthreads_or) once the loads
+// that a kernel starts with are on their way. One thread reads the word: a block of this launch may set it meanwhile, and
+// a block of which some threads saw it and others not would wait and read what its first thread never wrote.
+__device__ __forceinline__ unsigned stop_word(const StepArgs &a) {
+    return threadIdx.x == 0 ? *(volatile unsigned *)(a.barrier + BAR_ABORT) : 0u;
 }
 
 // The end of a chunked window, on every way out of it: the last block to get here advances the step counter and
@@ -1516,7 +1516,7 @@ enum { WITH_PULL, PLAIN, DENSE };
 template <int NPB, bool INL, int KIND>
 __global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
     persistent_kernel(const __grid_constant__ StepArgs a, const int n_steps) {
-    if (stopped(a)) return;
+    const unsigned stop = stop_word(a);
     const long long n0 = *a.step;
     __shared__ Scratch<NPB> sc;
     if (threadIdx.x == 0) sc.rec0 = *a.rec0;  // (read at each step it would miss the L1, in the step's chain)
@@ -1533,7 +1533,7 @@ __global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
     __shared__ SConn s_tab[SMEM_CONNS];
     const SConn *s_conn = fill_conns<INL>(a, s_tab, a.n_push);
     PullStage *stage = KIND == WITH_PULL ? warp_stage(a) : nullptr;
-    __syncthreads();
+    if (__syncthreads_or(stop)) return;
     for (int k = 0; k < n_steps; ++k) {
         step_body<NPB, INL, KIND == DENSE ? 2 : 4, KIND == WITH_PULL>(a, n0 + k, k, &mine, s_cache, s_conn, stage,
                                                                            sc);
@@ -1545,14 +1545,13 @@ __global__ void __launch_bounds__(NPB, KIND == DENSE ? 3 : 2)
 
 // ------------------------------------------------------------------ chunks of steps
 
-// Networks whose every link has a delay of at least K >= 2 steps (a single transmission delay of 1.5 ms is 15; which
-// of them run in chunks: chunk_steps, naer2b.cu): what
-// a step reads was sent at least K steps earlier, so K steps need no grid barrier between them. A block runs K
-// steps of its tile of TN neurons straight through (phase 1: slots read and cleared, update, spikes listed; no
-// barrier of any kind, one thread per neuron, its random draws made beforehand by the whole block), then delivers
-// all their spikes (phase 2: every link of their rows, arriving after the chunk), then meets the grid. What bounds a chunk is its barrier, its slots' loads and its
-// deliveries' latencies, once per K steps instead of every step: 1,000 neurons at K = 15 step in 0.88 us (4.0 with a
-// barrier per step), 12,500 neurons at K = 15 in 1.5 us (4.6).
+// Networks whose every link has a delay of at least K >= 2 steps (a single transmission delay of 1.5 ms is 15; which of
+// them run in chunks: chunk_steps, naer2b.cu): what a step reads was sent at least K steps earlier, so K steps need no
+// grid barrier between them. A block runs K steps of its tile of TN neurons straight through (phase 1: slots read and
+// cleared, update, spikes listed; no barrier of any kind, one thread per neuron, its random draws made beforehand by the
+// whole block), then delivers all their spikes (phase 2: every link of their rows, arriving after the chunk), then meets
+// the grid. What bounds a chunk is its barrier, its slots' loads and its deliveries' latencies, once per K steps instead
+// of every step: 1,000 neurons at K = 15 step in 0.88 us (4.0 with a barrier per step), 12,500 neurons in 1.5 us (4.2).
 // The slots' depth is at least K + the largest delay into their population, so that a block K - 1 steps ahead of
 // another never adds into a slot that the other has yet to read.
 
@@ -1652,10 +1651,7 @@ __device__ __forceinline__ void chunk_deliver(const StepArgs &a, const PopDev &P
 template <int TN>
 __global__ void __launch_bounds__(CHUNK_THREADS, 2)
     chunk_kernel(const __grid_constant__ StepArgs a, const int n_steps, const int chunk, const int n_tiles) {
-    if (stopped(a)) {
-        finish_window(a, n_steps);
-        return;
-    }
+    const unsigned stop = stop_word(a);
     __shared__ SConn s_tab[SMEM_CONNS];
     __shared__ int s_rows[2 * MERGE_OUT * TN];
     __shared__ uint16_t s_spk[TN * chunk_most(TN)];
@@ -1690,7 +1686,11 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2)
                         s_rows[(2 * c + 1) * TN + tid] = r.r1;
                     }
             }
-            __syncthreads();  // the previous tile's deliveries are done with the list
+            // the previous tile's deliveries are done with the list (and, at the first tile, nothing is written yet)
+            if (__syncthreads_or(stop)) {
+                finish_window(a, n_steps);
+                return;
+            }
             if (tid == 0) s_cnt = 0;
             if (!single || round == 0) draws(tile, n0, kend);
             __syncthreads();

@@ -19,7 +19,7 @@ neurons' state in registers and its row bounds throughout, and the steps are sep
 wait that gives up sets an abort word, and the kernel winds down). A step is a chain of memory latencies, so what it
 costs is the launches around it and the loads that a launch starts with. Measured, us per step, links looked up ->
 arrival bits, one launch per population -> window: 12,500 neurons of 1,250 links (47 spikes a step) 92 -> 19.4 ->
-7.5; 1,501 neurons of 150 plastic links 33 -> 11.2 -> 6.1; 3,001 event-driven neurons of 125 links 73 -> 36 ->
+7.3; 1,501 neurons of 150 plastic links 33 -> 11.2 -> 6.1; 3,001 event-driven neurons of 125 links 73 -> 36 ->
 11.6.
 """
 
@@ -470,7 +470,7 @@ def population(pop_name: str, attrs: dict, hooks: dict, incoming: list, n_out: i
     src.append(f"""// population {pop_name}
 template <bool WINDOW>
 __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const int blk, long long n, const int n_steps,
-                                         const double dt, const N2Grid &grid) {{
+                                         const double dt, const N2Grid &grid, const u32 stop) {{
     const int jl = threadIdx.x / SCAN, sc = threadIdx.x % SCAN;
     const int j = blk * NPB_C + jl;
     const bool live = j < p.n, own = sc == 0;
@@ -486,7 +486,8 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
         s.optr[k / (NPB_C + 1)][q] = p.outs[k / (NPB_C + 1)].ptr[min(blk * NPB_C + q, p.n)];
     }}
 """)
-    src.append('    if (!WINDOW) asm volatile("griddepcontrol.wait;" ::: "memory");\n')
+    src.append('    if (!WINDOW) asm volatile("griddepcontrol.wait;" ::: "memory");\n'
+               "    if (WINDOW && __syncthreads_or(stop)) return;  // an earlier window gave up: nothing runs\n")
     for a, py in attrs.items():
         ct, _, _ = ctype_of(py)
         src.append(f"    {ct} s_{a} = (live && own) ? p.s_{a}[j] : ({ct})0;\n")
@@ -580,7 +581,7 @@ __device__ __forceinline__ void n2_steps(const Params &p, N2Scratch &s, const in
 STEP_KERNEL = f"""
 extern "C" __global__ void __launch_bounds__({THREADS}) n2b_user_step(const __grid_constant__ Params p) {{
     __shared__ N2Scratch s;
-    n2_steps<false>(p, s, (int)blockIdx.x, p.step, 1, 0.0, N2Grid{{}});
+    n2_steps<false>(p, s, (int)blockIdx.x, p.step, 1, 0.0, N2Grid{{}}, 0u);
 }}
 """
 
@@ -613,8 +614,8 @@ def window_source(exact: bool, kinds: list, edges: int, per_sm: int) -> str:
 
 extern "C" __global__ void __launch_bounds__({THREADS}, {per_sm}) n2b_user_window(const __grid_constant__ Window w) {{
     __shared__ N2Scratch s;
-    // an earlier window gave up: nothing runs (one thread reads for the block: another block may set it meanwhile)
-    if (__syncthreads_or(threadIdx.x == 0 && *(volatile u32 *)(w.grid.bar + 32))) return;
+    // set when an earlier window gave up (one thread reads for the block: another block may set it meanwhile)
+    const u32 stop = threadIdx.x == 0 ? *(volatile u32 *)(w.grid.bar + 32) : 0u;
     int k = 0;
     while ((int)blockIdx.x >= w.first[k + 1]) ++k;
     const int b = (int)blockIdx.x - w.first[k];
@@ -622,7 +623,7 @@ extern "C" __global__ void __launch_bounds__({THREADS}, {per_sm}) n2b_user_windo
     before = 0
     for g, (_, count) in enumerate(kinds):
         src.append(f"    if (k >= {before} && k < {before + count}) n2p{g}::n2_steps<true>(w.p{g}[{f'k - {before}' if count > 1 else 0}], "
-                   "s, b, w.step0, (int)w.n_steps, w.dt, w.grid);\n")
+                   "s, b, w.step0, (int)w.n_steps, w.dt, w.grid, stop);\n")
         before += count
     src.append("}\n")
     return "".join(src)

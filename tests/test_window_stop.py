@@ -41,12 +41,12 @@ def test_one_thread_reads_the_stop_word():
     assert len(reads) >= 2
     for at in reads:
         line = text[text.rindex("\n", 0, at):text.index("\n", at)]
-        assert "__syncthreads_or(threadIdx.x == 0 && " in line or "(spin & 15) == 15" in line, line
+        assert "threadIdx.x == 0 ? " in line or "(spin & 15) == 15" in line, line
+    assert text.count("= stop_word(a)") == text.count("if (__syncthreads_or(stop))") == 2
     window = plan_of(_user_net())["window"]["source"]
     kernel = window[window.index("n2b_user_window"):]
-    assert re.search(r"if \(__syncthreads_or\(threadIdx\.x == 0 && \*\(volatile u32 \*\)\(w\.grid\.bar \+ 32\)\)\)",
-                     kernel)
-    assert kernel.count("volatile") == 1
+    assert "const u32 stop = threadIdx.x == 0 ? *(volatile u32 *)(w.grid.bar + 32) : 0u;" in kernel
+    assert kernel.count("volatile") == 1 and "if (WINDOW && __syncthreads_or(stop)) return;" in window
 
 
 @pytest.mark.gpu
